@@ -85,6 +85,41 @@ def test_batched_mixed_problem_sizes():
         assert param_rel(b.get_params(i), (R, T, X)) < 1e-5
 
 
+@pytest.mark.parametrize("threads", [64, 128, 256])
+@pytest.mark.parametrize("cams,points,twice,k22", [
+    (1, 9, False, 1.0), (2, 31, False, 1.0), (3, 1, False, 1.0), (3, 32, False, 1.0), (3, 33, True, 1.0),
+    (3, 257, True, 1.0), (4, 64, False, 1.0), (4, 65, True, 1.0), (3, 40, False, 1.25)])
+def test_batched_tile_edges(cams, points, twice, k22, threads):
+    """Points at the edges of a warp's 32, every camera count, tracks that name a camera twice or
+    miss one, and an intrinsic matrix whose last row is not (0, 0, 1): two iterations against the
+    restatement.  With the first lambda at 1e-3 of the largest diagonal entry the damped systems have
+    condition numbers up to ~1e6 (points along a viewing ray), so FP64 sums in another order stay
+    below 1e-9."""
+    rng = np.random.default_rng(100 * cams + points)
+    sc = scenes.circle_scene(n_cams=max(cams, 4), n_points=points, obs_per_point=4, seed=points, inlier_threshold=2.0)
+    use = sc.view < cams
+    drop = (sc.point % 5 == 1) & (sc.view == cams - 1) if cams > 2 else np.zeros(sc.n_obs, bool)
+    meas, view, point = sc.meas[use & ~drop], sc.view[use & ~drop], sc.point[use & ~drop]
+    if twice:   # a second measurement of camera 0 (and of the last camera) in every third track
+        for c in (0, cams - 1):
+            again = (view == c) & (point % 3 == 0)
+            meas = np.concatenate([meas, meas[again] + rng.normal(scale=0.5, size=(int(again.sum()), 2))])
+            view, point = np.concatenate([view, view[again]]), np.concatenate([point, point[again]])
+        o = np.argsort(point, kind="stable")
+        meas, view, point = meas[o], view[o], point[o]
+    K = sc.K[:cams].copy()
+    K[:, 2, 2] = k22
+    sc = scenes.Scene(sc.model, sc.mode, sc.inlier_threshold, K, sc.R[:cams].copy(), sc.T[:cams].copy(), sc.X, meas,
+                      view.astype(np.int32), point.astype(np.int32), None)
+    (_, R, T, _, X), info = Restatement().minimize(sc, max_iterations=2)
+    b = capi.Batch([sc, sc])
+    b.set_schedule(threads, threads, 0)
+    res, _ = b.minimize(max_iterations=2)
+    for i in range(2):
+        assert (res[i].status, res[i].iterations, res[i].n_rejected) == (info["status"], info["iterations"], info["n_rejected"])
+        assert param_rel(b.get_params(i), (R, T, X)) < 1e-9
+
+
 @pytest.fixture(scope="module")
 def bench_batch():
     """The bench's own batch (4096 triplets of 50-800 points, seed 0) and 64 of its triplets

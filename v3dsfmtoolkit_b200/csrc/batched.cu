@@ -13,11 +13,9 @@
 // Model: StdMetricBundleOptimizer, up to kMaxCams = 4 cameras per problem (reduced system up to
 // 24 x 24), any number of points, each point observed by up to kMaxTrack cameras.  Everything
 // is FP64.  Per-point quantities are recomputed from the parameters in every pass over the
-// points instead of being stored (FLOPs are cheap, shared memory is not): pass REL (weights,
-// cost, gradient, max diagonal), pass SCHUR (one 6x6 camera-pair block of the reduced system per
-// round, accumulated in registers and folded by a transposing warp reduction -- deterministic,
-// no atomics), a warp Cholesky of the reduced system, pass STEP (point back-substitution, trial
-// points, trial cost with frozen weights).
+// points instead of being stored: one pass per iteration linearises and builds the damped reduced
+// system on the FP64 tensor cores, a warp solves it, and a second pass takes the step
+// (back-substitution, trial points, trial cost with frozen weights).
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -34,7 +32,6 @@ namespace {
 
 constexpr int kMaxCams = 4;
 constexpr int kMaxTrack = 16;
-constexpr int kMaxN = 6 * kMaxCams;  // reduced system dimension
 
 struct BatchDev {
   int count = 0;
@@ -72,36 +69,6 @@ struct BatchOpts {
   int max_iter;
 };
 
-template <int H, int V>
-__device__ __forceinline__ void rt_stage_b(double (&v)[V], int lane, int m) {
-#pragma unroll
-  for (int t = 0; t < H; ++t) {
-    const bool up = (lane & m) != 0;
-    const double send = up ? v[t] : v[t + H];
-    const double keep = up ? v[t + H] : v[t];
-    v[t] = keep + __shfl_xor_sync(0xffffffffu, send, m);
-  }
-}
-
-// Block-wide deterministic sum of V = 64 values; thread t < 64 returns the total of value t.
-template <int NT>
-__device__ __forceinline__ double block_sum64(double (&v)[64], double* red /* [NT/32][64] */) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  rt_stage_b<32>(v, lane, 16);
-  rt_stage_b<16>(v, lane, 8);
-  rt_stage_b<8>(v, lane, 4);
-  rt_stage_b<4>(v, lane, 2);
-  rt_stage_b<2>(v, lane, 1);
-  red[wid * 64 + 2 * lane] = v[0];
-  red[wid * 64 + 2 * lane + 1] = v[1];
-  __syncthreads();
-  double s = 0.0;
-  if (threadIdx.x < 64)
-    for (int w = 0; w < NT / 32; ++w) s += red[w * 64 + threadIdx.x];
-  __syncthreads();
-  return s;
-}
-
 template <int NT>
 __device__ __forceinline__ double block_max(double v, double* red) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -116,88 +83,283 @@ __device__ __forceinline__ double block_max(double v, double* red) {
 
 struct CamS {
   double R[9], T[3], K[9];
+  double f, fy;   // focal lengths of the Jacobian rows: K00 and (K11 / K00) K00
+  int affine;     // the last row of K is 0 0 1: the projection divides by the depth itself
 };
 
-// Weighted Jacobian blocks and weighted residual of observation k at (cams, X).
-__device__ __forceinline__ void lin_obs(const CamS* cams, const double X[3], const BatchDev& b, int k, double wk,
-                                        double A[2][6], double B[2][3], double r[2], double* e_out) {
-  const int c = b.cam[k];
-  Cam cm;
+// ---- one problem per block: the pieces of k_batched_lm -----------------------------------------
+
+// Columns of the per-warp operand tiles: 32 points x 2 residual rows, padded so that the eight rows
+// that a fragment load touches fall into different banks (a row is 4 double banks after the last).
+constexpr int kTileK = 64, kTileLd = kTileK + 4;
+
+template <int NC>
+struct BatchLay {
+  static constexpr int kPairs = NC * (NC + 1) / 2;
+  static constexpr int kA = NC * 6 * kTileLd;    // A_c, column per (point, residual row)
+  static constexpr int kZ = 8 * kTileLd;         // right operand of one camera pair
+  static constexpr int kWarp = kA + kZ;          // doubles per warp (the A part also holds its sums)
+  static constexpr int kDim = 6 * NC;
+  static constexpr int kSld = kDim + 1;
+  static_assert(kPairs * 64 <= kA, "a warp's block sums take the place of its A tiles");
+};
+
+__device__ __forceinline__ void dmma884(double& c0, double& c1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(c0), "+d"(c1)
+               : "d"(a), "d"(b));
+}
+
+// One observation at (cam, X): the residual, v = R X, the depth's point and d proj / d XX, whose
+// nonzero entries are {P00, P02, P11, P12}.
+struct ObsLin {
+  double e[2], v[3], P[4];
+};
+__device__ __forceinline__ void project_obs(const CamS& c, const double X[3], double mx, double my, ObsLin& o) {
 #pragma unroll
-  for (int q = 0; q < 9; ++q) cm.R[q] = cams[c].R[q];
+  for (int r = 0; r < 3; ++r) o.v[r] = c.R[3 * r] * X[0] + c.R[3 * r + 1] * X[1] + c.R[3 * r + 2] * X[2];
+  const double y0 = o.v[0] + c.T[0], y1 = o.v[1] + c.T[1], y2 = o.v[2] + c.T[2];
+  const double iz = 1.0 / y2;
+  double ih = iz;
+  if (!c.affine) ih = 1.0 / (c.K[6] * y0 + c.K[7] * y1 + c.K[8] * y2);
+  o.e[0] = (c.K[0] * y0 + c.K[1] * y1 + c.K[2] * y2) * ih - mx;
+  o.e[1] = (c.K[3] * y0 + c.K[4] * y1 + c.K[5] * y2) * ih - my;
+  o.P[0] = c.f * iz;
+  o.P[1] = -o.P[0] * y0 * iz;
+  o.P[2] = c.fy * iz;
+  o.P[3] = -o.P[2] * y1 * iz;
+}
+__device__ __forceinline__ void weigh(ObsLin& o, double w, double r[2]) {
+  r[0] = -w * o.e[0];
+  r[1] = -w * o.e[1];
 #pragma unroll
-  for (int q = 0; q < 3; ++q) cm.T[q] = cams[c].T[q];
+  for (int t = 0; t < 4; ++t) o.P[t] *= w;
+}
+__device__ __forceinline__ void point_block(const CamS& c, const ObsLin& o, double B[2][3]) {
 #pragma unroll
-  for (int q = 0; q < 9; ++q) cm.K[q] = cams[c].K[q];
-  cm.d[0] = cm.d[1] = cm.d[2] = cm.d[3] = 0.0;
-  double e[2], Cc[2][1];
-  linearize_obs<kModelStd, 6, 0>(cm, X, b.meas[2 * k], b.meas[2 * k + 1], 0, 1.0, e, A, B, Cc);
-  if (e_out) { e_out[0] = e[0]; e_out[1] = e[1]; }
-  r[0] = -wk * e[0];
-  r[1] = -wk * e[1];
+  for (int q = 0; q < 3; ++q) {
+    B[0][q] = o.P[0] * c.R[q] + o.P[1] * c.R[6 + q];
+    B[1][q] = o.P[2] * c.R[3 + q] + o.P[3] * c.R[6 + q];
+  }
+}
+__device__ __forceinline__ void camera_block(const ObsLin& o, double A[2][6]) {
+  A[0][0] = o.P[0]; A[0][1] = 0.0; A[0][2] = o.P[1];
+  A[1][0] = 0.0; A[1][1] = o.P[2]; A[1][2] = o.P[3];
+  A[0][3] = o.P[1] * o.v[1];
+  A[0][4] = o.P[0] * o.v[2] - o.P[1] * o.v[0];
+  A[0][5] = -o.P[0] * o.v[1];
+  A[1][3] = o.P[3] * o.v[1] - o.P[2] * o.v[2];
+  A[1][4] = -o.P[3] * o.v[0];
+  A[1][5] = o.P[2] * o.v[0];
+}
+
+__device__ __forceinline__ void add_point(const double B[2][3], const double r[2], double V[6], double gb[3]) {
 #pragma unroll
   for (int rr = 0; rr < 2; ++rr) {
+    V[0] += B[rr][0] * B[rr][0]; V[1] += B[rr][0] * B[rr][1]; V[2] += B[rr][0] * B[rr][2];
+    V[3] += B[rr][1] * B[rr][1]; V[4] += B[rr][1] * B[rr][2]; V[5] += B[rr][2] * B[rr][2];
 #pragma unroll
-    for (int q = 0; q < 6; ++q) A[rr][q] *= wk;
-#pragma unroll
-    for (int q = 0; q < 3; ++q) B[rr][q] *= wk;
+    for (int c = 0; c < 3; ++c) gb[c] += B[rr][c] * r[rr];
   }
 }
 
-// (V_j + lambda I)^-1 (packed 00,01,02,11,12,22), gb_j and q = Vinv gb over the point's track.
-__device__ __forceinline__ bool point_elim(const CamS* cams, const double X[3], const BatchDev& b, int o0, int n,
-                                           double lam, double vi[6], double gb[3], double q[3]) {
-  double V[6] = {0, 0, 0, 0, 0, 0};
-  gb[0] = gb[1] = gb[2] = 0.0;
-  for (int t = 0; t < n; ++t) {
-    double A[2][6], B[2][3], r[2];
-    lin_obs(cams, X, b, o0 + t, b.w[o0 + t], A, B, r, nullptr);
-#pragma unroll
-    for (int rr = 0; rr < 2; ++rr) {
-      V[0] += B[rr][0] * B[rr][0]; V[1] += B[rr][0] * B[rr][1]; V[2] += B[rr][0] * B[rr][2];
-      V[3] += B[rr][1] * B[rr][1]; V[4] += B[rr][1] * B[rr][2]; V[5] += B[rr][2] * B[rr][2];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) gb[c] += B[rr][c] * r[rr];
-    }
-  }
-  V[0] += lam; V[3] += lam; V[5] += lam;
-  const double c00 = V[3] * V[5] - V[4] * V[4], c01 = V[2] * V[4] - V[1] * V[5], c02 = V[1] * V[4] - V[2] * V[3];
-  const double det = V[0] * c00 + V[1] * c01 + V[2] * c02;
+// (V + lambda I)^-1 by cofactors; *det tells a singular point (0) from a non-finite one.
+__device__ __forceinline__ bool invert_point(const double V[6], double lam, double vi[6], double* det_out) {
+  const double a0 = V[0] + lam, a3 = V[3] + lam, a5 = V[5] + lam;
+  const double c00 = a3 * a5 - V[4] * V[4], c01 = V[2] * V[4] - V[1] * a5, c02 = V[1] * V[4] - V[2] * a3;
+  const double det = a0 * c00 + V[1] * c01 + V[2] * c02;
+  *det_out = det;
   if (!(det != 0.0) || !isfinite(det)) return false;
   const double id = 1.0 / det;
   vi[0] = c00 * id; vi[1] = c01 * id; vi[2] = c02 * id;
-  vi[3] = (V[0] * V[5] - V[2] * V[2]) * id;
-  vi[4] = (V[1] * V[2] - V[0] * V[4]) * id;
-  vi[5] = (V[0] * V[3] - V[1] * V[1]) * id;
-  q[0] = vi[0] * gb[0] + vi[1] * gb[1] + vi[2] * gb[2];
-  q[1] = vi[1] * gb[0] + vi[3] * gb[1] + vi[4] * gb[2];
-  q[2] = vi[2] * gb[0] + vi[4] * gb[1] + vi[5] * gb[2];
+  vi[3] = (a0 * a5 - V[2] * V[2]) * id;
+  vi[4] = (V[1] * V[2] - a0 * V[4]) * id;
+  vi[5] = (a0 * a3 - V[1] * V[1]) * id;
   return true;
 }
+__device__ __forceinline__ void mul_sym3(const double vi[6], const double x[3], double y[3]) {
+  y[0] = vi[0] * x[0] + vi[1] * x[1] + vi[2] * x[2];
+  y[1] = vi[1] * x[0] + vi[3] * x[1] + vi[4] * x[2];
+  y[2] = vi[2] * x[0] + vi[4] * x[1] + vi[5] * x[2];
+}
 
-// W = A^T B (6x3) and T = W Vinv of one observation.
-__device__ __forceinline__ void wt_of(const double A[2][6], const double B[2][3], const double vi[6], double W[6][3],
-                                      double Tm[6][3]) {
+__device__ __forceinline__ void store_a(double* Ac, int lane, const double A[2][6]) {
 #pragma unroll
-  for (int a = 0; a < 6; ++a)
+  for (int a = 0; a < 6; ++a) *reinterpret_cast<double2*>(Ac + a * kTileLd + 2 * lane) = make_double2(A[0][a], A[1][a]);
+}
+
+// acc += A Z^T over the warp's 32 points: rows 0..5 of the left tile against `rows` rows of the right
+// one; the other rows are read from `zero`.  Four accumulators in turn: a chain of 16 dependent DMMAs
+// would take about 500 cycles, and an SM holds only 12 warps.
+__device__ __forceinline__ void tile_product(const double* Ac, const double* Z, const double* zero, int rows, int lane,
+                                             double (&acc)[2]) {
+  const int r = lane >> 2, k = lane & 3;
+  const double* ap = (r < 6 ? Ac + r * kTileLd : zero) + k;
+  const double* zp = (r < rows ? Z + r * kTileLd : zero) + k;
+  double part[4][2];
 #pragma unroll
-    for (int c = 0; c < 3; ++c) W[a][c] = A[0][a] * B[0][c] + A[1][a] * B[1][c];
+  for (int t = 0; t < 4; ++t) part[t][0] = part[t][1] = 0.0;
+#pragma unroll 1
+  for (int s = 0; s < kTileK; s += 16)
+#pragma unroll
+    for (int t = 0; t < 4; ++t) dmma884(part[t][0], part[t][1], ap[s + 4 * t], zp[s + 4 * t]);
+#pragma unroll
+  for (int t = 0; t < 2; ++t) acc[t] += (part[0][t] + part[1][t]) + (part[2][t] + part[3][t]);
+}
+
+// Z = (delta I - BV_t B_u^T) A_u for the lane's point (zero unless `use`); A_u is read back from the
+// lane's own columns of its tile.
+__device__ __forceinline__ void store_z(double* Z, const double* Au, int lane, const double BV[2][3], const double Bu[2][3],
+                                        bool diag, bool use) {
+  double P[2][2];
+#pragma unroll
+  for (int r = 0; r < 2; ++r)
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      P[r][c] = ((diag && r == c) ? 1.0 : 0.0) - (BV[r][0] * Bu[c][0] + BV[r][1] * Bu[c][1] + BV[r][2] * Bu[c][2]);
+      if (!use) P[r][c] = 0.0;
+    }
 #pragma unroll
   for (int a = 0; a < 6; ++a) {
-    Tm[a][0] = W[a][0] * vi[0] + W[a][1] * vi[1] + W[a][2] * vi[2];
-    Tm[a][1] = W[a][0] * vi[1] + W[a][1] * vi[3] + W[a][2] * vi[4];
-    Tm[a][2] = W[a][0] * vi[2] + W[a][1] * vi[4] + W[a][2] * vi[5];
+    const double2 u = *reinterpret_cast<const double2*>(Au + a * kTileLd + 2 * lane);
+    *reinterpret_cast<double2*>(Z + a * kTileLd + 2 * lane) =
+        make_double2(P[0][0] * u.x + P[0][1] * u.y, P[1][0] * u.x + P[1][1] * u.y);
   }
+}
+__device__ __forceinline__ void store_row(double* Z, int row, int lane, double x, double y) {
+  *reinterpret_cast<double2*>(Z + row * kTileLd + 2 * lane) = make_double2(x, y);
+}
+
+// Warp Cholesky of the reduced system (order 6 NC, identity beyond the problem's cameras) with the
+// right-hand side as one more row, then the back-substitution: lane r keeps row r in registers and a
+// step exchanges one column through shared memory.  False when a pivot is not positive.
+template <int NC>
+__device__ __forceinline__ bool warp_solve(double* S, const double* rhs, double* x, double* colb /* [2][32] */, int n6) {
+  constexpr int ND = BatchLay<NC>::kDim, LD = BatchLay<NC>::kSld;
+  const int lane = threadIdx.x & 31;
+  double row[ND];
+#pragma unroll
+  for (int c = 0; c < ND; ++c) {
+    double v = lane == c ? 1.0 : 0.0;
+    if (lane < n6 && c <= lane) v = S[lane * LD + c];
+    if (lane == ND) v = c < n6 ? rhs[c] : 0.0;
+    row[c] = v;
+  }
+  bool ok = true;
+  double inv_own = 1.0;
+#pragma unroll
+  for (int k = 0; k < ND; ++k) {
+    const double d = __shfl_sync(0xffffffffu, row[k], k);
+    if (!(d > 0.0)) ok = false;
+    const double inv = rsqrt(d > 0.0 ? d : 1.0);
+    if (lane == k) inv_own = inv;
+    const double l = row[k] * inv;
+    row[k] = l;
+    if (k + 1 < ND) {
+      double* cb = colb + 32 * (k & 1);   // two buffers: one barrier a step
+      cb[lane] = l;
+      __syncwarp();
+#pragma unroll
+      for (int c = k + 1; c < ND; ++c) row[c] -= l * cb[c];
+    }
+  }
+  __syncwarp();
+  if (lane < ND) {
+#pragma unroll
+    for (int c = 0; c < ND; ++c)
+      if (c <= lane) S[lane * LD + c] = row[c];
+  }
+  if (lane == ND) {
+#pragma unroll
+    for (int c = 0; c < ND; ++c) colb[c] = row[c];
+  }
+  __syncwarp();
+  double y = lane < ND ? colb[lane] : 0.0;
+#pragma unroll
+  for (int k = 0; k < ND; ++k) row[k] = (lane < k) ? S[k * LD + lane] : 0.0;   // column `lane` of L
+#pragma unroll
+  for (int k = ND - 1; k >= 0; --k) {
+    const double xk = __shfl_sync(0xffffffffu, y * inv_own, k);
+    if (lane == k) x[k] = xk;
+    y -= row[k] * xk;
+  }
+  return ok;
+}
+
+// One point of a pass: its track, and the measurement of each camera that sees it.  `mask` is empty
+// for a track that names a camera twice (it takes the general way) and beyond the last point.
+template <int NC>
+struct Track {
+  double X[3];
+  double2 m[NC];
+  int o0, n;
+  unsigned slot, mask;   // track position of camera c in bits 4c..4c+3 of slot, if bit c of mask
+  bool twice;
+};
+template <int NC>
+__device__ __forceinline__ Track<NC> load_track(const BatchDev& b, const double* Xc, int pt0, int M, int j) {
+  Track<NC> t;
+  const bool in = j < M;
+  const size_t g = (size_t)(pt0 + (in ? j : 0));
+  t.o0 = in ? b.ptr[g] : 0;
+  t.n = in ? b.ptr[g + 1] - t.o0 : 0;
+  t.slot = t.mask = 0;
+  t.twice = false;
+  for (int k = 0; k < t.n; ++k) {
+    const int c = b.cam[t.o0 + k];
+    t.twice |= (t.mask >> c) & 1u;
+    t.mask |= 1u << c;
+    t.slot |= (unsigned)k << (4 * c);
+  }
+  if (t.twice) t.mask = 0;
+#pragma unroll
+  for (int q = 0; q < 3; ++q) t.X[q] = in ? Xc[3 * g + q] : 0.0;
+#pragma unroll
+  for (int c = 0; c < NC; ++c)
+    t.m[c] = ((t.mask >> c) & 1u)
+                 ? *reinterpret_cast<const double2*>(b.meas + 2 * (size_t)(t.o0 + (int)((t.slot >> (4 * c)) & 15u)))
+                 : make_double2(0.0, 0.0);
+  return t;
 }
 
 template <int NT>
-__global__ void __launch_bounds__(NT) k_batched_lm(BatchDev b, BatchOpts o, int first, int last) {
-  __shared__ CamS cams[kMaxCams], tcams[kMaxCams];
-  __shared__ double S[kMaxN * kMaxN], rhs[kMaxN], da[kMaxN], ga[kMaxN], udiag[kMaxN];
-  __shared__ double red[(NT / 32) * 64];
-  __shared__ double sc[16];   // scalars: 0 err, 1 lambda, 2 nu, 3 newErr, 4 d2, 5 dg, 6 plen, 7 gmax, 8 maxdiag
-  __shared__ int si[8];       // 0 problem, 1 stop, 2 computeDerivatives, 3 fail, 4 accept, 5 status, 6 it, 7 rejected
-  const int tid = threadIdx.x;
+__device__ __forceinline__ double block_sum(double v, double* red) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  v = warp_sum(v);
+  if (lane == 0) red[wid] = v;
+  __syncthreads();
+  double s = 0.0;
+  for (int w = 0; w < NT / 32; ++w) s += red[w];
+  __syncthreads();
+  return s;
+}
+
+// One thread block per problem at a time.  A pass over the points gives each warp 32 points, one per
+// lane.  The reduced system is a product on the FP64 tensor cores: with residual rows 2p, 2p+1 of a
+// point's cameras as the inner dimension, block (i, l) is
+//     sum_p A_i^T (delta_il I - B_i (V + lambda I)^-1 B_l^T) A_l,
+// so one pass builds U, the Schur complement, the reduced rhs (a seventh column r_i - B_i q) and the
+// gradient (an eighth, r_i) from one linearisation of every observation; each warp sums its points in
+// eight-by-eight accumulators and the warps' sums are added in order (deterministic, no atomics).
+// Bound by FP64 latency: 168 registers and 14 KB of operand tiles per warp leave 12 warps per SM, the
+// FP64 pipe is active 24% and the DMMA pipe 16% of the cycles.  Of the 2.2 ms that 4096 triplets of
+// 50-800 points take for 4 iterations the products are 0.8, the step pass 0.5, the solve 0.25 (timed
+// by leaving each out).  A pass per camera pair that linearised each point again for it (39
+// linearisations per point and iteration instead of 6) took 6.7 ms; the same for 61 triplets 1.29 ms
+// against 0.17.
+template <int NT, int NC>
+__global__ void __launch_bounds__(NT, NT > 128 ? 1 : 384 / NT) k_batched_lm(BatchDev b, BatchOpts o, int first, int last) {
+  using L = BatchLay<NC>;
+  constexpr int NW = NT / 32, ND = L::kDim, LD = L::kSld;
+  extern __shared__ double dyn[];   // [NW][L::kWarp]
+  __shared__ CamS cams[NC], tcams[NC];
+  __shared__ double S[ND * LD], rhs[ND], da[ND], ga[ND], udiag[ND], colb[64], red[NW], zrow[kTileK];
+  __shared__ double sc[8];    // 0 err, 1 lambda, 2 nu, 3 newErr, 4 d2, 5 dg, 6 plen
+  __shared__ int si[8];       // 0 problem, 1 stop, 3 fail, 4 accept, 5 status, 7 rejected
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  double* Aw = dyn + wid * L::kWarp;
+  double* Zw = Aw + L::kA;
+  for (int e = tid; e < kTileK; e += NT) zrow[e] = 0.0;   // read after the barrier below
   for (;;) {
     if (tid == 0) {
       const unsigned slot = atomicAdd(b.queue, 1u);
@@ -208,294 +370,350 @@ __global__ void __launch_bounds__(NT) k_batched_lm(BatchDev b, BatchOpts o, int 
     if (p < 0) return;
     const int N = b.n_cams[p], M = b.n_pts[p], c0 = b.cam_off[p], pt0 = b.pt_off[p];
     const double thr = b.thr[p];
+    const int chunks = (M + 31) / 32;
+    const double* Xc = b.X;   // current and trial points; an accepted step swaps them
+    double* Xt = b.Xt;
     if (tid < N) {
-      for (int q = 0; q < 9; ++q) { cams[tid].R[q] = b.R[9 * (c0 + tid) + q]; cams[tid].K[q] = b.K[9 * (c0 + tid) + q]; }
-      for (int q = 0; q < 3; ++q) cams[tid].T[q] = b.T[3 * (c0 + tid) + q];
+      CamS& c = cams[tid];
+      for (int q = 0; q < 9; ++q) { c.R[q] = b.R[9 * (c0 + tid) + q]; c.K[q] = b.K[9 * (c0 + tid) + q]; }
+      for (int q = 0; q < 3; ++q) c.T[q] = b.T[3 * (c0 + tid) + q];
+      c.f = c.K[0];
+      c.fy = (c.K[4] / c.K[0]) * c.K[0];
+      c.affine = c.K[6] == 0.0 && c.K[7] == 0.0 && c.K[8] == 1.0;
     }
     // cached parameter length (v3d_metricbundle.h:37-45)
     {
-      double v[64];
-#pragma unroll
-      for (int t = 0; t < 64; ++t) v[t] = 0.0;
+      double v = 0.0;
       for (int j = tid; j < M; j += NT) {
-        const double* X = b.X + 3 * (size_t)(pt0 + j);
-        v[0] += X[0] * X[0] + X[1] * X[1] + X[2] * X[2];
+        const double* X = Xc + 3 * (size_t)(pt0 + j);
+        v += X[0] * X[0] + X[1] * X[1] + X[2] * X[2];
       }
       if (tid < N) {
         const double* T = b.T + 3 * (size_t)(c0 + tid);
-        v[0] += T[0] * T[0] + T[1] * T[1] + T[2] * T[2] + 3.0;
+        v += T[0] * T[0] + T[1] * T[1] + T[2] * T[2] + 3.0;
       }
-      const double s = block_sum64<NT>(v, red);
+      const double s = block_sum<NT>(v, red);
       if (tid == 0) {
         sc[6] = sqrt(s);
         sc[1] = 1e-3;   // lambda of a new optimizer object
         sc[2] = 2.0;    // _nu
-        si[1] = 0; si[2] = 1; si[5] = V3DBA_STATUS_TIMEOUT; si[7] = 0;
+        si[1] = 0; si[5] = V3DBA_STATUS_TIMEOUT; si[7] = 0;
       }
       __syncthreads();
     }
     int it = 0;
     for (it = 0; it < o.max_iter; ++it) {
-      if (si[2]) {
-        // ---- pass REL: weights, cost, gradient, max diagonal ----
-        double v[64];
+      // Sums of one pass over the points.  mode 0: the first iteration's linearisation, for the
+      // initial lambda (diagonal of U beside the gradient); mode 1: the damped reduced system.
+      // After a rejected step the parameters, and so the weights and sums, are the same again.
+      for (int mode = it == 0 ? 0 : 1; mode < 2; ++mode) {
+        const double lam = sc[1];
+        double acc[L::kPairs][2], err = 0.0, gbmax = 0.0, vdmax = -1e30;
 #pragma unroll
-        for (int t = 0; t < 64; ++t) v[t] = 0.0;
-        double gbmax = 0.0, vdmax = -1e30;
-        for (int j = tid; j < M; j += NT) {
-          const int g = pt0 + j;
-          const int o0 = b.ptr[g], n = b.ptr[g + 1] - o0;
-          const double X[3] = {b.X[3 * (size_t)g], b.X[3 * (size_t)g + 1], b.X[3 * (size_t)g + 2]};
-          double V0 = 0, V3 = 0, V5 = 0, gb[3] = {0, 0, 0};
-          for (int t = 0; t < n; ++t) {
-            const int k = o0 + t;
-            double A[2][6], B[2][3], r[2], e[2];
-            lin_obs(cams, X, b, k, 1.0, A, B, r, e);
-            const double wk = huber_weight(thr, e);
-            b.w[k] = wk;
-            v[0] += wk * wk * (e[0] * e[0] + e[1] * e[1]);
-            r[0] *= wk; r[1] *= wk;
+        for (int t = 0; t < L::kPairs; ++t) acc[t][0] = acc[t][1] = 0.0;
+        Track<NC> tr = load_track<NC>(b, Xc, pt0, M, 32 * wid + lane);
+        for (int ch = wid; ch < chunks; ch += NW) {
+          const double X[3] = {tr.X[0], tr.X[1], tr.X[2]};
+          const int o0 = tr.o0, n = tr.n;
+          const bool twice = tr.twice;
+          double V[6] = {0, 0, 0, 0, 0, 0}, gb[3] = {0, 0, 0}, B[NC][2][3], r[NC][2];
+          // no branch on the presence of a camera: the cameras' chains of divisions and roots overlap
 #pragma unroll
-            for (int rr = 0; rr < 2; ++rr) {
+          for (int c = 0; c < NC; ++c) {
+            if (c >= N) {
 #pragma unroll
-              for (int q = 0; q < 6; ++q) A[rr][q] *= wk;
-#pragma unroll
-              for (int q = 0; q < 3; ++q) B[rr][q] *= wk;
-              V0 += B[rr][0] * B[rr][0];
-              V3 += B[rr][1] * B[rr][1];
-              V5 += B[rr][2] * B[rr][2];
-#pragma unroll
-              for (int q = 0; q < 3; ++q) gb[q] += B[rr][q] * r[rr];
+              for (int q = 0; q < 3; ++q) B[c][0][q] = B[c][1][q] = 0.0;
+              r[c][0] = r[c][1] = 0.0;
+              continue;
             }
-            const int c = b.cam[k];
+            const bool has = (tr.mask >> c) & 1u;
+            ObsLin ol;
+            project_obs(cams[c], X, tr.m[c].x, tr.m[c].y, ol);
+            const double w = huber_weight(thr, ol.e);
+            if (has) b.w[o0 + (int)((tr.slot >> (4 * c)) & 15u)] = w;
+            weigh(ol, w, r[c]);
+            if (!has) ol.P[0] = ol.P[1] = ol.P[2] = ol.P[3] = r[c][0] = r[c][1] = 0.0;
+            err += r[c][0] * r[c][0] + r[c][1] * r[c][1];
+            point_block(cams[c], ol, B[c]);
+            double A[2][6];
+            camera_block(ol, A);
+            add_point(B[c], r[c], V, gb);
+            store_a(Aw + c * 6 * kTileLd, lane, A);
+          }
+          if (tr.mask) {
+            gbmax = fmax(gbmax, fmax(fabs(gb[0]), fmax(fabs(gb[1]), fabs(gb[2]))));
+            vdmax = fmax(vdmax, fmax(V[0], fmax(V[3], V[5])));
+          }
+          tr = load_track<NC>(b, Xc, pt0, M, 32 * (ch + NW) + lane);   // in flight during the products
+          // without the elimination (mode 0) the same product is U, and its right-hand side the gradient
+          double vi[6] = {0, 0, 0, 0, 0, 0}, q[3], det;
+          bool ok = true;
+          if (mode == 1) {
+            ok = invert_point(V, lam, vi, &det);
+            if (!ok && !isfinite(det)) {   // a point at infinity contributes nothing
+              const double zero2[2][6] = {};
 #pragma unroll
-            for (int cc = 0; cc < kMaxCams; ++cc) {
-              if (cc != c) continue;
-#pragma unroll
-              for (int a = 0; a < 6; ++a) {
-                v[1 + 6 * cc + a] += A[0][a] * r[0] + A[1][a] * r[1];
-                v[1 + 24 + 6 * cc + a] += A[0][a] * A[0][a] + A[1][a] * A[1][a];
+              for (int c = 0; c < NC; ++c) {
+                if (c < N) store_a(Aw + c * 6 * kTileLd, lane, zero2);
+                r[c][0] = r[c][1] = 0.0;
               }
             }
           }
-          if (n > 0) {
-            gbmax = fmax(gbmax, fmax(fabs(gb[0]), fmax(fabs(gb[1]), fabs(gb[2]))));
-            vdmax = fmax(vdmax, fmax(V0, fmax(V3, V5)));
+          mul_sym3(vi, gb, q);
+          int pr = 0;
+#pragma unroll
+          for (int i = 0; i < NC; ++i) {
+            double BV[2][3];
+            mul_sym3(vi, B[i][0], BV[0]);
+            mul_sym3(vi, B[i][1], BV[1]);
+#pragma unroll
+            for (int l = i; l < NC; ++l, ++pr) {
+              if (l >= N || (l != i && mode == 0)) continue;
+              store_z(Zw, Aw + l * 6 * kTileLd, lane, BV, B[l], i == l, ok);
+              if (i == l) {
+                const double e0 = r[i][0] - (B[i][0][0] * q[0] + B[i][0][1] * q[1] + B[i][0][2] * q[2]);
+                const double e1 = r[i][1] - (B[i][1][0] * q[0] + B[i][1][1] * q[1] + B[i][1][2] * q[2]);
+                store_row(Zw, 6, lane, ok ? e0 : 0.0, ok ? e1 : 0.0);
+                store_row(Zw, 7, lane, r[i][0], r[i][1]);
+              }
+              __syncwarp();
+              tile_product(Aw + i * 6 * kTileLd, Zw, zrow, i == l ? 8 : 6, lane, acc[pr]);
+              __syncwarp();
+            }
+          }
+          // tracks that name a camera twice: their observation pairs one per round and point
+          if (__any_sync(0xffffffffu, twice)) {
+            double vi[6] = {0, 0, 0, 0, 0, 0}, q[3] = {0, 0, 0};
+            bool ok = false, dead = false;
+            const int nt = twice ? n : 0;
+            {
+              double V2[6] = {0, 0, 0, 0, 0, 0}, gb2[3] = {0, 0, 0}, det;
+              for (int t = 0; t < nt; ++t) {
+                const int k = o0 + t;
+                const CamS& cm = cams[b.cam[k]];
+                ObsLin ol;
+                double rr[2], Bt[2][3];
+                project_obs(cm, X, b.meas[2 * (size_t)k], b.meas[2 * (size_t)k + 1], ol);
+                const double w = huber_weight(thr, ol.e);
+                b.w[k] = w;
+                err += w * w * (ol.e[0] * ol.e[0] + ol.e[1] * ol.e[1]);
+                weigh(ol, w, rr);
+                point_block(cm, ol, Bt);
+                add_point(Bt, rr, V2, gb2);
+              }
+              if (twice) {
+                gbmax = fmax(gbmax, fmax(fabs(gb2[0]), fmax(fabs(gb2[1]), fabs(gb2[2]))));
+                vdmax = fmax(vdmax, fmax(V2[0], fmax(V2[3], V2[5])));
+                ok = invert_point(V2, lam, vi, &det);
+                dead = mode == 1 && !ok && !isfinite(det);
+                mul_sym3(vi, gb2, q);
+              }
+            }
+#pragma unroll 1
+            for (int i = 0; i < N; ++i)
+#pragma unroll 1
+              for (int l = i; l < N; ++l) {
+                if (mode == 0 && l != i) continue;
+                double* Ac = Aw + i * 6 * kTileLd;
+                int t = 0, u = -1;
+                for (;;) {
+                  // the lane's next pair (t, u) of an observation in camera i with one in camera l; the
+                  // diagonal's U term and gradient come with t == u (mode 0 has only those)
+                  bool have = false;
+                  while (!have) {
+                    if (++u >= nt) { u = 0; ++t; }
+                    if (t >= nt) break;
+                    have = b.cam[o0 + t] == i && b.cam[o0 + u] == l && (mode == 1 || t == u);
+                  }
+                  if (!__any_sync(0xffffffffu, have)) break;
+                  double At[2][6] = {}, Z[8][2] = {};
+                  if (have && !dead) {
+                    double Au[2][6], Bt[2][3], Bu[2][3], rt[2], ru[2], BV[2][3];
+                    ObsLin ol;
+                    project_obs(cams[i], X, b.meas[2 * (size_t)(o0 + t)], b.meas[2 * (size_t)(o0 + t) + 1], ol);
+                    weigh(ol, b.w[o0 + t], rt);
+                    point_block(cams[i], ol, Bt);
+                    camera_block(ol, At);
+                    project_obs(cams[l], X, b.meas[2 * (size_t)(o0 + u)], b.meas[2 * (size_t)(o0 + u) + 1], ol);
+                    weigh(ol, b.w[o0 + u], ru);
+                    point_block(cams[l], ol, Bu);
+                    camera_block(ol, Au);
+                    mul_sym3(vi, Bt[0], BV[0]);
+                    mul_sym3(vi, Bt[1], BV[1]);
+                    for (int rr = 0; rr < 2; ++rr) {
+                      double P[2];
+                      for (int cc = 0; cc < 2; ++cc)
+                        P[cc] = ((t == u && rr == cc) ? 1.0 : 0.0) -
+                                (mode == 1 ? BV[rr][0] * Bu[cc][0] + BV[rr][1] * Bu[cc][1] + BV[rr][2] * Bu[cc][2] : 0.0);
+                      const bool use = mode == 0 || ok;
+                      for (int a = 0; a < 6; ++a) Z[a][rr] = use ? P[0] * Au[0][a] + P[1] * Au[1][a] : 0.0;
+                      if (t == u) {
+                        if (mode == 1 && ok) Z[6][rr] = rt[rr] - (Bt[rr][0] * q[0] + Bt[rr][1] * q[1] + Bt[rr][2] * q[2]);
+                        Z[7][rr] = rt[rr];
+                      }
+                    }
+                  }
+                  store_a(Ac, lane, At);
+                  for (int a = 0; a < 8; ++a) store_row(Zw, a, lane, Z[a][0], Z[a][1]);
+                  __syncwarp();
+                  double add[2] = {0.0, 0.0};
+                  tile_product(Ac, Zw, zrow, 8, lane, add);
+                  const int at = i * NC - i * (i - 1) / 2 + (l - i);
+#pragma unroll
+                  for (int pr = 0; pr < L::kPairs; ++pr)
+                    if (pr == at) { acc[pr][0] += add[0]; acc[pr][1] += add[1]; }
+                  __syncwarp();
+                }
+              }
           }
         }
-        const double s = block_sum64<NT>(v, red);
-        if (tid == 0) sc[0] = s;
-        else if (tid <= 24) ga[tid - 1] = s;
-        else if (tid <= 48) udiag[tid - 25] = s;
+        // the warps' sums, in warp order
+        __syncwarp();
+#pragma unroll
+        for (int t = 0; t < L::kPairs; ++t)
+          *reinterpret_cast<double2*>(Aw + t * 64 + (lane >> 2) * 8 + 2 * (lane & 3)) = make_double2(acc[t][0], acc[t][1]);
+        const double errs = block_sum<NT>(err, red);
         const double gm = block_max<NT>(gbmax, red);
         const double vm = block_max<NT>(vdmax, red);
-        if (tid == 0) {
-          double gmax = gm;
-          for (int a = 0; a < 6 * N; ++a) gmax = fmax(gmax, fabs(ga[a]));
-          sc[7] = gmax;
-          if (gmax < o.grad_thr) { si[5] = V3DBA_STATUS_CONVERGED; si[1] = 1; }
-          if (it == 0) {
-            if (b.init_cost) b.init_cost[p] = sc[0];
-            if (!si[1]) {
-              double md = vm;
-              for (int a = 0; a < 6 * N; ++a) md = fmax(md, udiag[a]);
-              sc[1] = o.tau * md;
+        for (int e = tid; e < L::kPairs * 64; e += NT) {
+          double s = 0.0;
+          for (int w = 0; w < NW; ++w) s += dyn[w * L::kWarp + e];
+          int i = 0, t = e >> 6;
+          while (t >= NC - i) { t -= NC - i; ++i; }
+          const int l = i + t, a = (e >> 3) & 7, c = e & 7;
+          if (a >= 6 || l >= N) continue;
+          // S_il[a][c] is element (6l + c, 6i + a); only the lower triangle is stored
+          if (c < 6) {
+            if (mode == 0) { if (i == l && a == c) udiag[6 * i + a] = s; }
+            else if (i != l || c >= a) S[(6 * l + c) * LD + 6 * i + a] = s + ((i == l && a == c) ? lam : 0.0);
+          } else if (i == l) {
+            if (c == 7) ga[6 * i + a] = s;
+            else if (mode == 1) rhs[6 * i + a] = s;
+          }
+        }
+        __syncthreads();
+        if (wid == 0) {
+          double gx = lane < 6 * N ? fabs(ga[lane]) : 0.0, dx = (mode == 0 && lane < 6 * N) ? udiag[lane] : -1e30;
+          gx = warp_max(gx);
+          dx = warp_max(dx);
+          if (lane == 0) {
+            sc[0] = errs;
+            if (fmax(gx, gm) < o.grad_thr) { si[5] = V3DBA_STATUS_CONVERGED; si[1] = 1; }
+            if (mode == 0) {
+              if (b.init_cost) b.init_cost[p] = errs;
+              if (!si[1]) sc[1] = o.tau * fmax(dx, vm);
             }
           }
         }
         __syncthreads();
         if (si[1]) break;
       }
-      // ---- pass SCHUR: one camera-pair block per round ----
+      if (si[1]) break;
       const double lam = sc[1];
-      for (int i = 0; i < N; ++i)
-        for (int l = i; l < N; ++l) {
-          double v[64];
-#pragma unroll
-          for (int t = 0; t < 64; ++t) v[t] = 0.0;
-          for (int j = tid; j < M; j += NT) {
-            const int g = pt0 + j;
-            const int o0 = b.ptr[g], n = b.ptr[g + 1] - o0;
-            const double X[3] = {b.X[3 * (size_t)g], b.X[3 * (size_t)g + 1], b.X[3 * (size_t)g + 2]};
-            double vi[6], gb[3], q[3];
-            if (!point_elim(cams, X, b, o0, n, lam, vi, gb, q)) continue;
-            for (int t = 0; t < n; ++t) {
-              if (b.cam[o0 + t] != i) continue;
-              double A[2][6], B[2][3], r[2], W[6][3], Tm[6][3];
-              lin_obs(cams, X, b, o0 + t, b.w[o0 + t], A, B, r, nullptr);
-              wt_of(A, B, vi, W, Tm);
-              if (i == l) {
-#pragma unroll
-                for (int a = 0; a < 6; ++a) {
-#pragma unroll
-                  for (int c = 0; c < 6; ++c) v[a * 6 + c] += A[0][a] * A[0][c] + A[1][a] * A[1][c];
-                  v[36 + a] += A[0][a] * r[0] + A[1][a] * r[1] - (W[a][0] * q[0] + W[a][1] * q[1] + W[a][2] * q[2]);
-                }
-              }
-              for (int u = 0; u < n; ++u) {
-                if (b.cam[o0 + u] != l) continue;
-                double A2[2][6], B2[2][3], r2[2], W2[6][3], T2[6][3];
-                lin_obs(cams, X, b, o0 + u, b.w[o0 + u], A2, B2, r2, nullptr);
-                wt_of(A2, B2, vi, W2, T2);
-#pragma unroll
-                for (int a = 0; a < 6; ++a)
-#pragma unroll
-                  for (int c = 0; c < 6; ++c)
-                    v[a * 6 + c] -= Tm[a][0] * W2[c][0] + Tm[a][1] * W2[c][1] + Tm[a][2] * W2[c][2];
-              }
-            }
-          }
-          const double s = block_sum64<NT>(v, red);
-          if (tid < 36) {
-            // S_il[a][c] is element (6l + c, 6i + a); only the lower triangle is stored
-            const int a = tid / 6, c = tid % 6;
-            if (i != l || c >= a) S[(6 * l + c) * kMaxN + 6 * i + a] = s + ((i == l && a == c) ? lam : 0.0);
-          } else if (tid < 42 && i == l) {
-            rhs[6 * i + tid - 36] = s;
-          }
-          __syncthreads();
-        }
-      // ---- warp 0: Cholesky of the reduced system and solve ----
-      if (tid < 32) {
-        const int n6 = 6 * N;
-        bool ok = true;
-        for (int k = 0; k < n6; ++k) {
-          __syncwarp();
-          const double d = S[k * kMaxN + k];
-          if (!(d > 0.0)) ok = false;
-          const double sd = d > 0.0 ? sqrt(d) : 1.0;
-          __syncwarp();
-          if (tid == 0) S[k * kMaxN + k] = sd;
-          for (int r = k + 1 + tid; r < n6; r += 32) S[r * kMaxN + k] /= sd;
-          __syncwarp();
-          for (int r = k + 1 + tid; r < n6; r += 32)
-            for (int c = k + 1; c <= r; ++c) S[r * kMaxN + c] -= S[r * kMaxN + k] * S[c * kMaxN + k];
-        }
+      if (wid == 0) {
+        const bool ok = warp_solve<NC>(S, rhs, da, colb, 6 * N);
+        if (lane == 0) si[3] = ok ? 0 : 1;
         __syncwarp();
-        if (tid == 0) {
-          si[3] = ok ? 0 : 1;
-          if (ok) {
-            for (int r = 0; r < n6; ++r) {
-              double s = rhs[r];
-              for (int c = 0; c < r; ++c) s -= S[r * kMaxN + c] * da[c];
-              da[r] = s / S[r * kMaxN + r];
-            }
-            for (int r = n6 - 1; r >= 0; --r) {
-              double s = da[r];
-              for (int c = r + 1; c < n6; ++c) s -= S[c * kMaxN + r] * da[c];
-              da[r] = s / S[r * kMaxN + r];
-            }
-          }
+        if (ok && lane < N) {   // trial cameras
+          CamS c = cams[lane];
+          const double* d = da + 6 * lane;
+          c.T[0] += d[0]; c.T[1] += d[1]; c.T[2] += d[2];
+          rotate_update(d + 3, c.R);
+          tcams[lane] = c;
         }
       }
       __syncthreads();
       if (!si[3]) {
-        // trial cameras
-        if (tid < N) {
-          CamS c = cams[tid];
-          const double* d = da + 6 * tid;
-          c.T[0] += d[0]; c.T[1] += d[1]; c.T[2] += d[2];
-          rotate_update(d + 3, c.R);
-          tcams[tid] = c;
-        }
-        __syncthreads();
-        // ---- pass STEP: point back-substitution, trial points, trial cost ----
-        double v[64];
-#pragma unroll
-        for (int t = 0; t < 64; ++t) v[t] = 0.0;
+        // ---- points: back-substitution, trial points, trial cost with frozen weights ----
+        double nerr = 0.0, d2 = 0.0, dg = 0.0;
         for (int j = tid; j < M; j += NT) {
-          const int g = pt0 + j;
+          const size_t g = (size_t)(pt0 + j);
           const int o0 = b.ptr[g], n = b.ptr[g + 1] - o0;
-          const double X[3] = {b.X[3 * (size_t)g], b.X[3 * (size_t)g + 1], b.X[3 * (size_t)g + 2]};
-          double vi[6], gb[3], q[3];
-          double db[3] = {0, 0, 0};
-          if (point_elim(cams, X, b, o0, n, lam, vi, gb, q)) {
-            double acc[3] = {gb[0], gb[1], gb[2]};
-            for (int t = 0; t < n; ++t) {
-              double A[2][6], B[2][3], r[2], W[6][3], Tm[6][3];
-              lin_obs(cams, X, b, o0 + t, b.w[o0 + t], A, B, r, nullptr);
-              wt_of(A, B, vi, W, Tm);
-              const double* d = da + 6 * b.cam[o0 + t];
-#pragma unroll
-              for (int c = 0; c < 3; ++c)
-                acc[c] -= W[0][c] * d[0] + W[1][c] * d[1] + W[2][c] * d[2] + W[3][c] * d[3] + W[4][c] * d[4] + W[5][c] * d[5];
-            }
-            db[0] = vi[0] * acc[0] + vi[1] * acc[1] + vi[2] * acc[2];
-            db[1] = vi[1] * acc[0] + vi[3] * acc[1] + vi[4] * acc[2];
-            db[2] = vi[2] * acc[0] + vi[4] * acc[1] + vi[5] * acc[2];
-            v[1] += db[0] * db[0] + db[1] * db[1] + db[2] * db[2];
-            v[2] += db[0] * gb[0] + db[1] * gb[1] + db[2] * gb[2];
-          }
-          const double Xn[3] = {X[0] + db[0], X[1] + db[1], X[2] + db[2]};
-          b.Xt[3 * (size_t)g] = Xn[0];
-          b.Xt[3 * (size_t)g + 1] = Xn[1];
-          b.Xt[3 * (size_t)g + 2] = Xn[2];
+          const double X[3] = {Xc[3 * g], Xc[3 * g + 1], Xc[3 * g + 2]};
+          double V[6] = {0, 0, 0, 0, 0, 0}, gb[3] = {0, 0, 0}, s[3] = {0, 0, 0}, vi[6], db[3] = {0, 0, 0}, det;
           for (int t = 0; t < n; ++t) {
             const int k = o0 + t;
             const int c = b.cam[k];
-            Cam cm;
+            const double2 m = *reinterpret_cast<const double2*>(b.meas + 2 * (size_t)k);
+            const CamS& cm = cams[c];
+            ObsLin ol;
+            double r[2], B[2][3];
+            project_obs(cm, X, m.x, m.y, ol);
+            weigh(ol, b.w[k], r);
+            point_block(cm, ol, B);
+            add_point(B, r, V, gb);
+            // A da = P (dT + omega x v)
+            const double* d = da + 6 * c;
+            const double t0 = d[0] + (d[4] * ol.v[2] - d[5] * ol.v[1]);
+            const double t1 = d[1] + (d[5] * ol.v[0] - d[3] * ol.v[2]);
+            const double t2 = d[2] + (d[3] * ol.v[1] - d[4] * ol.v[0]);
+            const double a0 = ol.P[0] * t0 + ol.P[1] * t2, a1 = ol.P[2] * t1 + ol.P[3] * t2;
 #pragma unroll
-            for (int qq = 0; qq < 9; ++qq) cm.R[qq] = tcams[c].R[qq];
+            for (int q = 0; q < 3; ++q) s[q] += B[0][q] * a0 + B[1][q] * a1;
+          }
+          if (invert_point(V, lam, vi, &det)) {
 #pragma unroll
-            for (int qq = 0; qq < 3; ++qq) cm.T[qq] = tcams[c].T[qq];
-#pragma unroll
-            for (int qq = 0; qq < 9; ++qq) cm.K[qq] = tcams[c].K[qq];
-            double XX[3], e[2];
-            residual<kModelStd>(cm, Xn, b.meas[2 * k], b.meas[2 * k + 1], XX, e);
+            for (int q = 0; q < 3; ++q) s[q] = gb[q] - s[q];
+            mul_sym3(vi, s, db);
+            d2 += db[0] * db[0] + db[1] * db[1] + db[2] * db[2];
+            dg += db[0] * gb[0] + db[1] * gb[1] + db[2] * gb[2];
+          }
+          const double Xn[3] = {X[0] + db[0], X[1] + db[1], X[2] + db[2]};
+          Xt[3 * g] = Xn[0];
+          Xt[3 * g + 1] = Xn[1];
+          Xt[3 * g + 2] = Xn[2];
+          for (int t = 0; t < n; ++t) {
+            const int k = o0 + t;
+            const double2 m = *reinterpret_cast<const double2*>(b.meas + 2 * (size_t)k);
+            ObsLin ol;
+            project_obs(tcams[b.cam[k]], Xn, m.x, m.y, ol);
             const double wk = b.w[k];
-            v[0] += wk * wk * (e[0] * e[0] + e[1] * e[1]);
+            nerr += wk * wk * (ol.e[0] * ol.e[0] + ol.e[1] * ol.e[1]);
           }
         }
-        const double s = block_sum64<NT>(v, red);
-        if (tid < 3) sc[3 + tid] = s;
-        __syncthreads();
-        if (tid == 0) {
-          double d2 = sc[4], dg = sc[5];
-          for (int a = 0; a < 6 * N; ++a) { d2 += da[a] * da[a]; dg += da[a] * ga[a]; }
-          sc[4] = d2;
-          si[4] = 0;
-          if (sqrt(d2) < o.upd_thr * (sc[6] + o.upd_thr)) {
-            si[5] = V3DBA_STATUS_SMALL_UPDATE;
-            si[1] = 1;
-          } else {
-            const double rho = (sc[0] - sc[3]) / (sc[1] * d2 + dg);
-            si[4] = rho > 0.0 ? 1 : 0;
+        nerr = block_sum<NT>(nerr, red);
+        d2 = block_sum<NT>(d2, red);
+        dg = block_sum<NT>(dg, red);
+        if (wid == 0) {
+          const double dl = lane < 6 * N ? da[lane] : 0.0, gl = lane < 6 * N ? ga[lane] : 0.0;
+          d2 += warp_sum(dl * dl);
+          dg += warp_sum(dl * gl);
+          if (lane == 0) {
+            si[4] = 0;
+            if (sqrt(d2) < o.upd_thr * (sc[6] + o.upd_thr)) {
+              si[5] = V3DBA_STATUS_SMALL_UPDATE;
+              si[1] = 1;
+            } else {
+              const double rho = (sc[0] - nerr) / (lam * d2 + dg);
+              if (rho > 0.0) {
+                const double r = 2.0 * rho - 1.0;
+                sc[1] = fmax(lam * fmax(1.0 / 3.0, 1.0 - r * r * r), 1e-10);
+                si[4] = 1;
+              }
+            }
           }
         }
-        __syncthreads();
-        if (si[1]) break;
       } else if (tid == 0) {
         si[4] = 0;
       }
       __syncthreads();
+      if (si[1]) break;
       if (si[4]) {
         if (tid < N) cams[tid] = tcams[tid];
-        for (int j = tid; j < M; j += NT) {
-          const size_t g = pt0 + j;
-          b.X[3 * g] = b.Xt[3 * g];
-          b.X[3 * g + 1] = b.Xt[3 * g + 1];
-          b.X[3 * g + 2] = b.Xt[3 * g + 2];
-        }
-      }
-      if (tid == 0) {
-        if (si[4]) {
-          const double rho = (sc[0] - sc[3]) / (sc[1] * sc[4] + sc[5]);
-          const double r = 2.0 * rho - 1.0;
-          double lam2 = sc[1] * fmax(1.0 / 3.0, 1.0 - r * r * r);
-          if (lam2 < 1e-10) lam2 = 1e-10;
-          sc[1] = lam2;
-          sc[2] = 2.0;
-          si[2] = 1;
-        } else {
-          sc[1] *= sc[2];
-          sc[2] *= 2.0;
-          si[2] = 0;
-          si[7]++;
-        }
+        double* const was = const_cast<double*>(Xc);
+        Xc = Xt;
+        Xt = was;
+        if (tid == 0) sc[2] = 2.0;
+      } else if (tid == 0) {
+        sc[1] *= sc[2];
+        sc[2] *= 2.0;
+        si[7]++;
       }
       __syncthreads();
     }
     // write back
+    if (Xc != b.X)
+      for (int e = tid; e < 3 * M; e += NT) b.X[3 * (size_t)pt0 + e] = Xc[3 * (size_t)pt0 + e];
     if (tid < N) {
       for (int q = 0; q < 9; ++q) b.R[9 * (c0 + tid) + q] = cams[tid].R[q];
       for (int q = 0; q < 3; ++q) b.T[3 * (c0 + tid) + q] = cams[tid].T[q];
@@ -523,10 +741,11 @@ struct v3dba_batch_s {
   std::vector<void*> allocs;
   std::vector<int> h_cam_off, h_n_cams, h_pt_off, h_n_pts, h_order, h_size;
   int total_cams = 0, total_pts = 0, total_obs = 0;
+  int max_cams = 0;               // cameras of the largest problem
   double* d_init = nullptr;       // initial R, T, X (for reset)
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-  int small_threads = 64, large_threads = 128;   // autotuned block sizes
+  int small_threads = 0, large_threads = 0;   // block sizes: set or autotuned, else 0 (default_threads)
   int split = 0;                  // problems [0, split) of the order use large_threads
 };
 
@@ -568,24 +787,42 @@ void batch_free(v3dba_batch_t h) {
   delete h;
 }
 
+struct BatchKernel {
+  void (*fn)(BatchDev, BatchOpts, int, int);
+  size_t smem;
+};
+template <int NT, int NC>
+BatchKernel batch_kernel_of() {
+  return {k_batched_lm<NT, NC>, sizeof(double) * (NT / 32) * BatchLay<NC>::kWarp};
+}
+// Triplets (three cameras, the usual problem) have their own instances: a fourth camera costs four
+// more camera pairs of accumulators and a third more shared memory per warp.
+BatchKernel batch_kernel(int threads, int max_cams) {
+  if (max_cams <= 3)
+    return threads == 64 ? batch_kernel_of<64, 3>() : threads == 128 ? batch_kernel_of<128, 3>() : batch_kernel_of<256, 3>();
+  return threads == 64 ? batch_kernel_of<64, 4>() : threads == 128 ? batch_kernel_of<128, 4>() : batch_kernel_of<256, 4>();
+}
+
+// Threads per problem of a batch that sets no schedule.  A problem's passes take time in inverse
+// proportion to its warps, but the 256-thread instance runs one block per SM where the others keep 12
+// warps.  Measured (4 iterations, 50-800 points; ms with 64 / 128 / 256 threads): 61 problems 0.50 /
+// 0.29 / 0.17, 300: 0.61 / 0.34 / 0.26, 600: 0.73 / 0.39 / 0.46, 1200: 0.78 / 0.68 / 0.87, 4096: 2.19 /
+// 2.21 / 2.85 and, with 20-90 points, 0.58 / 0.75 / 1.60.
+int default_threads(int count, int sms) { return count <= 2 * sms ? 256 : count <= 8 * sms ? 128 : 64; }
+
 int launch_range(v3dba_batch_t h, int threads, int first, int last, const BatchOpts& o) {
   if (last <= first) return V3DBA_OK;
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (threads == 0) threads = default_threads(last - first, sms);
   V3DBA_CUDA_TRY(cudaMemsetAsync(h->d.queue, 0, sizeof(unsigned), h->stream));
+  const BatchKernel k = batch_kernel(threads, h->max_cams);
+  V3DBA_CUDA_TRY(cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem));
   int per_sm = 1;
-  if (threads == 64) {
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batched_lm<64>, 64, 0);
-  } else if (threads == 128) {
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batched_lm<128>, 128, 0);
-  } else {
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batched_lm<256>, 256, 0);
-  }
+  V3DBA_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k.fn, threads, k.smem));
   const int grid = std::max(1, std::min(last - first, sms * std::max(per_sm, 1)));
-  if (threads == 64) k_batched_lm<64><<<grid, 64, 0, h->stream>>>(h->d, o, first, last);
-  else if (threads == 128) k_batched_lm<128><<<grid, 128, 0, h->stream>>>(h->d, o, first, last);
-  else k_batched_lm<256><<<grid, 256, 0, h->stream>>>(h->d, o, first, last);
+  k.fn<<<grid, threads, k.smem, h->stream>>>(h->d, o, first, last);
   V3DBA_LAUNCH_CHECK();
   return V3DBA_OK;
 }
@@ -645,6 +882,7 @@ int v3dba_batch_create(const v3dba_problem* problems, int count, v3dba_batch_t* 
     h->h_cam_off.push_back(co); h->h_n_cams.push_back(q.n_cameras);
     h->h_pt_off.push_back(po); h->h_n_pts.push_back(q.n_points);
     h->h_size.push_back(q.n_measurements);
+    h->max_cams = std::max(h->max_cams, q.n_cameras);
     thr[p] = q.inlier_threshold;
     std::copy(q.R, q.R + 9 * q.n_cameras, R.begin() + 9 * (size_t)co);
     std::copy(q.T, q.T + 3 * q.n_cameras, T.begin() + 3 * (size_t)co);
@@ -1154,6 +1392,7 @@ int triplet_stage_core(int count, const double* R, const double* T, const double
   v3dba_batch_t h = new (std::nothrow) v3dba_batch_s();
   if (!h) return V3DBA_ERR_OUT_OF_MEMORY;
   h->total_cams = 3 * count;
+  h->max_cams = 3;
   h->total_pts = (int)n_slots;
   h->total_obs = (int)n_meas;
   int rc;
@@ -1254,7 +1493,7 @@ int triplet_stage_core(int count, const double* R, const double* T, const double
   bo.grad_thr = 1e-10;
   bo.upd_thr = 1e-10;
   bo.max_iter = o.max_iterations;
-  BTRY(launch_range(h, 128, 0, count, bo));
+  BTRY(launch_range(h, 0, 0, count, bo));
   if (n_trk > 0) {
     k_triplet_scatter<<<(unsigned)((n_trk + 255) / 256), 256, 0, h->stream>>>(h->d, s, d_Xout);
     BLAUNCH();
