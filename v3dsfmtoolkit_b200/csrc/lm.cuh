@@ -62,6 +62,16 @@ struct DevState {
   int* bc_beg = nullptr;    // [nch_blk] range in the pair list
   int* bc_end = nullptr;
   int* blk_bc_ptr = nullptr;  // [nb+1] chunks of block b
+  // Schur complement by groups of points that the same cameras see (FP64 blocks; build_schur_groups):
+  // chunks of points of one group, each with a partial sum for every pair of its cameras
+  int gr_n = 0;               // chunks; 0: the pair lists are used
+  int* gr_desc = nullptr;     // [gr_n][4] first point in gr_pt, points, first partial sum, cameras
+  int* gr_pt = nullptr;       // [M] points in group order
+  unsigned char* gr_rank = nullptr;   // [K] rank of the observation's camera among its track's
+  int* gr_bptr = nullptr;     // [nb+1] partial sums of block b ...
+  int* gr_ent = nullptr;      // ... as indices of DA x DA blocks in gr_part, in chunk order
+  double* gr_part = nullptr;
+  int gr_smem = 0;            // shared memory of a chunk, bytes
   double* part_cc = nullptr;  // camera-chunk partials
   double* part_bc = nullptr;  // block-chunk partials
   // parameters
@@ -107,6 +117,18 @@ struct DevState {
   int relin_blocks_pt = 0, relin_blocks_cam = 0;
   int trial_blocks_pt = 0, trial_blocks_cam = 0, trial_blocks_obs = 0;
 };
+
+// Limits of a chunk of the grouped Schur complement, and its shared memory: G is [3 points, padded to
+// whole DMMA steps][leading dimension], a row per (camera, unknown); the leading dimension is 4 mod 8
+// doubles, so that the 4 x 4 elements of a fragment load lie in different banks.
+constexpr int kGroupPoints = 32;    // points per chunk, fewer where the cameras are many
+constexpr int kGroupTrack = 64;     // observations per point
+constexpr int kGroupRows = 360;     // unknowns of the cameras of a group
+constexpr int kGroupSmem = 72 * 1024;   // three blocks per SM
+__host__ __device__ constexpr int group_ld(int rows) { return (rows + 3) / 8 * 8 + 4; }
+__host__ __device__ constexpr int group_doubles(int points, int rows) {
+  return (3 * points + 3) / 4 * 4 * group_ld(rows) + 8 + 6 * points + (kGroupPoints + 3 * kGroupTrack) / 2;
+}
 
 // Stages of one LM iteration, in launch order.
 enum LmStage {

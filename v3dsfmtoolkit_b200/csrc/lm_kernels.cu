@@ -15,6 +15,7 @@
 // per observation and the point elimination writes no per-observation block at all, against
 // 126 instead of 108 FMAs and one more point-block gather per Schur pair.
 #include <algorithm>
+#include <atomic>
 #include <cstdio>
 
 #include "common.cuh"
@@ -708,6 +709,132 @@ __device__ __forceinline__ void schur_chunks_body(DevState s, double* __restrict
   for (int t = 0; t < SV::VP / 32; ++t) part[(size_t)ch * SV::VP + lane * (SV::VP / 32) + t] = double(acc[t]);
 }
 
+__device__ __forceinline__ void dmma884(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
+}
+
+// FP64 blocks, points grouped by their cameras: one block per chunk of up to 32 points that the same L
+// cameras see.  With (V + lambda I)^-1 = C^-T C^-1 and G_k = A_k^T B_k C^-T, the chunk's part of the
+// whole L x L block matrix is G G^T, G one row per camera unknown and three columns per point, formed in
+// shared memory (observations of a point in the same camera add up first) and multiplied with DMMA.
+// Every observation's blocks are read once per trial instead of once per pair (144 bytes instead of 340
+// times the pairs of its track), the gathers that bound the pair lists: their L2 to L1 traffic was 870
+// MB at 5.8 TB/s (pairs staged through shared memory and multiplied with DMMA reached 9.4 TB/s, and no
+// more).  200 cameras, 50,000 points, 1.8M pairs: 118.6 -> 46.3 us (finish 4.3 -> 8.5); 300 rig poses,
+// 40,000 points, 3.2M pairs (two observations per pose): 118 -> 47 us (5.7 -> 7.0).  Bound by the
+// latency of a chunk (pattern, blocks, product): the DMMAs are 14 us of it.
+constexpr int kGroupThreads = 256;
+template <int DA>
+__global__ void __launch_bounds__(kGroupThreads, DA <= 9 ? 3 : 2) k_schur_groups(DevState s) {
+  pdl_wait();
+  pdl_trigger();
+  using L_ = Lay<DA, 0, double>;
+  extern __shared__ double group_sm[];
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int4 d = reinterpret_cast<const int4*>(s.gr_desc)[blockIdx.x];
+  const int p0 = d.x, np = d.y, e0 = d.z, L = d.w;
+  const int rows = DA * L, ld = group_ld(rows), K = (3 * np + 3) / 4 * 4;
+  double* Gs = group_sm;
+  double* Cs = Gs + K * ld + 8;                          // [np][6] C^-1 (00 10 11 20 21 22)
+  int* first = reinterpret_cast<int*>(Cs + 6 * np);      // [np] first observation of the point
+  int* rank = first + kGroupPoints;                      // [track] rank of the observation's camera
+  int* head = rank + kGroupTrack;                        // [L] first observation in the camera ...
+  int* next = head + kGroupTrack;                        // [track] ... and the next one, or -1
+  if (tid < np) {
+    const int j = s.gr_pt[p0 + tid];
+    first[tid] = s.p_ptr[j];
+    const double lam = *s.d_lambda;
+    double V[L_::SV], c[6] = {0, 0, 0, 0, 0, 0};
+    vload(reinterpret_cast<const double*>(s.p_V) + (size_t)j * L_::SV, V);
+    // A pivot that rounding made negative (a direction no observation sees, lambda below the last bit)
+    // counts by its size: that direction's G is zero to rounding, whatever the sign.
+    const double d0 = V[0] + lam, i0 = rsqrt(fabs(d0)), l10 = V[1] * i0, l20 = V[2] * i0;
+    const double d1 = V[3] + lam - l10 * l10, i1 = rsqrt(fabs(d1)), l21 = (V[4] - l20 * l10) * i1;
+    const double d2 = V[5] + lam - l20 * l20 - l21 * l21, i2 = rsqrt(fabs(d2));
+    // a singular point contributes nothing here and failed in k_point_eliminate; a fixed one neither
+    if (j >= s.d.nnB && isfinite(i0) && isfinite(i1) && isfinite(i2)) {
+      c[0] = i0;
+      c[1] = -l10 * i0 * i1;
+      c[2] = i1;
+      c[3] = -(l20 * i0 + l21 * c[1]) * i2;
+      c[4] = -l21 * i1 * i2;
+      c[5] = i2;
+    }
+#pragma unroll
+    for (int t = 0; t < 6; ++t) Cs[6 * tid + t] = c[t];
+  } else if (tid >= kGroupThreads - kGroupTrack) {       // two other warps: the pattern
+    const int t = tid - (kGroupThreads - kGroupTrack), j = s.gr_pt[p0], k0 = s.p_ptr[j], n = s.p_ptr[j + 1] - k0;
+    rank[t] = t < n ? (int)s.gr_rank[k0 + t] : -1;
+  }
+  for (int e = 3 * np * ld + tid; e < K * ld; e += kGroupThreads) Gs[e] = 0.0;   // the last DMMA step's padding
+  __syncthreads();
+  if (tid < kGroupTrack) {
+    int h = -1, nx = -1;
+    const int mine = rank[tid];
+    for (int u = kGroupTrack - 1; u >= 0; --u) {
+      const int ru = rank[u];
+      if (ru == tid) h = u;
+      if (u > tid && ru == mine) nx = u;
+    }
+    head[tid] = h;
+    next[tid] = nx;
+  }
+  __syncthreads();
+  // one column (of three) of a point's rows in one camera per thread
+  for (int idx = tid; idx < 3 * np * L; idx += kGroupThreads) {
+    const int q = idx / (3 * L), rest = idx - q * 3 * L, sl = rest / 3, u = rest - 3 * sl;
+    const double* c = Cs + 6 * q;
+    const double c0 = u == 0 ? c[0] : u == 1 ? c[1] : c[3], c1 = u == 0 ? 0.0 : u == 1 ? c[2] : c[4], c2 = u == 2 ? c[5] : 0.0;
+    double g[DA];
+#pragma unroll
+    for (int a = 0; a < DA; ++a) g[a] = 0.0;
+    for (int t = head[sl]; t >= 0; t = next[t]) {
+      const size_t k = (size_t)(first[q] + t);
+      double A[L_::SA], B[kSB];
+      vload(reinterpret_cast<const double*>(s.o_A) + k * L_::SA, A);
+      vload(s.o_B + k * kSB, B);
+      const double h0 = B[0] * c0 + B[1] * c1 + B[2] * c2, h1 = B[3] * c0 + B[4] * c1 + B[5] * c2;   // of B_k C^-T
+#pragma unroll
+      for (int a = 0; a < DA; ++a) g[a] += A[a] * h0 + A[DA + a] * h1;
+    }
+    double* out = Gs + (3 * q + u) * ld + DA * sl;
+#pragma unroll
+    for (int a = 0; a < DA; ++a) out[a] = g[a];
+  }
+  __syncthreads();
+  // lower tiles of G G^T, up to three of a tile row at a time (they share the row's fragment)
+  const int T = (rows + 7) / 8, r = lane >> 2, kk = lane & 3;
+  int unit = 0;
+  for (int ti = T - 1; ti >= 0; --ti)
+    for (int tj = 0; tj <= ti; tj += 3, ++unit) {
+      if (unit % (kGroupThreads / 32) != (tid >> 5)) continue;
+      const int nt = min(3, ti - tj + 1);
+      double acc[3][2] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
+      const double* ga = Gs + kk * ld + 8 * ti + r;
+      const double* gb = Gs + kk * ld + 8 * tj + r;
+#pragma unroll 2
+      for (int k = 0; k < K; k += 4, ga += 4 * ld, gb += 4 * ld) {
+        const double a = *ga;
+        dmma884(acc[0], a, gb[0]);
+        if (nt > 1) dmma884(acc[1], a, gb[8]);
+        if (nt > 2) dmma884(acc[2], a, gb[16]);
+      }
+#pragma unroll
+      for (int t = 0; t < 3; ++t) {
+        if (t >= nt) break;
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int R = 8 * ti + r, C = 8 * (tj + t) + 2 * kk + u;
+          if (R >= rows || C > R) continue;
+          const int sr = R / DA, sc = C / DA;
+          s.gr_part[(size_t)(e0 + sr * (sr + 1) / 2 + sc) * (DA * DA) + (R - sr * DA) * DA + (C - sc * DA)] = acc[t][u];
+        }
+      }
+    }
+}
+
 template <int DA, typename Real>
 __global__ void __launch_bounds__(128) k_schur_chunks(DevState s, double* __restrict__ part) {
   pdl_wait();      // the previous stage's writes are visible
@@ -724,7 +851,8 @@ __device__ __forceinline__ void schur_finish_body(DevState s, const double* __re
   using SV = SchurV<DA>;
   constexpr int PER = SV::VP / 32;
   const int lane = threadIdx.x & 31;
-  const int b = bid * 4 + (threadIdx.x >> 5);
+  const bool grouped = !stores_products<Real>() && s.gr_n > 0;
+  const int b = grouped ? bid : bid * 4 + (threadIdx.x >> 5);
   if (b >= s.nb) return;
   const int i = s.b_i[b], l = s.b_l[b];
   // beside rhs_finish in one launch, the identity block of a fixed camera is rhs_finish's alone
@@ -732,9 +860,44 @@ __device__ __forceinline__ void schur_finish_body(DevState s, const double* __re
   double sum[PER];
 #pragma unroll
   for (int t = 0; t < PER; ++t) sum[t] = 0.0;
-  for (int ch = s.blk_bc_ptr[b]; ch < s.blk_bc_ptr[b + 1]; ++ch)
+  if (grouped) {
+    // Grouped points: the four warps take the block's partial sums in turn, four in flight each (a
+    // camera's own block has one per chunk that the camera is in), and add up in warp order.  A partial
+    // sum holds the rows of the later camera; of a camera with itself, the lower triangle.
+    __shared__ double ws[3][SV::VP];
+    const int w = threadIdx.x >> 5;
+    int at[PER];
 #pragma unroll
-    for (int t = 0; t < PER; ++t) sum[t] += part[(size_t)ch * SV::VP + lane + 32 * t];
+    for (int t = 0; t < PER; ++t) {
+      const int e = min(lane + 32 * t, SV::NV - 1), a = e / DA, c = e % DA;
+      at[t] = (i == l && a > c) ? a * DA + c : c * DA + a;
+    }
+    const int e1 = s.gr_bptr[b + 1];
+    for (int e = s.gr_bptr[b] + w; e < e1; e += 16) {
+      double v[4][PER];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const double* p = s.gr_part + (size_t)s.gr_ent[min(e + 4 * u, e1 - 1)] * (DA * DA);
+#pragma unroll
+        for (int t = 0; t < PER; ++t) v[u][t] = p[at[t]];
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int t = 0; t < PER; ++t) sum[t] += e + 4 * u < e1 ? v[u][t] : 0.0;
+    }
+    if (w > 0)
+#pragma unroll
+      for (int t = 0; t < PER; ++t) ws[w - 1][lane + 32 * t] = sum[t];
+    __syncthreads();
+    if (w > 0) return;
+#pragma unroll
+    for (int t = 0; t < PER; ++t) sum[t] += ws[0][lane + 32 * t] + ws[1][lane + 32 * t] + ws[2][lane + 32 * t];
+  } else {
+    for (int ch = s.blk_bc_ptr[b]; ch < s.blk_bc_ptr[b + 1]; ++ch)
+#pragma unroll
+      for (int t = 0; t < PER; ++t) sum[t] += part[(size_t)ch * SV::VP + lane + 32 * t];
+  }
   const double lam = *s.d_lambda;
   const Real* cU = reinterpret_cast<const Real*>(s.c_U) + (size_t)i * L::SU;
   const size_t ld = s.ld;
@@ -1205,6 +1368,20 @@ inline PartLayout part_layout(const DevState& s) {
 
 template <int MODEL, int DA, int DC, typename Real>
 struct Ops {
+  static bool grouped(const DevState& s) { return !stores_products<Real>() && s.gr_n > 0; }
+  static cudaError_t launch_groups(const DevState& s, cudaStream_t st) {
+    // the groups' shared memory, allowed on the current device the first time it is used there
+    static std::atomic<uint64_t> allowed{0};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const uint64_t bit = 1ull << (dev & 63);
+    if (!(allowed.load() & bit)) {
+      const cudaError_t e = cudaFuncSetAttribute(k_schur_groups<DA>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGroupSmem);
+      if (e != cudaSuccess) return e;
+      allowed.fetch_or(bit);
+    }
+    return launch_pdl(k_schur_groups<DA>, dim3(s.gr_n), dim3(kGroupThreads), (size_t)s.gr_smem, st, s);
+  }
   // Launches one stage of the LM iteration (see LmStage in lm.cuh).
   static int stage(DevState& s, int id, int init_lambda, double tau, cudaStream_t st) {
     const PartLayout pl = part_layout<DA, DC>(s);
@@ -1236,12 +1413,17 @@ struct Ops {
         e = launch_pdl(k_point_eliminate<DA, DC, Real>, dim3(bp), dim3(kPtThreads), 0, st, s, s.part + pl.elim);
         break;
       case kStageSchurChunks:
+        if (grouped(s)) {
+          e = launch_groups(s, st);
+          break;
+        }
         if (s.nch_blk == 0) return V3DBA_OK;
         e = launch_pdl(k_schur_chunks<DA, Real>, dim3(cdiv(s.nch_blk, 4)), dim3(128), 0, st, s, s.part_bc);
         break;
       case kStageSchurFinish:
         if (s.nb == 0) return V3DBA_OK;
-        e = launch_pdl(k_schur_finish<DA, Real>, dim3(cdiv(s.nb, 4)), dim3(128), 0, st, s, (const double*)s.part_bc);
+        e = launch_pdl(k_schur_finish<DA, Real>, dim3(grouped(s) ? s.nb : cdiv(s.nb, 4)), dim3(128), 0, st, s,
+                       (const double*)s.part_bc);
         break;
       case kStageRhsChunks:
         if (s.nch_cam == 0) return V3DBA_OK;
@@ -1304,11 +1486,12 @@ struct Ops {
     int rc = stage(s, kStagePointEliminate, 0, 0.0, st);
     if (rc) return rc;
     const PartLayout pl = part_layout<DA, DC>(s);
-    const int g1 = s.nch_blk > 0 ? cdiv(s.nch_blk, 4) : 0, g2 = s.nch_cam > 0 ? cdiv(s.nch_cam, kCamWarps) : 0;
+    if (grouped(s) && (rc = launched(launch_groups(s, st)))) return rc;
+    const int g1 = !grouped(s) && s.nch_blk > 0 ? cdiv(s.nch_blk, 4) : 0, g2 = s.nch_cam > 0 ? cdiv(s.nch_cam, kCamWarps) : 0;
     if (g1 + g2 > 0 && (rc = launched(launch_pdl(k_chunks_merged<DA, DC, Real>, dim3(g1 + g2), dim3(128), 0, st, s,
                                                  g1, g2))))
       return rc;
-    const int f1 = s.nb > 0 ? cdiv(s.nb, 4) : 0, f2 = cdiv(std::max(s.d.N, 1), kCamWarps);
+    const int f1 = grouped(s) ? s.nb : s.nb > 0 ? cdiv(s.nb, 4) : 0, f2 = cdiv(std::max(s.d.N, 1), kCamWarps);
     const int bp = cdiv(std::max(s.d.M, 1), kPtThreads);
     return launched(launch_pdl(k_finish_merged<DA, DC, Real>, dim3(f1 + f2 + (DC > 0 ? 1 : 0)), dim3(128), 0, st, s,
                                f1, f2, (const double*)(s.part + pl.elim), bp));

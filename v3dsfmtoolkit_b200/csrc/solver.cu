@@ -38,6 +38,7 @@ struct v3dba_handle_s {
   std::vector<int> blk_i, blk_l;   // camera-pair blocks (host copy)
   std::vector<uint8_t> tile_nz;    // tile pattern of the dense reduced system
   bool dense_ready = false;
+  bool groups_ready = false;       // build_schur_groups ran (FP64 blocks)
   double* S_dense = nullptr;
   double* x_dense = nullptr;
   double* x_pcg = nullptr;
@@ -201,6 +202,16 @@ int use_pcg(v3dba_handle h) {
   s.x = h->x_pcg;
   s.Sb = h->pcg.Sb;
   s.diag_blk = h->pcg.diag_blk;
+  return V3DBA_OK;
+}
+
+// The grouping of the points for the FP64 blocks' Schur complement: made on first use.
+int use_groups(v3dba_handle h) {
+  if (h->groups_ready) return V3DBA_OK;
+  const DevAlloc alloc = [h](void** q, size_t bytes) { return dalloc(h, reinterpret_cast<char**>(q), bytes); };
+  const int rc = build_schur_groups(h->s, alloc, h->stream);
+  if (rc) return rc;
+  h->groups_ready = true;
   return V3DBA_OK;
 }
 
@@ -714,7 +725,8 @@ extern "C" int v3dba_minimize(v3dba_handle h, const v3dba_options* opts, v3dba_r
   if (learned && !h->precond) return V3DBA_ERR_INVALID_ARGUMENT;
   if (gauge && D.DA != 6) return V3DBA_ERR_UNSUPPORTED;
   {
-    const int rc0 = pcg ? use_pcg(h) : use_dense(h);
+    int rc0 = pcg ? use_pcg(h) : use_dense(h);
+    if (!rc0 && fp64) rc0 = use_groups(h);
     if (rc0) return rc0;
     if (gauge) {
       const int rc1 = use_gnn(h, learned);
@@ -804,6 +816,7 @@ extern "C" int v3dba_minimize(v3dba_handle h, const v3dba_options* opts, v3dba_r
       // the quadratic model is no longer trusted: stop adding FP32 rounding to it
       fp64 = true;
       ops = ops64;
+      if ((rc = use_groups(h))) return rc;
       res->fp64_from_iteration = it;
       relinearize_again = true;
       if (o.verbosity >= 2) printf("v3dba: normal-equation blocks switched to FP64 at iteration %d\n", it);
@@ -843,6 +856,7 @@ extern "C" int v3dba_profile_stages(v3dba_handle h, int precision, int reps, dou
   cudaStream_t st = h->stream;
   int rc;
   if ((rc = use_dense(h))) return rc;
+  if (precision == V3DBA_PRECISION_FP64 && (rc = use_groups(h))) return rc;
   // a valid state for every stage: linearise, damp with tau * max diagonal, build and solve once
   if ((rc = ops->relinearize(s, true, 1e-3, st))) return rc;
   V3DBA_CUDA_TRY(cudaMemsetAsync(s.d_fail, 0, sizeof(int), st));
@@ -917,6 +931,7 @@ extern "C" int v3dba_cholesky_schedule(v3dba_handle h, int* schedule, int* n_lev
 
 namespace v3dba {
 int handle_use_dense(v3dba_handle h) { return use_dense(h); }
+int handle_use_groups(v3dba_handle h) { return use_groups(h); }
 DevState& handle_state(v3dba_handle h) { return h->s; }
 TileChol& handle_chol(v3dba_handle h) { return h->chol; }
 cudaStream_t handle_stream(v3dba_handle h) { return h->stream; }

@@ -17,6 +17,7 @@
 // Only the per-camera and per-block pointers (a few KB) return to the host, for the work
 // chunks and the factorisation plan.
 #include <algorithm>
+#include <cstdlib>
 #include <cstring>
 #include <functional>
 #include <vector>
@@ -216,6 +217,92 @@ __global__ void k_run_starts(const int* __restrict__ flag_scan, const int* __res
   b_start[b] = (int)t;
   b_i[b] = o_cam[pk[q]];
   b_l[b] = o_cam[pm[q]];
+}
+
+// ---- groups of points with the same cameras --------------------------------------------------
+
+// Sort key of a point's camera sequence; tracks without observations come last.
+__global__ void k_track_hash(const int* __restrict__ p_ptr, const int* __restrict__ o_cam, int M, uint32_t* key,
+                             int* max_len) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= M) return;
+  const int k0 = p_ptr[j], k1 = p_ptr[j + 1];
+  uint32_t h = 2166136261u;
+  for (int k = k0; k < k1; ++k) h = (h ^ (uint32_t)o_cam[k]) * 16777619u + (h >> 15);
+  key[j] = k1 > k0 ? h & 0x7fffffffu : 0xffffffffu;
+  if (k1 - k0 > 32) atomicMax(max_len, k1 - k0);   // (shorter tracks need no look)
+}
+
+// flag[t] = 1 where the camera sequence of the t-th point differs from the one before.
+__global__ void k_track_heads(const int* __restrict__ perm, const int* __restrict__ p_ptr, const int* __restrict__ o_cam,
+                              int M, int* flag) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= M) return;
+  bool same = false;
+  if (t > 0) {
+    const int a = perm[t], b = perm[t - 1];
+    const int ka = p_ptr[a], kb = p_ptr[b], n = p_ptr[a + 1] - ka;
+    same = p_ptr[b + 1] - kb == n;
+    for (int q = 0; q < n && same; ++q) same = o_cam[ka + q] == o_cam[kb + q];
+  }
+  flag[t] = same ? 0 : 1;
+}
+
+// {first position, distinct cameras} of every group; a group of empty tracks has none.
+__global__ void k_group_info(const int* __restrict__ flag, const int* __restrict__ gid, const int* __restrict__ perm,
+                             const int* __restrict__ p_ptr, const int* __restrict__ o_cam, int M, int* info) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= M || !flag[t]) return;
+  const int k0 = p_ptr[perm[t]], k1 = p_ptr[perm[t] + 1];
+  int L = 0;
+  for (int k = k0; k < k1; ++k) {
+    bool first = true;
+    for (int m = k0; m < k && first; ++m) first = o_cam[m] != o_cam[k];
+    L += first;
+  }
+  info[2 * gid[t]] = t;
+  info[2 * gid[t] + 1] = L;
+}
+
+// Rank of every observation's camera among the distinct cameras of its track.
+__global__ void k_track_rank(const int* __restrict__ p_ptr, const int* __restrict__ o_cam, const int* __restrict__ o_pt,
+                             int K, unsigned char* rank) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= K) return;
+  const int k0 = p_ptr[o_pt[k]], k1 = p_ptr[o_pt[k] + 1], c = o_cam[k];
+  int below = 0;
+  for (int u = k0; u < k1; ++u) {
+    bool add = o_cam[u] < c;
+    for (int w = k0; w < u && add; ++w) add = o_cam[w] != o_cam[u];
+    below += add;
+  }
+  rank[k] = (unsigned char)below;
+}
+
+// Block index of every camera pair of a chunk (one block of kGroupTrack threads), in the order of the
+// chunk's partial sums: cameras ascending, pair (r, c), r >= c, at r (r + 1) / 2 + c.
+__global__ void __launch_bounds__(kGroupTrack) k_group_blocks(const int* __restrict__ desc, const int* __restrict__ pt,
+                                                              const int* __restrict__ p_ptr, const int* __restrict__ o_cam,
+                                                              const unsigned char* __restrict__ rank,
+                                                              const int* __restrict__ b_i, const int* __restrict__ b_l,
+                                                              int nb, int* key) {
+  __shared__ int distinct[kGroupTrack];
+  const int* d = desc + 4 * blockIdx.x;
+  const int k0 = p_ptr[pt[d[0]]], n = p_ptr[pt[d[0]] + 1] - k0, L = d[3], t = threadIdx.x;
+  if (t < n) distinct[rank[k0 + t]] = o_cam[k0 + t];
+  __syncthreads();
+  for (int e = t; e < L * (L + 1) / 2; e += kGroupTrack) {
+    int r = 0;
+    while ((r + 1) * (r + 2) / 2 <= e) ++r;
+    const int l = distinct[r], i = distinct[e - r * (r + 1) / 2];
+    int lo = 0, hi = nb - 1;   // blocks in (i, l) order
+    while (lo < hi) {
+      const int mid = (lo + hi) / 2;
+      if (b_i[mid] < i || (b_i[mid] == i && b_l[mid] < l)) lo = mid + 1;
+      else hi = mid;
+    }
+    key[d[2] + e] = lo;
+  }
 }
 
 struct Scratch {
@@ -532,6 +619,105 @@ int build_structure_device(const v3dba_problem* p, const DevAlloc& alloc, cudaSt
   V3DBA_CUDA_TRY(cudaMemcpyAsync(S.b_l, S.h_b_l.data(), sizeof(int) * S.h_b_l.size(), cudaMemcpyHostToDevice, st));
   V3DBA_CUDA_TRY(cudaMemcpyAsync(S.b_ptr, S.h_b_ptr.data(), sizeof(int) * S.h_b_ptr.size(), cudaMemcpyHostToDevice, st));
   V3DBA_CUDA_TRY(cudaStreamSynchronize(st));   // the host vectors above must outlive their copies
+  return V3DBA_OK;
+}
+
+int build_schur_groups(DevState& s, const DevAlloc& alloc, cudaStream_t st) {
+  // Points below which the plan costs more than a call saves (about 0.1 ms against 20 us an iteration)
+  constexpr int kMinObs = 65536;
+  s.gr_n = 0;
+  const char* want = std::getenv("V3DBA_SCHUR");
+  const bool force = want && !std::strcmp(want, "groups");
+  const int M = s.d.M, DA = s.d.DA;
+  if ((want && !std::strcmp(want, "pairs")) || M <= 0 || s.nb <= 0 || (!force && s.d.K < kMinObs)) return V3DBA_OK;
+  Scratch sc;
+  sc.st = st;
+  int rc;
+  uint32_t *ka, *kb;
+  int *va, *vb, *flag, *gid, *info;
+  if ((rc = sc.get(&ka, M)) || (rc = sc.get(&kb, M)) || (rc = sc.get(&va, M)) || (rc = sc.get(&vb, M)) ||
+      (rc = sc.get(&flag, M)) || (rc = sc.get(&gid, M + 1)) || (rc = sc.get(&info, 1)))
+    return rc;
+  const int g = cdiv(M, 256);
+  V3DBA_CUDA_TRY(cudaMemsetAsync(info, 0, sizeof(int), st));
+  k_track_hash<<<g, 256, 0, st>>>(s.p_ptr, s.o_cam, M, ka, info);
+  V3DBA_LAUNCH_CHECK();
+  k_iota<<<g, 256, 0, st>>>(va, M);
+  V3DBA_LAUNCH_CHECK();
+  if ((rc = radix_sort(sc, &ka, &va, kb, vb, M, 32, st))) return rc;
+  k_track_heads<<<g, 256, 0, st>>>(va, s.p_ptr, s.o_cam, M, flag);
+  V3DBA_LAUNCH_CHECK();
+  V3DBA_CUDA_TRY(cudaMemcpyAsync(gid, flag, sizeof(int) * M, cudaMemcpyDeviceToDevice, st));
+  V3DBA_CUDA_TRY(cudaMemsetAsync(gid + M, 0, sizeof(int), st));
+  if ((rc = scan_exclusive(sc, gid, M + 1, st))) return rc;
+  int head[2] = {0, 0};
+  V3DBA_CUDA_TRY(cudaMemcpyAsync(&head[0], gid + M, sizeof(int), cudaMemcpyDeviceToHost, st));
+  V3DBA_CUDA_TRY(cudaMemcpyAsync(&head[1], info, sizeof(int), cudaMemcpyDeviceToHost, st));
+  V3DBA_CUDA_TRY(cudaStreamSynchronize(st));
+  const int G = head[0];
+  if (head[1] > kGroupTrack || (!force && (int64_t)4 * G > M)) return V3DBA_OK;
+  if ((rc = sc.get(&info, 2 * (size_t)G))) return rc;
+  k_group_info<<<g, 256, 0, st>>>(flag, gid, va, s.p_ptr, s.o_cam, M, info);
+  V3DBA_LAUNCH_CHECK();
+  std::vector<int> gi(2 * (size_t)G);
+  V3DBA_CUDA_TRY(cudaMemcpyAsync(gi.data(), info, sizeof(int) * 2 * (size_t)G, cudaMemcpyDeviceToHost, st));
+  V3DBA_CUDA_TRY(cudaStreamSynchronize(st));
+  struct Chunk {
+    int first, points, L;
+  };
+  std::vector<Chunk> chunks;
+  int64_t entries = 0;
+  int smem = 0;
+  for (int q = 0; q < G; ++q) {
+    const int L = gi[2 * q + 1], end = q + 1 < G ? gi[2 * q + 2] : M;
+    if (L == 0) continue;
+    if (L * DA > kGroupRows) return V3DBA_OK;
+    int np = kGroupPoints;
+    while (np > 4 && group_doubles(np, L * DA) * (int)sizeof(double) > kGroupSmem) np -= 4;
+    const int pieces = (end - gi[2 * q] + np - 1) / np;   // of nearly equal size
+    for (int c = 0, t = gi[2 * q]; c < pieces; ++c) {
+      const int points = (end - t + pieces - c - 1) / (pieces - c);
+      chunks.push_back({t, points, L});
+      entries += (int64_t)L * (L + 1) / 2;
+      smem = std::max(smem, group_doubles(points, L * DA) * (int)sizeof(double));
+      t += points;
+    }
+  }
+  // A partial sum is written and read back where a pair gathers 340 bytes, and a chunk pays for 8 x 8
+  // tiles and whole DMMA steps: the two are level at about four pairs a sum (200 cameras, pairs against
+  // groups with their finish: 4,000 points 20.7 / 26.6 us, 8,000 points (4.2 pairs a sum) 30.0 / 30.1,
+  // 16,000 points 48.0 / 34.5, 50,000 points 122.9 / 54.8).
+  if (chunks.empty() || entries > 0x3fffffff || (!force && 4 * entries > s.P)) return V3DBA_OK;
+  // the costly chunks first, so that the last ones to run are short
+  std::stable_sort(chunks.begin(), chunks.end(),
+                   [](const Chunk& a, const Chunk& b) { return a.L * a.L * a.points > b.L * b.L * b.points; });
+  std::vector<int> desc;
+  desc.reserve(4 * chunks.size());
+  int e0 = 0;
+  for (const Chunk& c : chunks) {
+    desc.insert(desc.end(), {c.first, c.points, e0, c.L});
+    e0 += c.L * (c.L + 1) / 2;
+  }
+  auto dal = [&](auto** q, size_t n) -> int {
+    using T = typename std::remove_reference<decltype(**q)>::type;
+    return alloc(reinterpret_cast<void**>(q), sizeof(T) * n);
+  };
+  int* key;
+  if ((rc = dal(&s.gr_desc, desc.size())) || (rc = dal(&s.gr_pt, (size_t)M)) || (rc = dal(&s.gr_rank, (size_t)s.d.K)) || (rc = dal(&s.gr_bptr, (size_t)s.nb + 1)) ||
+      (rc = dal(&s.gr_ent, (size_t)entries)) || (rc = dal(&s.gr_part, (size_t)entries * DA * DA)) ||
+      (rc = sc.get(&key, (size_t)entries)))
+    return rc;
+  V3DBA_CUDA_TRY(cudaMemcpyAsync(s.gr_desc, desc.data(), sizeof(int) * desc.size(), cudaMemcpyHostToDevice, st));
+  V3DBA_CUDA_TRY(cudaMemcpyAsync(s.gr_pt, va, sizeof(int) * M, cudaMemcpyDeviceToDevice, st));
+  k_track_rank<<<cdiv(s.d.K, 256), 256, 0, st>>>(s.p_ptr, s.o_cam, s.o_pt, s.d.K, s.gr_rank);
+  V3DBA_LAUNCH_CHECK();
+  k_group_blocks<<<(unsigned)chunks.size(), kGroupTrack, 0, st>>>(s.gr_desc, s.gr_pt, s.p_ptr, s.o_cam, s.gr_rank, s.b_i, s.b_l,
+                                                                  s.nb, key);
+  V3DBA_LAUNCH_CHECK();
+  if ((rc = group_by_key_device(key, (int)entries, s.nb, s.gr_ent, s.gr_bptr, st))) return rc;
+  V3DBA_CUDA_TRY(cudaStreamSynchronize(st));   // `desc` must outlive its copy
+  s.gr_smem = smem;
+  s.gr_n = (int)chunks.size();
   return V3DBA_OK;
 }
 

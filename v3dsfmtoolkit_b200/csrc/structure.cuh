@@ -9,6 +9,8 @@
 
 namespace v3dba {
 
+struct DevState;
+
 // Allocates `bytes` of device memory that the caller owns (the handle's buffers).
 using DevAlloc = std::function<int(void**, size_t)>;
 
@@ -33,6 +35,11 @@ struct DeviceStructure {
 
 // Builds the structure of `p` (validated indices) on the device, on stream `st`.
 int build_structure_device(const v3dba_problem* p, const DevAlloc& alloc, cudaStream_t st, DeviceStructure& S);
+
+// Groups the points of a problem by their cameras (the camera sequence of the track) for the grouped
+// Schur complement and fills the gr_ fields of `s`; leaves gr_n = 0 where the pair lists are the better
+// way.  V3DBA_SCHUR=groups|pairs in the environment forces either where the limits allow it.
+int build_schur_groups(DevState& s, const DevAlloc& alloc, cudaStream_t st);
 
 // Stable grouping of n items by device int keys in [0, nv): perm[t] is the t-th item in key
 // order (input order among equal keys), items ptr[v] .. ptr[v+1]-1 of perm have key v.  perm
