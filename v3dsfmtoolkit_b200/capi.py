@@ -425,15 +425,20 @@ def bundle_point_structure(tracks, n_required=2):
     ptr, pos, view, ids, mpos = _tracks_args(tracks)
     n, K = ptr.size - 1, int(ptr[-1])
     npts, nm = C.c_int(), C.c_int()
-    pts, meas = np.zeros((max(n, 1), 3)), np.zeros((max(K, 1), 2))
-    mid, cv, cp = (np.zeros(max(K, 1), np.int32) for _ in range(3))
-    xs = np.zeros(max(n, 1), np.int32)
+    # the kept tracks' counts, so that the results are written where they stay (a list that the call
+    # refuses has lengths that mean nothing: arrays of the largest size then)
+    length = np.diff(ptr)
+    keep = length >= int(n_required) if n_required >= 0 else np.zeros(n, dtype=bool)
+    valid = n == 0 or (ptr[0] == 0 and int(length.min()) >= 0)
+    M, Kk = (int(np.count_nonzero(keep)), int(length[keep].sum())) if valid else (n, max(K, 0))
+    pts, meas = np.zeros((M, 3)), np.zeros((Kk, 2))
+    mid, cv, cp = (np.zeros(Kk, np.int32) for _ in range(3))
+    xs = np.zeros(M, np.int32)
     check(_lib().v3dba_bundle_point_structure(n, _i(ptr), _d(pos), _i(view), _i(ids), _f32p(mpos), int(n_required),
                                               C.byref(npts), C.byref(nm), _d(pts), _d(meas), _i(mid), _i(cv), _i(cp),
                                               _i(xs)), "v3dba_bundle_point_structure")
-    M, Kk = npts.value, nm.value
-    return dict(points3d=pts[:M].copy(), measurements=meas[:Kk].copy(), measurement_ids=mid[:Kk].copy(),
-                corresponding_view=cv[:Kk].copy(), corresponding_point=cp[:Kk].copy(), xs_indices=xs[:M].copy())
+    return dict(points3d=pts, measurements=meas, measurement_ids=mid, corresponding_view=cv, corresponding_point=cp,
+                xs_indices=xs)
 
 
 def create_point_structure(bps, from_scratch=True, tracks=None):

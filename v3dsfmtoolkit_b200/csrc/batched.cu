@@ -743,6 +743,7 @@ struct v3dba_batch_s {
   int total_cams = 0, total_pts = 0, total_obs = 0;
   int max_cams = 0;               // cameras of the largest problem
   double* d_init = nullptr;       // initial R, T, X (for reset)
+  CallRes res;                    // owns the stream and the events
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   int small_threads = 0, large_threads = 0;   // block sizes: set or autotuned, else 0 (default_threads)
@@ -781,9 +782,7 @@ void batch_free(v3dba_batch_t h) {
     for (void* p : h->allocs) cudaFreeAsync(p, h->stream);
     cudaStreamSynchronize(h->stream);
   }
-  if (h->ev0) cudaEventDestroy(h->ev0);
-  if (h->ev1) cudaEventDestroy(h->ev1);
-  if (h->stream) cudaStreamDestroy(h->stream);
+  h->res.release();
   delete h;
 }
 
@@ -809,6 +808,14 @@ BatchKernel batch_kernel(int threads, int max_cams) {
 // 0.29 / 0.17, 300: 0.61 / 0.34 / 0.26, 600: 0.73 / 0.39 / 0.46, 1200: 0.78 / 0.68 / 0.87, 4096: 2.19 /
 // 2.21 / 2.85 and, with 20-90 points, 0.58 / 0.75 / 1.60.
 int default_threads(int count, int sms) { return count <= 2 * sms ? 256 : count <= 8 * sms ? 128 : 64; }
+
+int batch_resources(v3dba_batch_t h) {
+  const int rc = h->res.acquire();
+  h->stream = h->res.st;
+  h->ev0 = h->res.ev0;
+  h->ev1 = h->res.ev1;
+  return rc;
+}
 
 int launch_range(v3dba_batch_t h, int threads, int first, int last, const BatchOpts& o) {
   if (last <= first) return V3DBA_OK;
@@ -924,12 +931,7 @@ int v3dba_batch_create(const v3dba_problem* problems, int count, v3dba_batch_t* 
   h->split = 0;
   int rc;
 #define BTRY(x) do { if ((rc = (x)) != V3DBA_OK) { batch_free(h); return rc; } } while (0)
-  if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaEventCreate(&h->ev0) != cudaSuccess || cudaEventCreate(&h->ev1) != cudaSuccess) {
-    cudaGetLastError();
-    batch_free(h);
-    return V3DBA_ERR_CUDA;
-  }
+  BTRY(batch_resources(h));
   h->d.count = count;
   BTRY(bupload(h, &h->d.cam_off, h->h_cam_off));
   BTRY(bupload(h, &h->d.n_cams, h->h_n_cams));
@@ -1047,12 +1049,14 @@ int v3dba_batch_minimize(v3dba_batch_t h, const v3dba_options* opts, v3dba_resul
     const int n = h->d.count;
     std::vector<int> st(n), it(n), rj(n);
     std::vector<double> c(n), ic(n), lm(n);
-    V3DBA_CUDA_TRY(cudaMemcpy(st.data(), h->d.status, n * sizeof(int), cudaMemcpyDeviceToHost));
-    V3DBA_CUDA_TRY(cudaMemcpy(it.data(), h->d.iterations, n * sizeof(int), cudaMemcpyDeviceToHost));
-    V3DBA_CUDA_TRY(cudaMemcpy(rj.data(), h->d.rejected, n * sizeof(int), cudaMemcpyDeviceToHost));
-    V3DBA_CUDA_TRY(cudaMemcpy(c.data(), h->d.cost, n * sizeof(double), cudaMemcpyDeviceToHost));
-    V3DBA_CUDA_TRY(cudaMemcpy(ic.data(), h->d.init_cost, n * sizeof(double), cudaMemcpyDeviceToHost));
-    V3DBA_CUDA_TRY(cudaMemcpy(lm.data(), h->d.lambda_out, n * sizeof(double), cudaMemcpyDeviceToHost));
+    if ((rc = copy_down({{st.data(), h->d.status, n * sizeof(int)},
+                         {it.data(), h->d.iterations, n * sizeof(int)},
+                         {rj.data(), h->d.rejected, n * sizeof(int)},
+                         {c.data(), h->d.cost, n * sizeof(double)},
+                         {ic.data(), h->d.init_cost, n * sizeof(double)},
+                         {lm.data(), h->d.lambda_out, n * sizeof(double)}},
+                        h->stream)))
+      return rc;
     for (int p = 0; p < n; ++p) {
       v3dba_result& r = results[p];
       std::memset(&r, 0, sizeof(r));
@@ -1076,10 +1080,11 @@ int v3dba_batch_get_params(v3dba_batch_t h, int index, double* R, double* T, dou
 
 int v3dba_batch_get_all_params(v3dba_batch_t h, double* R, double* T, double* X) {
   if (!h) return V3DBA_ERR_INVALID_ARGUMENT;
-  if (R) V3DBA_CUDA_TRY(cudaMemcpy(R, h->d.R, 9 * (size_t)h->total_cams * sizeof(double), cudaMemcpyDeviceToHost));
-  if (T) V3DBA_CUDA_TRY(cudaMemcpy(T, h->d.T, 3 * (size_t)h->total_cams * sizeof(double), cudaMemcpyDeviceToHost));
-  if (X) V3DBA_CUDA_TRY(cudaMemcpy(X, h->d.X, 3 * (size_t)h->total_pts * sizeof(double), cudaMemcpyDeviceToHost));
-  return V3DBA_OK;
+  std::vector<HostCopy> list;
+  if (R) list.push_back({R, h->d.R, 9 * (size_t)h->total_cams * sizeof(double)});
+  if (T) list.push_back({T, h->d.T, 3 * (size_t)h->total_cams * sizeof(double)});
+  if (X) list.push_back({X, h->d.X, 3 * (size_t)h->total_pts * sizeof(double)});
+  return copy_down(list, h->stream);
 }
 
 int v3dba_batch_autotune(v3dba_batch_t h, const v3dba_options* opts, int* large_threads, int* small_threads,
@@ -1405,14 +1410,9 @@ int triplet_stage_core(int count, const double* R, const double* T, const double
 #define BCUDA(x) do { cudaError_t _e = (x); if (_e != cudaSuccess) { cudaGetLastError(); done(); \
     return _e == cudaErrorMemoryAllocation ? V3DBA_ERR_OUT_OF_MEMORY : V3DBA_ERR_CUDA; } } while (0)
 #define BLAUNCH() do { note_launches(1); BCUDA(cudaPeekAtLastError()); } while (0)
-#define BUP(dst, src, n) do { if ((n) > 0) BCUDA(cudaMemcpyAsync(dst, src, sizeof(*(src)) * (n), cudaMemcpyHostToDevice, h->stream)); } while (0)
-#define BDOWN(dst, src, n) do { if ((n) > 0) BCUDA(cudaMemcpyAsync(dst, src, sizeof(*(src)) * (n), cudaMemcpyDeviceToHost, h->stream)); } while (0)
-  if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaEventCreate(&h->ev0) != cudaSuccess || cudaEventCreate(&h->ev1) != cudaSuccess) {
-    cudaGetLastError();
-    batch_free(h);
-    return V3DBA_ERR_CUDA;
-  }
+#define BUP(dst, src, n) up.push_back({dst, src, sizeof(*(src)) * (n)})
+#define BDOWN(dst, src, n) down.push_back({dst, src, sizeof(*(src)) * (n)})
+  BTRY(batch_resources(h));
   h->d.count = count;
   StageDev s;
   int *d_trk_tri, *d_tptr, *d_trk_off, *d_n_trk_of, *d_view;
@@ -1459,6 +1459,7 @@ int triplet_stage_core(int count, const double* R, const double* T, const double
   BTRY(ar.commit(h->stream));
   trace.mark("alloc", h->stream);
   // inputs: one copy of each caller array
+  std::vector<HostCopy> up;
   BUP(h->d.R, R, 27 * (size_t)count);
   BUP(h->d.T, T, 9 * (size_t)count);
   BUP(d_focal, focal, 3 * (size_t)count);
@@ -1467,6 +1468,7 @@ int triplet_stage_core(int count, const double* R, const double* T, const double
   BUP(d_view, view, n_meas);
   BUP(d_mpos, pos, 2 * n_meas);
   BUP(h->d.order, order.data(), (size_t)count);
+  BTRY(copy_up(up, h->stream));
   trace.mark("upload", h->stream);
   s.n_trk = (int)n_trk;
   s.trk_tri = d_trk_tri;
@@ -1500,6 +1502,7 @@ int triplet_stage_core(int count, const double* R, const double* T, const double
   }
   BCUDA(cudaEventRecord(h->ev1, h->stream));
   trace.mark("kernels", h->stream);
+  std::vector<HostCopy> down;
   BDOWN(verdict_out, s.verdict, (size_t)count);
   BDOWN(npts_out, s.n_surv, (size_t)count);
   BDOWN(status_out, h->d.status, (size_t)count);
@@ -1509,7 +1512,7 @@ int triplet_stage_core(int count, const double* R, const double* T, const double
   BDOWN(T_out, h->d.T, 9 * (size_t)count);
   if (X_out) BDOWN(X_out, d_Xout, 3 * n_trk);
   if (kept_out) BDOWN(kept_out, s.kept, n_meas);
-  BCUDA(cudaStreamSynchronize(h->stream));
+  BTRY(copy_down(down, h->stream));
   trace.mark("download");
   if (device_ms) {
     float ms = 0.f;

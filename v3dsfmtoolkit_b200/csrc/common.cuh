@@ -56,6 +56,41 @@ struct Arena {
   std::vector<Req> req_;
 };
 
+// What a call or handle needs from the driver besides memory: a stream, two timing events and a page of
+// pinned memory.  Creating and destroying them took 2.6-3.2 and 0.9 ms per handle (80 ms and more on a
+// busy host), a multiple of a small adjustment, so a few sets are kept per device for the next call.
+// acquire() takes one from the pool or makes one; release() returns it (its stream must be idle), or
+// destroys it when kCallResKept are kept already.  Any thread may call both; a set has one owner at a
+// time.  The kept sets are destroyed at process exit.
+struct CallRes {
+  cudaStream_t st = nullptr;
+  cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  double* pinned = nullptr;   // kCallResDoubles doubles
+  int dev = -1;
+  int acquire();
+  void release();
+};
+constexpr int kCallResKept = 8;
+constexpr int kCallResDoubles = 32;
+
+// One copy between the caller's memory and the device.
+struct HostCopy {
+  void* dst;
+  const void* src;
+  size_t bytes;
+};
+// Copies device -> caller (down) and waits for it.  Large copies (kRingDown bytes and more) go through a
+// ring of pinned slots: the driver's own path to pageable memory copies with one thread, which also takes
+// the page faults of arrays that the caller has just allocated (42 MB of points into new arrays: 5.2 ms
+// against 0.7 ms on the bus), so a few threads copy from the slots instead (3.0 ms).
+int copy_down(const std::vector<HostCopy>& list, cudaStream_t st);
+// Copies the caller's arrays -> device, from kRingUp bytes on the same way round (67 MB: 6.4 -> 3.3 ms);
+// smaller arrays are often in this thread's cache, and reading them from other cores costs more than it
+// saves (16 MB: 0.8 -> 2.4 ms).  Later work on the stream is ordered after the copies, and the caller's
+// arrays have been read when it returns.
+int copy_up(const std::vector<HostCopy>& list, cudaStream_t st);
+constexpr size_t kRingDown = (size_t)8 << 20, kRingUp = (size_t)32 << 20;
+
 // Allocation-failure injection for tests (v3dba_debug_fail_allocation): true when the device
 // allocation about to be made is to report out-of-memory instead, as a failed cudaMalloc would.
 // Every device allocation of the handle / batch / structure paths asks first.

@@ -1,8 +1,14 @@
 // Host-side helpers shared by the entry points.
 #include <atomic>
 #include <chrono>
+#include <condition_variable>
 #include <cstdlib>
 #include <cstring>
+#include <deque>
+#include <functional>
+#include <mutex>
+#include <system_error>
+#include <thread>
 
 #include "common.cuh"
 
@@ -53,6 +59,352 @@ bool injected_alloc_failure() {
   while (c >= 0 && !g_alloc_countdown.compare_exchange_weak(c, c - 1, std::memory_order_relaxed)) {
   }
   return c == 0;
+}
+
+// ---- call resources and pinned rings kept between calls --------------------------------------------
+
+namespace {
+
+// Pinned slots for large downloads, each with the event of its copy.
+struct Ring {
+  static constexpr int kSlots = 8;
+  static constexpr size_t kSlot = (size_t)2 << 20;
+  char* mem = nullptr;
+  cudaEvent_t ev[kSlots] = {};
+  int dev = -1;
+};
+constexpr int kRingsKept = 2;
+
+void destroy(CallRes& r) {
+  if (r.pinned) cudaFreeHost(r.pinned);
+  if (r.ev0) cudaEventDestroy(r.ev0);
+  if (r.ev1) cudaEventDestroy(r.ev1);
+  if (r.st) cudaStreamDestroy(r.st);
+  r = CallRes();
+}
+void destroy(Ring& r) {
+  if (r.mem) cudaFreeHost(r.mem);
+  for (cudaEvent_t& e : r.ev)
+    if (e) cudaEventDestroy(e);
+  r = Ring();
+}
+
+// Never destroyed itself (other threads may be in a call when the process ends); what it keeps is
+// destroyed by a handler that runs before the CUDA runtime's own, registered after its first use.
+struct Kept {
+  std::mutex m;
+  std::vector<CallRes> res;
+  std::vector<Ring> rings;
+  bool closing = false;
+};
+Kept& kept() {
+  static Kept* k = [] {
+    auto* n = new Kept;
+    cudaFree(nullptr);
+    std::atexit([] {
+      Kept& k2 = kept();
+      std::lock_guard<std::mutex> lock(k2.m);
+      k2.closing = true;
+      for (CallRes& r : k2.res) destroy(r);
+      for (Ring& r : k2.rings) destroy(r);
+      k2.res.clear();
+      k2.rings.clear();
+    });
+    return n;
+  }();
+  return *k;
+}
+
+template <typename T>
+bool take(std::vector<T>& v, int dev, T& out) {
+  for (size_t i = v.size(); i-- > 0;)
+    if (v[i].dev == dev) {
+      out = v[i];
+      v.erase(v.begin() + (long)i);
+      return true;
+    }
+  return false;
+}
+
+int ring_acquire(Ring& r) {
+  int dev = 0;
+  V3DBA_CUDA_TRY(cudaGetDevice(&dev));
+  {
+    Kept& k = kept();
+    std::lock_guard<std::mutex> lock(k.m);
+    if (take(k.rings, dev, r)) return V3DBA_OK;
+  }
+  r.dev = dev;
+  cudaError_t e = cudaMallocHost(reinterpret_cast<void**>(&r.mem), Ring::kSlots * Ring::kSlot);
+  for (int t = 0; t < Ring::kSlots && e == cudaSuccess; ++t) e = cudaEventCreateWithFlags(&r.ev[t], cudaEventDisableTiming);
+  if (e == cudaSuccess) return V3DBA_OK;
+  cudaGetLastError();
+  destroy(r);
+  return V3DBA_ERR_OUT_OF_MEMORY;
+}
+void ring_release(Ring& r) {
+  Kept& k = kept();
+  std::lock_guard<std::mutex> lock(k.m);
+  if ((int)k.rings.size() < kRingsKept && !k.closing) {
+    k.rings.push_back(r);
+    r = Ring();
+  } else {
+    destroy(r);
+  }
+}
+
+}  // namespace
+
+int CallRes::acquire() {
+  int d = 0;
+  V3DBA_CUDA_TRY(cudaGetDevice(&d));
+  {
+    Kept& k = kept();
+    std::lock_guard<std::mutex> lock(k.m);
+    if (take(k.res, d, *this)) return V3DBA_OK;
+  }
+  dev = d;
+  cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaEventCreate(&ev0);
+  if (e == cudaSuccess) e = cudaEventCreate(&ev1);
+  if (e == cudaSuccess) e = cudaMallocHost(reinterpret_cast<void**>(&pinned), kCallResDoubles * sizeof(double));
+  if (e == cudaSuccess) return V3DBA_OK;
+  cudaGetLastError();
+  destroy(*this);
+  return e == cudaErrorMemoryAllocation ? V3DBA_ERR_OUT_OF_MEMORY : V3DBA_ERR_CUDA;
+}
+
+void CallRes::release() {
+  if (!st) return;
+  Kept& k = kept();
+  std::lock_guard<std::mutex> lock(k.m);
+  int same = 0;
+  for (const CallRes& r : k.res) same += r.dev == dev;
+  if (same < kCallResKept && !k.closing) {
+    k.res.push_back(*this);
+    *this = CallRes();
+  } else {
+    destroy(*this);
+  }
+}
+
+namespace {
+
+// A list of copies, the large ones cut into pieces of at most a slot.  The pieces end where a 2 MB page
+// of the caller's memory ends, so that no two threads fault one page.
+struct Pieces {
+  std::vector<HostCopy> p;
+  bool staged = false;
+  Ring ring;
+  cudaError_t err = cudaSuccess;
+
+  Pieces(const std::vector<HostCopy>& list, bool down, cudaStream_t st) {
+    constexpr size_t kPieceMin = (size_t)256 << 10;
+    size_t large = 0;
+    for (const HostCopy& c : list)
+      if (c.bytes >= kPieceMin) large += c.bytes;
+    staged = large >= (down ? kRingDown : kRingUp) && ring_acquire(ring) == V3DBA_OK;
+    for (const HostCopy& c : list) {
+      if (!c.bytes) continue;
+      if (!staged || c.bytes < kPieceMin) {
+        if (err == cudaSuccess)
+          err = cudaMemcpyAsync(c.dst, c.src, c.bytes, down ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice, st);
+        continue;
+      }
+      for (size_t at = 0; at < c.bytes;) {
+        const uintptr_t host = reinterpret_cast<uintptr_t>(down ? c.dst : c.src) + at;
+        const size_t n = std::min(c.bytes - at, Ring::kSlot - (host & (Ring::kSlot - 1)));
+        p.push_back({static_cast<char*>(c.dst) + at, static_cast<const char*>(c.src) + at, n});
+        at += n;
+      }
+    }
+  }
+  ~Pieces() {
+    if (!staged) return;
+    if (err == cudaSuccess) ring_release(ring);
+    else destroy(ring);
+  }
+  char* slot(int i) const { return ring.mem + (size_t)(i % Ring::kSlots) * Ring::kSlot; }
+  cudaEvent_t event(int i) const { return ring.ev[i % Ring::kSlots]; }
+};
+
+// Up to kThreads threads that help a call with its copies.  They are started when a call first asks for
+// help (starting them for every call cost 1 ms and more), serve any number of calls at a time, and end
+// when nobody has asked for kIdle.  Never destroyed (a thread may be asleep in it when the process ends).
+struct Crew {
+  static constexpr int kThreads = 7;
+  static constexpr std::chrono::seconds kIdle{2};
+  struct Job {
+    std::function<void()> work;
+    int wanted = 0, running = 0;
+  };
+  std::mutex m;
+  std::condition_variable asked, left;
+  std::deque<Job*> jobs;
+  int threads = 0, idle = 0;
+
+  static Crew& get() {
+    static Crew* c = new Crew;
+    return *c;
+  }
+  void thread() {
+    std::unique_lock<std::mutex> lock(m);
+    for (;;) {
+      ++idle;
+      const bool job = asked.wait_for(lock, kIdle, [&] { return !jobs.empty(); });
+      --idle;
+      if (!job) {
+        --threads;
+        return;
+      }
+      Job* j = jobs.front();
+      if (--j->wanted == 0) jobs.pop_front();
+      ++j->running;
+      lock.unlock();
+      j->work();
+      lock.lock();
+      if (--j->running == 0) left.notify_all();
+    }
+  }
+  void ask(Job& j, int wanted) {
+    std::lock_guard<std::mutex> lock(m);
+    try {
+      for (int more = std::min(wanted - idle, kThreads - threads); more > 0; --more) {
+        std::thread([this] { thread(); }).detach();
+        ++threads;
+      }
+    } catch (const std::system_error&) {   // fewer, or none
+    }
+    if (threads == 0) return;
+    j.wanted = wanted;
+    jobs.push_back(&j);
+    asked.notify_all();
+  }
+  // Ends the job: who has not begun does not begin, who has is waited for.
+  void end(Job& j) {
+    std::unique_lock<std::mutex> lock(m);
+    if (j.wanted > 0) {
+      j.wanted = 0;
+      jobs.erase(std::remove(jobs.begin(), jobs.end(), &j), jobs.end());
+    }
+    left.wait(lock, [&] { return j.running == 0; });
+  }
+};
+
+// The helpers of one call: they run `work` until it returns, at most until the end of the scope.  They
+// may come late or not at all (busy with other calls, or the system has no threads left): the calling
+// thread takes pieces too whenever it has nothing else to do.
+struct Helpers {
+  Crew::Job job;
+  template <typename F>
+  Helpers(int pieces, F work) {
+    job.work = work;
+    Crew::get().ask(job, std::min({Crew::kThreads, pieces, std::max(1, (int)std::thread::hardware_concurrency() / 2)}));
+  }
+  ~Helpers() { Crew::get().end(job); }
+};
+
+}  // namespace
+
+// In both directions the pieces are taken in order, `arrived` / `done` and the flags only move forward,
+// and every wait ends with the copies before it or with `stop`.
+int copy_down(const std::vector<HostCopy>& list, cudaStream_t st) {
+  Pieces pc(list, true, st);
+  const int n = (int)pc.p.size();
+  cudaError_t& err = pc.err;
+  if (n > 0 && err == cudaSuccess) {
+    std::vector<std::atomic<char>> taken(n);
+    for (auto& t : taken) t.store(0, std::memory_order_relaxed);
+    std::atomic<int> next{0}, arrived{0};
+    std::atomic<bool> stop{false};
+    auto take = [&](int i) {
+      std::memcpy(pc.p[i].dst, pc.slot(i), pc.p[i].bytes);
+      taken[i].store(1, std::memory_order_release);
+    };
+    Helpers helpers(n, [&]() {
+      for (int i; (i = next.fetch_add(1)) < n; take(i))
+        while (arrived.load(std::memory_order_acquire) <= i) {
+          if (stop.load()) return;
+          std::this_thread::yield();
+        }
+    });
+    int issued = 0, a = 0;   // a: arrived
+    while (a < n && err == cudaSuccess) {
+      while (issued < n && issued - a < Ring::kSlots && err == cudaSuccess &&
+             (issued < Ring::kSlots || taken[issued - Ring::kSlots].load(std::memory_order_acquire))) {
+        err = cudaMemcpyAsync(pc.slot(issued), pc.p[issued].src, pc.p[issued].bytes, cudaMemcpyDeviceToHost, st);
+        if (err == cudaSuccess) err = cudaEventRecord(pc.event(issued), st);
+        ++issued;
+      }
+      if (err != cudaSuccess) break;
+      if (a == issued) {   // every slot waits to be taken out of
+        int i = next.load();
+        if (i < a && next.compare_exchange_strong(i, i + 1)) take(i);
+        else std::this_thread::yield();
+        continue;
+      }
+      if ((err = cudaEventSynchronize(pc.event(a))) != cudaSuccess) break;
+      arrived.store(++a, std::memory_order_release);
+    }
+    // who is still at work ends with its piece; pieces that nobody has begun are this thread's
+    if (err != cudaSuccess) stop.store(true);
+    else
+      for (int i; (i = next.fetch_add(1)) < n;) take(i);
+  }
+  if (err == cudaSuccess) err = cudaStreamSynchronize(st);
+  V3DBA_CUDA_TRY(err);
+  return V3DBA_OK;
+}
+
+int copy_up(const std::vector<HostCopy>& list, cudaStream_t st) {
+  Pieces pc(list, false, st);
+  const int n = (int)pc.p.size();
+  cudaError_t& err = pc.err;
+  if (n > 0 && err == cudaSuccess) {
+    std::vector<std::atomic<char>> filled(n);
+    for (auto& t : filled) t.store(0, std::memory_order_relaxed);
+    std::atomic<int> next{0}, done{0};   // done: pieces that have left their slots
+    std::atomic<bool> stop{false};
+    auto fill = [&](int i) {
+      std::memcpy(pc.slot(i), pc.p[i].src, pc.p[i].bytes);
+      filled[i].store(1, std::memory_order_release);
+    };
+    Helpers helpers(n, [&]() {
+      for (int i; (i = next.fetch_add(1)) < n; fill(i))
+        while (done.load(std::memory_order_acquire) + Ring::kSlots <= i) {
+          if (stop.load()) return;
+          std::this_thread::yield();
+        }
+    });
+    int issued = 0, d = 0;
+    while (d < n && err == cudaSuccess) {
+      bool moved = false;
+      if (issued < n && filled[issued].load(std::memory_order_acquire)) {
+        err = cudaMemcpyAsync(pc.p[issued].dst, pc.slot(issued), pc.p[issued].bytes, cudaMemcpyHostToDevice, st);
+        if (err == cudaSuccess) err = cudaEventRecord(pc.event(issued), st);
+        if (err != cudaSuccess) break;
+        ++issued;
+        moved = true;
+      }
+      if (d < issued) {
+        const cudaError_t q = cudaEventQuery(pc.event(d));
+        if (q == cudaSuccess) {
+          done.store(++d, std::memory_order_release);
+          moved = true;
+        } else if (q != cudaErrorNotReady) {
+          err = q;
+        }
+      }
+      if (!moved) {
+        int i = next.load();
+        if (i < n && i < d + Ring::kSlots && next.compare_exchange_strong(i, i + 1)) fill(i);
+        else std::this_thread::yield();
+      }
+    }
+    if (err != cudaSuccess) stop.store(true);
+  }
+  V3DBA_CUDA_TRY(err);
+  return V3DBA_OK;
 }
 
 int Arena::commit(cudaStream_t st) {

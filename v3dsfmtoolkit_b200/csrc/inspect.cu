@@ -180,7 +180,7 @@ extern "C" int v3dba_dense_cholesky_solve(int n, const double* S, const double* 
   for (int r = 0; r < n; ++r)
     for (int c = 0; c <= r; ++c)
       if (S[(size_t)r * n + c] != 0.0) nz[(size_t)(r / 64) * nt + c / 64] = 1;
-  int rc = tile_chol_plan(tc, n, nz);
+  int rc = tile_chol_plan(tc, n, nz, nullptr);
   if (rc) { tile_chol_free(tc); return rc; }
   std::vector<double> full((size_t)tc.ld * tc.n_pad, 0.0);
   for (int c = 0; c < n; ++c) {
@@ -224,7 +224,7 @@ extern "C" int v3dba_dense_cholesky_profile(int n, const double* S, const double
   for (int r = 0; r < n; ++r)
     for (int c = 0; c <= r; ++c)
       if (S[(size_t)r * n + c] != 0.0) nz[(size_t)(r / 64) * nt + c / 64] = 1;
-  int rc = tile_chol_plan(tc, n, nz);
+  int rc = tile_chol_plan(tc, n, nz, nullptr);
   if (rc) { tile_chol_free(tc); return rc; }
   std::vector<double> full((size_t)tc.ld * tc.n_pad, 0.0);
   for (int c = 0; c < n; ++c) {

@@ -188,6 +188,8 @@ struct TileChol {
   int* d_panel_ptr = nullptr;
   int* d_upd_ptr = nullptr;
   double* d_ldiag = nullptr;                    // nt inverted diagonal tiles (L_kk^-1)
+  void* d_plan = nullptr;                       // holds the six arrays above
+  cudaStream_t st = nullptr;                    // the memory's stream
   // Level schedule under a nested-dissection order of the tiles (chol_order.cu).  When it
   // shortens the chain of dependent diagonal factorisations enough, tile_chol_solve runs
   // k_chol_levels with it instead of the column-by-column cluster kernel.
@@ -253,9 +255,12 @@ struct PcgState {
   double* gauge_rows = nullptr;  // [N x 28] per-camera terms of Z^T S Z
   double* gauge_L = nullptr;     // packed Cholesky factor of Z^T S Z and its ok flag
   int* iters = nullptr;
+  cudaStream_t st = nullptr;    // the memory's stream
+  std::vector<void*> mem;
   bool ready = false;
 };
-int pcg_plan(PcgState& ps, const std::vector<int>& b_i, const std::vector<int>& b_l, int N);
+// The device memory of both comes from the stream's pool and is freed on the same stream.
+int pcg_plan(PcgState& ps, const std::vector<int>& b_i, const std::vector<int>& b_l, int N, cudaStream_t st);
 int pcg_alloc(PcgState& ps, int nb, int N, int DA);
 void pcg_free(PcgState& ps);
 // Solves S x = b (b in ps.b, blocks in ps.Sb); iteration count in *ps.iters (device).
@@ -263,7 +268,8 @@ int pcg_solve(PcgState& ps, int N, int DA, bool fp64, double tol, int max_iter, 
               cudaStream_t st);
 
 // Builds the plan from the lower-triangle tile pattern (tile_nz[r*nt+c], r >= c).
-int tile_chol_plan(TileChol& tc, int n, std::vector<uint8_t>& tile_nz);
+// Its device memory comes from the stream's pool and is freed on the same stream.
+int tile_chol_plan(TileChol& tc, int n, std::vector<uint8_t>& tile_nz, cudaStream_t st);
 void tile_chol_free(TileChol& tc);
 // Zeroes the pattern tiles of S (column-major, ld) and sets the padding diagonal to 1.
 int tile_chol_zero(const TileChol& tc, double* S, double* rhs, cudaStream_t st);

@@ -564,7 +564,8 @@ __global__ void k_pcg_precond(const void* Sb, const int* diag_blk, int N, int DA
 
 }  // namespace
 
-int pcg_plan(PcgState& ps, const std::vector<int>& b_i, const std::vector<int>& b_l, int N) {
+int pcg_plan(PcgState& ps, const std::vector<int>& b_i, const std::vector<int>& b_l, int N, cudaStream_t st) {
+  ps.st = st;
   // row structure over both triangles: row i holds (i, l) for every stored block (i, l) and
   // (i, k) for every stored block (k, i) with k < i (transposed)
   std::vector<std::vector<std::pair<int, int>>> rows(N);   // (column, entry code)
@@ -590,25 +591,29 @@ int pcg_plan(PcgState& ps, const std::vector<int>& b_i, const std::vector<int>& 
     rp.push_back((int)rc.size());
     if (diag[i] < 0 || rd[i] < 0) return V3DBA_ERR_INVALID_INPUT;
   }
-  auto up = [](auto** d, const auto& h) -> int {
+  auto up = [&ps, st](auto** d, const auto& h) -> int {
     using T = typename std::remove_reference<decltype(h)>::type::value_type;
     if (injected_alloc_failure()) return V3DBA_ERR_OUT_OF_MEMORY;
-    V3DBA_CUDA_TRY(cudaMalloc(d, sizeof(T) * std::max<size_t>(h.size(), 1)));
-    if (!h.empty()) V3DBA_CUDA_TRY(cudaMemcpy(*d, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice));
+    V3DBA_CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(d), sizeof(T) * std::max<size_t>(h.size(), 1), st));
+    ps.mem.push_back(*d);
+    if (!h.empty()) V3DBA_CUDA_TRY(cudaMemcpyAsync(*d, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice, st));
     return V3DBA_OK;
   };
-  int rc2;
+  int rc2 = ensure_pool();
+  if (rc2) return rc2;
   if ((rc2 = up(&ps.rp, rp)) || (rc2 = up(&ps.rb, rb)) || (rc2 = up(&ps.rc, rc)) || (rc2 = up(&ps.rt, rt)) ||
       (rc2 = up(&ps.rd, rd)) || (rc2 = up(&ps.diag_blk, diag)))
     return rc2;
+  V3DBA_CUDA_TRY(cudaStreamSynchronize(st));   // the host arrays must outlive their copies
   return V3DBA_OK;
 }
 
 int pcg_alloc(PcgState& ps, int nb, int N, int DA) {
   const size_t n = (size_t)N * DA;
-  auto get = [](auto** d, size_t bytes) -> int {
+  auto get = [&ps](auto** d, size_t bytes) -> int {
     if (injected_alloc_failure()) return V3DBA_ERR_OUT_OF_MEMORY;
-    V3DBA_CUDA_TRY(cudaMalloc(d, bytes));
+    V3DBA_CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(d), bytes, ps.st));
+    ps.mem.push_back(*d);
     return V3DBA_OK;
   };
   int rc;
@@ -619,15 +624,14 @@ int pcg_alloc(PcgState& ps, int nb, int N, int DA) {
       (rc = get(&ps.gauge_rows, sizeof(double) * kGaugeTri * (size_t)std::max(N, 1))) ||
       (rc = get(&ps.gauge_L, sizeof(double) * (kGaugeTri + 1))) || (rc = get(&ps.iters, sizeof(int))))
     return rc;
+  V3DBA_CUDA_TRY(cudaStreamSynchronize(ps.st));   // other streams may use it from here on
   ps.b = ps.vec;
   ps.ready = true;
   return V3DBA_OK;
 }
 
 void pcg_free(PcgState& ps) {
-  cudaFree(ps.rp); cudaFree(ps.rb); cudaFree(ps.rc); cudaFree(ps.rt); cudaFree(ps.rd); cudaFree(ps.diag_blk);
-  cudaFree(ps.Sb); cudaFree(ps.Pinv); cudaFree(ps.vec); cudaFree(ps.part); cudaFree(ps.iters);
-  cudaFree(ps.gauge_rows); cudaFree(ps.gauge_L);
+  for (void* p : ps.mem) cudaFreeAsync(p, ps.st);
   ps = PcgState();
 }
 

@@ -1126,7 +1126,7 @@ int system_create(v3dba_precond_set s, int N, const std::vector<int>& b_i, const
   ps.N = N;
   ps.nb = (int)b_i.size();
   int rc;
-  if ((rc = pcg_plan(ps.ps, b_i, b_l, N)) || (rc = pcg_alloc(ps.ps, ps.nb, N, 6)) ||
+  if ((rc = pcg_plan(ps.ps, b_i, b_l, N, s->st)) || (rc = pcg_alloc(ps.ps, ps.nb, N, 6)) ||
       (rc = gnn_graph_build(ps.g, N, b_i, b_l))) {
     system_free(ps);
     return rc;

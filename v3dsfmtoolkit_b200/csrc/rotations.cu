@@ -425,6 +425,7 @@ using namespace v3dba;
 struct v3dba_rotations_s {
   int N = 0, P = 0, full_grid = 1, cur = 0, G = 32;
   double nu = 2.0;
+  CallRes res;               // owns the stream and the events
   cudaStream_t st = nullptr;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   char* arena = nullptr;
@@ -443,9 +444,7 @@ void release(v3dba_rotations h) {
   if (h->arena) cudaFreeAsync(h->arena, h->st);
   if (h->trace) cudaFreeAsync(h->trace, h->st);
   if (h->st) cudaStreamSynchronize(h->st);
-  if (h->e0) cudaEventDestroy(h->e0);
-  if (h->e1) cudaEventDestroy(h->e1);
-  if (h->st) cudaStreamDestroy(h->st);
+  h->res.release();
   delete h;
 }
 
@@ -541,9 +540,10 @@ int v3dba_rotations_create(int n_views, int n_pairs, const double* relative_rota
     }                                                                                                  \
   } while (0)
   TRY(ensure_pool());
-  CTRY(cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking));
-  CTRY(cudaEventCreate(&h->e0));
-  CTRY(cudaEventCreate(&h->e1));
+  TRY(h->res.acquire());
+  h->st = h->res.st;
+  h->e0 = h->res.ev0;
+  h->e1 = h->res.ev1;
   int dev = 0, sms = 148, per_sm = 1;
   CTRY(cudaGetDevice(&dev));
   CTRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -581,12 +581,8 @@ int v3dba_rotations_create(int n_views, int n_pairs, const double* relative_rota
   h->vlist = reinterpret_cast<int*>(b + o_vlist);
   int* keys = reinterpret_cast<int*>(b + o_keys);
   h->state = reinterpret_cast<RotState*>(b + o_state);
-  if (P > 0) {
-    CTRY(cudaMemcpyAsync(h->rel, relative_rotations, 72 * P, cudaMemcpyHostToDevice, h->st));
-    CTRY(cudaMemcpyAsync(h->pairs, view_pairs, 8 * P, cudaMemcpyHostToDevice, h->st));
-  }
+  TRY(copy_up({{h->rel, relative_rotations, 72 * P}, {h->pairs, view_pairs, 8 * P}, {h->R0, rotations, 72 * N}}, h->st));
   if (N > 0) {
-    CTRY(cudaMemcpyAsync(h->R0, rotations, 72 * N, cudaMemcpyHostToDevice, h->st));
     CTRY(cudaMemcpyAsync(h->R[0], h->R0, 72 * N, cudaMemcpyDeviceToDevice, h->st));
   }
   if (P > 0) {

@@ -42,6 +42,7 @@ struct v3dba_handle_s {
   double* S_dense = nullptr;
   double* x_dense = nullptr;
   double* x_pcg = nullptr;
+  CallRes res;                     // owns the stream, the events and the pinned readback area
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   double param_length = 0.0;
@@ -121,13 +122,14 @@ int copy_params(const ParamSet& dst, const ParamSet& src, const v3dba_handle h, 
 int upload_params(v3dba_handle h, const ParamSet& P, const double* K, const double* R, const double* T,
                   const double* dist, const double* X) {
   const Dims& D = h->s.d;
-  cudaStream_t st = h->stream;
-  if (h->nK) V3DBA_CUDA_TRY(cudaMemcpyAsync(P.K, K, sizeof(double) * h->nK, cudaMemcpyHostToDevice, st));
-  V3DBA_CUDA_TRY(cudaMemcpyAsync(P.R, R, sizeof(double) * 9 * D.N, cudaMemcpyHostToDevice, st));
-  V3DBA_CUDA_TRY(cudaMemcpyAsync(P.T, T, sizeof(double) * 3 * D.N, cudaMemcpyHostToDevice, st));
-  if (h->nD) V3DBA_CUDA_TRY(cudaMemcpyAsync(P.dist, dist, sizeof(double) * h->nD, cudaMemcpyHostToDevice, st));
-  V3DBA_CUDA_TRY(cudaMemcpyAsync(P.X, X, sizeof(double) * 3 * D.M, cudaMemcpyHostToDevice, st));
-  V3DBA_CUDA_TRY(cudaStreamSynchronize(st));
+  const int rc = copy_up({{P.K, K, sizeof(double) * h->nK},
+                          {P.R, R, sizeof(double) * 9 * (size_t)D.N},
+                          {P.T, T, sizeof(double) * 3 * (size_t)D.N},
+                          {P.dist, dist, sizeof(double) * h->nD},
+                          {P.X, X, sizeof(double) * 3 * (size_t)D.M}},
+                         h->stream);
+  if (rc) return rc;
+  V3DBA_CUDA_TRY(cudaStreamSynchronize(h->stream));
   return V3DBA_OK;
 }
 
@@ -142,17 +144,14 @@ int upload(v3dba_handle h, T** d, const std::vector<T>& v) {
 
 void free_handle(v3dba_handle h) {
   if (!h) return;
+  tile_chol_free(h->chol);
+  pcg_free(h->pcg);
   if (h->stream) {
     for (void* p : h->allocs) cudaFreeAsync(p, h->stream);
     cudaStreamSynchronize(h->stream);
   }
-  tile_chol_free(h->chol);
-  pcg_free(h->pcg);
   gnn_graph_free(h->gnn);
-  if (h->h_scalars) cudaFreeHost(h->h_scalars);
-  if (h->ev0) cudaEventDestroy(h->ev0);
-  if (h->ev1) cudaEventDestroy(h->ev1);
-  if (h->stream) cudaStreamDestroy(h->stream);
+  h->res.release();
   delete h;
 }
 
@@ -161,7 +160,7 @@ int use_dense(v3dba_handle h) {
   DevState& s = h->s;
   if (!h->dense_ready) {
     std::vector<uint8_t> nz = h->tile_nz;
-    int rc = tile_chol_plan(h->chol, std::max(s.n, 1), nz);
+    int rc = tile_chol_plan(h->chol, std::max(s.n, 1), nz, h->stream);
     if (rc) return rc;
     if (!h->S_dense && (rc = dalloc(h, &h->S_dense, (size_t)h->chol.ld * h->chol.n_pad))) return rc;
     if (!h->x_dense && (rc = dalloc(h, &h->x_dense, (size_t)h->chol.n_pad))) return rc;
@@ -183,7 +182,7 @@ int use_pcg(v3dba_handle h) {
   DevState& s = h->s;
   if (!h->pcg.ready) {
     pcg_free(h->pcg);   // a retry after a failed attempt (out of memory) starts clean
-    int rc = pcg_plan(h->pcg, h->blk_i, h->blk_l, s.d.N);
+    int rc = pcg_plan(h->pcg, h->blk_i, h->blk_l, s.d.N, h->stream);
     if (!rc) rc = pcg_alloc(h->pcg, s.nb, s.d.N, s.d.DA);
     if (rc) {
       pcg_free(h->pcg);
@@ -404,10 +403,11 @@ int v3dba_create(const v3dba_problem* p, v3dba_handle* out) {
 #define CTRY(x) do { cudaError_t _e = (x); if (_e != cudaSuccess) { cudaGetLastError(); free_handle(h); \
     return _e == cudaErrorMemoryAllocation ? V3DBA_ERR_OUT_OF_MEMORY : V3DBA_ERR_CUDA; } } while (0)
 
-  CTRY(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
-  CTRY(cudaEventCreate(&h->ev0));
-  CTRY(cudaEventCreate(&h->ev1));
-  CTRY(cudaMallocHost(&h->h_scalars, 24 * sizeof(double)));
+  TRY(h->res.acquire());
+  h->stream = h->res.st;
+  h->ev0 = h->res.ev0;
+  h->ev1 = h->res.ev1;
+  h->h_scalars = h->res.pinned;
 
   trace.mark("stream");
   DeviceStructure ds;
@@ -573,13 +573,13 @@ int v3dba_get_params(v3dba_handle h, double* K, double* R, double* T, double* di
   const Dims& D = h->s.d;
   const ParamSet& P = h->s.cur;
   cudaStream_t st = h->stream;
-  if (K && h->nK) V3DBA_CUDA_TRY(cudaMemcpyAsync(K, P.K, sizeof(double) * h->nK, cudaMemcpyDeviceToHost, st));
-  if (R) V3DBA_CUDA_TRY(cudaMemcpyAsync(R, P.R, sizeof(double) * 9 * D.N, cudaMemcpyDeviceToHost, st));
-  if (T) V3DBA_CUDA_TRY(cudaMemcpyAsync(T, P.T, sizeof(double) * 3 * D.N, cudaMemcpyDeviceToHost, st));
-  if (dist && h->nD) V3DBA_CUDA_TRY(cudaMemcpyAsync(dist, P.dist, sizeof(double) * h->nD, cudaMemcpyDeviceToHost, st));
-  if (X) V3DBA_CUDA_TRY(cudaMemcpyAsync(X, P.X, sizeof(double) * 3 * D.M, cudaMemcpyDeviceToHost, st));
-  V3DBA_CUDA_TRY(cudaStreamSynchronize(st));
-  return V3DBA_OK;
+  std::vector<HostCopy> list;
+  if (K) list.push_back({K, P.K, sizeof(double) * h->nK});
+  if (R) list.push_back({R, P.R, sizeof(double) * 9 * D.N});
+  if (T) list.push_back({T, P.T, sizeof(double) * 3 * D.N});
+  if (dist) list.push_back({dist, P.dist, sizeof(double) * h->nD});
+  if (X) list.push_back({X, P.X, sizeof(double) * 3 * D.M});
+  return copy_down(list, st);
 }
 
 int v3dba_reset_params(v3dba_handle h) {

@@ -466,11 +466,11 @@ int build_structure_device(const v3dba_problem* p, const DevAlloc& alloc, cudaSt
   int *d_view, *d_point;
   double* d_meas;
   if ((rc = sc.get(&d_view, K)) || (rc = sc.get(&d_point, K)) || (rc = sc.get(&d_meas, 2 * (size_t)K))) return rc;
-  if (K > 0) {
-    V3DBA_CUDA_TRY(cudaMemcpyAsync(d_view, p->view, sizeof(int) * K, cudaMemcpyHostToDevice, st));
-    V3DBA_CUDA_TRY(cudaMemcpyAsync(d_point, p->point, sizeof(int) * K, cudaMemcpyHostToDevice, st));
-    V3DBA_CUDA_TRY(cudaMemcpyAsync(d_meas, p->measurements, sizeof(double) * 2 * K, cudaMemcpyHostToDevice, st));
-  }
+  if ((rc = copy_up({{d_view, p->view, sizeof(int) * (size_t)K},
+                     {d_point, p->point, sizeof(int) * (size_t)K},
+                     {d_meas, p->measurements, sizeof(double) * 2 * (size_t)K}},
+                    st)))
+    return rc;
   const int gK = cdiv(std::max(K, 1), 256);
   // 1. point-major permutation
   uint32_t *ka, *kb;
@@ -751,32 +751,36 @@ using namespace v3dba;
 
 namespace {
 
-// A stream and a scratch list for one standalone call; the stream is synchronised and destroyed
-// at the end.
+// A stream and a scratch list for one standalone call; the stream is synchronised and given back at
+// the end.
 struct CallScope {
+  CallRes res;
   cudaStream_t st = nullptr;
   Scratch* sc = nullptr;
+  int open() {
+    int rc = ensure_pool();
+    if (rc || (rc = res.acquire())) return rc;
+    st = res.st;
+    return V3DBA_OK;
+  }
   ~CallScope() {
     if (sc) delete sc;   // frees the buffers on the stream
-    if (st) {
-      cudaStreamSynchronize(st);
-      cudaStreamDestroy(st);
-    }
+    if (st) cudaStreamSynchronize(st);
+    res.release();
   }
 };
 
+// Room for n values on the device, and their copy on the list when h is given.
 template <typename T>
-int up_copy(Scratch& sc, T** d, const T* h, size_t n, cudaStream_t st) {
-  int rc = sc.get(d, n);
-  if (rc) return rc;
-  if (n && h) V3DBA_CUDA_TRY(cudaMemcpyAsync(*d, h, sizeof(T) * n, cudaMemcpyHostToDevice, st));
-  return V3DBA_OK;
+int up_add(Scratch& sc, std::vector<HostCopy>& list, T** d, const T* h, size_t n) {
+  const int rc = sc.get(d, n);
+  if (!rc && n && h) list.push_back({*d, h, sizeof(T) * n});
+  return rc;
 }
 
 template <typename T>
-int down_copy(T* h, const T* d, size_t n, cudaStream_t st) {
-  if (n && h) V3DBA_CUDA_TRY(cudaMemcpyAsync(h, d, sizeof(T) * n, cudaMemcpyDeviceToHost, st));
-  return V3DBA_OK;
+void down_add(std::vector<HostCopy>& list, T* h, const T* d, size_t n) {
+  if (n && h) list.push_back({h, d, sizeof(T) * n});
 }
 
 bool valid_track_ptr(const int* ptr, int n) {
@@ -799,7 +803,8 @@ extern "C" int v3dba_bundle_point_structure(int n_tracks, const int* track_ptr, 
   if ((n_tracks && !track_pos) || (K && (!meas_view || !meas_id || !meas_pos))) return V3DBA_ERR_INVALID_ARGUMENT;
   NvtxRange nvtx("v3dba_bundle_point_structure");
   CallScope cs;
-  V3DBA_CUDA_TRY(cudaStreamCreateWithFlags(&cs.st, cudaStreamNonBlocking));
+  const int open_rc = cs.open();
+  if (open_rc) return open_rc;
   cs.sc = new Scratch();
   cs.sc->st = cs.st;
   Scratch& sc = *cs.sc;
@@ -808,13 +813,14 @@ extern "C" int v3dba_bundle_point_structure(int n_tracks, const int* track_ptr, 
   double *d_pos, *o_pts, *o_meas;
   float* d_mpos;
   int rc;
-  if ((rc = up_copy(sc, &d_ptr, track_ptr, (size_t)n_tracks + 1, st)) ||
-      (rc = up_copy(sc, &d_pos, track_pos, 3 * (size_t)n_tracks, st)) ||
-      (rc = up_copy(sc, &d_view, meas_view, (size_t)K, st)) || (rc = up_copy(sc, &d_id, meas_id, (size_t)K, st)) ||
-      (rc = up_copy(sc, &d_mpos, meas_pos, 2 * (size_t)K, st)) || (rc = sc.get(&d_keep, (size_t)n_tracks + 1)) ||
+  std::vector<HostCopy> up;
+  if ((rc = up_add(sc, up, &d_ptr, track_ptr, (size_t)n_tracks + 1)) ||
+      (rc = up_add(sc, up, &d_pos, track_pos, 3 * (size_t)n_tracks)) ||
+      (rc = up_add(sc, up, &d_view, meas_view, (size_t)K)) || (rc = up_add(sc, up, &d_id, meas_id, (size_t)K)) ||
+      (rc = up_add(sc, up, &d_mpos, meas_pos, 2 * (size_t)K)) || (rc = sc.get(&d_keep, (size_t)n_tracks + 1)) ||
       (rc = sc.get(&d_cnt, (size_t)n_tracks + 1)) || (rc = sc.get(&o_pts, 3 * (size_t)n_tracks)) ||
       (rc = sc.get(&o_meas, 2 * (size_t)K)) || (rc = sc.get(&o_ids, (size_t)K)) || (rc = sc.get(&o_view, (size_t)K)) ||
-      (rc = sc.get(&o_point, (size_t)K)) || (rc = sc.get(&o_xs, (size_t)n_tracks)))
+      (rc = sc.get(&o_point, (size_t)K)) || (rc = sc.get(&o_xs, (size_t)n_tracks)) || (rc = copy_up(up, st)))
     return rc;
   k_bps_flags<<<cdiv(n_tracks + 1, 256), 256, 0, st>>>(d_ptr, n_tracks, n_required, d_keep, d_cnt);
   V3DBA_LAUNCH_CHECK();
@@ -829,11 +835,14 @@ extern "C" int v3dba_bundle_point_structure(int n_tracks, const int* track_ptr, 
   V3DBA_CUDA_TRY(cudaMemcpyAsync(&tot[1], d_cnt + n_tracks, sizeof(int), cudaMemcpyDeviceToHost, st));
   V3DBA_CUDA_TRY(cudaStreamSynchronize(st));
   const int M = tot[0], Kk = tot[1];
-  if ((rc = down_copy(points3d, o_pts, 3 * (size_t)M, st)) || (rc = down_copy(measurements, o_meas, 2 * (size_t)Kk, st)) ||
-      (rc = down_copy(measurement_ids, o_ids, (size_t)Kk, st)) || (rc = down_copy(corresponding_view, o_view, (size_t)Kk, st)) ||
-      (rc = down_copy(corresponding_point, o_point, (size_t)Kk, st)) || (rc = down_copy(xs_indices, o_xs, (size_t)M, st)))
-    return rc;
-  V3DBA_CUDA_TRY(cudaStreamSynchronize(st));
+  std::vector<HostCopy> down;
+  down_add(down, points3d, o_pts, 3 * (size_t)M);
+  down_add(down, measurements, o_meas, 2 * (size_t)Kk);
+  down_add(down, measurement_ids, o_ids, (size_t)Kk);
+  down_add(down, corresponding_view, o_view, (size_t)Kk);
+  down_add(down, corresponding_point, o_point, (size_t)Kk);
+  down_add(down, xs_indices, o_xs, (size_t)M);
+  if ((rc = copy_down(down, st))) return rc;
   *n_points = M;
   *n_measurements = Kk;
   return V3DBA_OK;
@@ -851,12 +860,14 @@ extern "C" int v3dba_create_point_structure(int from_scratch, int n_points, int 
   if (!track_pos && (from_scratch ? n_points > 0 : n_tracks > 0)) return V3DBA_ERR_INVALID_ARGUMENT;
   NvtxRange nvtx("v3dba_create_point_structure");
   CallScope cs;
-  V3DBA_CUDA_TRY(cudaStreamCreateWithFlags(&cs.st, cudaStreamNonBlocking));
+  const int open_rc = cs.open();
+  if (open_rc) return open_rc;
   cs.sc = new Scratch();
   cs.sc->st = cs.st;
   Scratch& sc = *cs.sc;
   const cudaStream_t st = cs.st;
   int rc;
+  std::vector<HostCopy> up;
   if (from_scratch) {
     const int K = n_measurements, M = n_points;
     if (K && (!measurement_ids || !corresponding_view || !corresponding_point || !meas_view || !meas_id || !meas_pos))
@@ -866,22 +877,24 @@ extern "C" int v3dba_create_point_structure(int from_scratch, int n_points, int 
     int *d_cp, *d_ids, *d_cv, *d_perm, *d_ptr, *o_view, *o_id;
     double* d_meas;
     float* o_mpos;
-    if ((rc = up_copy(sc, &d_cp, corresponding_point, (size_t)K, st)) ||
-        (rc = up_copy(sc, &d_ids, measurement_ids, (size_t)K, st)) ||
-        (rc = up_copy(sc, &d_cv, corresponding_view, (size_t)K, st)) ||
-        (rc = up_copy(sc, &d_meas, measurements, 2 * (size_t)K, st)) || (rc = sc.get(&d_perm, (size_t)K)) ||
+    if ((rc = up_add(sc, up, &d_cp, corresponding_point, (size_t)K)) ||
+        (rc = up_add(sc, up, &d_ids, measurement_ids, (size_t)K)) ||
+        (rc = up_add(sc, up, &d_cv, corresponding_view, (size_t)K)) ||
+        (rc = up_add(sc, up, &d_meas, measurements, 2 * (size_t)K)) || (rc = sc.get(&d_perm, (size_t)K)) ||
         (rc = sc.get(&d_ptr, (size_t)M + 1)) || (rc = sc.get(&o_view, (size_t)K)) || (rc = sc.get(&o_id, (size_t)K)) ||
-        (rc = sc.get(&o_mpos, 2 * (size_t)K)))
+        (rc = sc.get(&o_mpos, 2 * (size_t)K)) || (rc = copy_up(up, st)))
       return rc;
     if ((rc = group_by_key_device(d_cp, K, M, d_perm, d_ptr, st))) return rc;
     if (K > 0) {
       k_cps_gather<<<cdiv(K, 256), 256, 0, st>>>(d_perm, d_meas, d_ids, d_cv, K, o_view, o_id, o_mpos);
       V3DBA_LAUNCH_CHECK();
     }
-    if ((rc = down_copy(track_ptr, d_ptr, (size_t)M + 1, st)) || (rc = down_copy(meas_view, o_view, (size_t)K, st)) ||
-        (rc = down_copy(meas_id, o_id, (size_t)K, st)) || (rc = down_copy(meas_pos, o_mpos, 2 * (size_t)K, st)))
-      return rc;
-    V3DBA_CUDA_TRY(cudaStreamSynchronize(st));
+    std::vector<HostCopy> down;
+    down_add(down, track_ptr, d_ptr, (size_t)M + 1);
+    down_add(down, meas_view, o_view, (size_t)K);
+    down_add(down, meas_id, o_id, (size_t)K);
+    down_add(down, meas_pos, o_mpos, 2 * (size_t)K);
+    if ((rc = copy_down(down, st))) return rc;
     if (M) std::memcpy(track_pos, points3d, sizeof(double) * 3 * (size_t)M);
     return V3DBA_OK;
   }
@@ -899,12 +912,12 @@ extern "C" int v3dba_create_point_structure(int from_scratch, int n_points, int 
   int *d_ptr, *d_xs, *d_off;
   double *d_pts, *d_meas, *d_pos;
   float* d_mpos;
-  if ((rc = up_copy(sc, &d_ptr, (const int*)track_ptr, (size_t)n_tracks + 1, st)) ||
-      (rc = up_copy(sc, &d_xs, xs_indices, (size_t)M, st)) || (rc = sc.get(&d_off, (size_t)M + 1)) ||
-      (rc = up_copy(sc, &d_pts, points3d, 3 * (size_t)M, st)) ||
-      (rc = up_copy(sc, &d_meas, measurements, 2 * (size_t)n_measurements, st)) ||
-      (rc = up_copy(sc, &d_pos, (const double*)track_pos, 3 * (size_t)n_tracks, st)) ||
-      (rc = up_copy(sc, &d_mpos, (const float*)meas_pos, 2 * (size_t)KT, st)))
+  if ((rc = up_add(sc, up, &d_ptr, (const int*)track_ptr, (size_t)n_tracks + 1)) ||
+      (rc = up_add(sc, up, &d_xs, xs_indices, (size_t)M)) || (rc = sc.get(&d_off, (size_t)M + 1)) ||
+      (rc = up_add(sc, up, &d_pts, points3d, 3 * (size_t)M)) ||
+      (rc = up_add(sc, up, &d_meas, measurements, 2 * (size_t)n_measurements)) ||
+      (rc = up_add(sc, up, &d_pos, (const double*)track_pos, 3 * (size_t)n_tracks)) ||
+      (rc = up_add(sc, up, &d_mpos, (const float*)meas_pos, 2 * (size_t)KT)) || (rc = copy_up(up, st)))
     return rc;
   k_cps_lengths<<<cdiv(M + 1, 256), 256, 0, st>>>(d_ptr, d_xs, M, d_off);
   V3DBA_LAUNCH_CHECK();
@@ -913,8 +926,8 @@ extern "C" int v3dba_create_point_structure(int from_scratch, int n_points, int 
     k_cps_inplace<<<cdiv(M, 128), 128, 0, st>>>(d_ptr, d_xs, d_off, M, d_pts, d_meas, d_pos, d_mpos);
     V3DBA_LAUNCH_CHECK();
   }
-  if ((rc = down_copy(track_pos, d_pos, 3 * (size_t)n_tracks, st)) || (rc = down_copy(meas_pos, d_mpos, 2 * (size_t)KT, st)))
-    return rc;
-  V3DBA_CUDA_TRY(cudaStreamSynchronize(st));
-  return V3DBA_OK;
+  std::vector<HostCopy> down;
+  down_add(down, track_pos, d_pos, 3 * (size_t)n_tracks);
+  down_add(down, meas_pos, d_mpos, 2 * (size_t)KT);
+  return copy_down(down, st);
 }

@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(256) k_chol_zero(double* __restrict__ S, int l
 
 // ---- host ----------------------------------------------------------------------------------
 
-int tile_chol_plan(TileChol& tc, int n, std::vector<uint8_t>& nz) {
+int tile_chol_plan(TileChol& tc, int n, std::vector<uint8_t>& nz, cudaStream_t st) {
   tile_chol_free(tc);   // a plan retried after a failed one (out of memory) starts clean
   const int nt = (n + TB - 1) / TB;
   tc.n = n;
@@ -288,21 +288,25 @@ int tile_chol_plan(TileChol& tc, int n, std::vector<uint8_t>& nz) {
     for (int c = 0; c < nt && c <= r; ++c)
       if (r == nt || nz[r * nt + c]) tc.h_tiles.push_back(r * (nt + 1) + c);
 
-  auto up = [](int** d, const std::vector<int>& h) -> int {
-    if (injected_alloc_failure()) return V3DBA_ERR_OUT_OF_MEMORY;
-    V3DBA_CUDA_TRY(cudaMalloc(d, sizeof(int) * std::max<size_t>(h.size(), 1)));
-    if (!h.empty()) V3DBA_CUDA_TRY(cudaMemcpy(*d, h.data(), sizeof(int) * h.size(), cudaMemcpyHostToDevice));
-    return V3DBA_OK;
-  };
-  int rc;
-  if ((rc = up(&tc.d_panel_rows, tc.h_panel_rows))) return rc;
-  if ((rc = up(&tc.d_panel_ptr, tc.h_panel_ptr))) return rc;
-  if ((rc = up(&tc.d_upd_r, tc.h_upd_r))) return rc;
-  if ((rc = up(&tc.d_upd_c, tc.h_upd_c))) return rc;
-  if ((rc = up(&tc.d_upd_ptr, tc.h_upd_ptr))) return rc;
-  if ((rc = up(&tc.d_tiles, tc.h_tiles))) return rc;
+  // the index arrays in one allocation and one copy
+  tc.st = st;
+  int rc = ensure_pool();
+  if (rc) return rc;
+  const std::vector<int>* src[6] = {&tc.h_panel_rows, &tc.h_panel_ptr, &tc.h_upd_r, &tc.h_upd_c, &tc.h_upd_ptr, &tc.h_tiles};
+  int** dst[6] = {&tc.d_panel_rows, &tc.d_panel_ptr, &tc.d_upd_r, &tc.d_upd_c, &tc.d_upd_ptr, &tc.d_tiles};
+  std::vector<int> all;
+  size_t at[6];
+  for (int t = 0; t < 6; ++t) {
+    at[t] = all.size();
+    all.insert(all.end(), src[t]->begin(), src[t]->end());
+  }
   if (injected_alloc_failure()) return V3DBA_ERR_OUT_OF_MEMORY;
-  V3DBA_CUDA_TRY(cudaMalloc(&tc.d_ldiag, sizeof(double) * (size_t)nt * TB * TB));
+  V3DBA_CUDA_TRY(cudaMallocAsync(&tc.d_plan, sizeof(int) * all.size(), st));
+  for (int t = 0; t < 6; ++t) *dst[t] = static_cast<int*>(tc.d_plan) + at[t];
+  V3DBA_CUDA_TRY(cudaMemcpyAsync(tc.d_plan, all.data(), sizeof(int) * all.size(), cudaMemcpyHostToDevice, st));
+  if (injected_alloc_failure()) return V3DBA_ERR_OUT_OF_MEMORY;
+  V3DBA_CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&tc.d_ldiag), sizeof(double) * (size_t)nt * TB * TB, st));
+  V3DBA_CUDA_TRY(cudaStreamSynchronize(st));   // `all` must outlive its copy
   if ((rc = tile_levels_plan(tc, orig))) return rc;
   static bool attr_set = false;
   if (!attr_set) {
@@ -316,14 +320,9 @@ int tile_chol_plan(TileChol& tc, int n, std::vector<uint8_t>& nz) {
 }
 
 void tile_chol_free(TileChol& tc) {
-  cudaFree(tc.d_panel_rows);
-  cudaFree(tc.d_panel_ptr);
-  cudaFree(tc.d_upd_r);
-  cudaFree(tc.d_upd_c);
-  cudaFree(tc.d_upd_ptr);
-  cudaFree(tc.d_tiles);
-  cudaFree(tc.d_ldiag);
-  cudaFree(tc.d_lv);
+  if (tc.d_plan) cudaFreeAsync(tc.d_plan, tc.st);
+  if (tc.d_ldiag) cudaFreeAsync(tc.d_ldiag, tc.st);
+  if (tc.d_lv) cudaFreeAsync(tc.d_lv, tc.st);
   tc = TileChol();
 }
 
