@@ -123,33 +123,30 @@ __device__ __noinline__ bool warp_chol_inv8(const double* D, double* Zd) {
 #pragma unroll
     for (int r = c; r < 8; ++r) a[pk8(r, c)] = D[c * LDT + r];
   bool ok = true;
-  double s[8];
-  // right-looking Cholesky, L over a
+  // Right-looking in both: step j takes pivot j, column j of L (over a) and row j of Z = L^-1, then
+  // adds column j's terms to the trailing block and to the sums M_rc = sum_{c <= t <= j} L_rt Z_tc of
+  // the later rows (Z_rc = -s_r M_rc), which fill the latency of the next pivot's root.
+  double z[36];   // M, row by row replaced by Z
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     const double d = a[pk8(j, j)];
     if (!(d > 0.0)) ok = false;
     const double sj = rsqrt_nr(d > 0.0 ? d : 1.0);
-    s[j] = sj;
 #pragma unroll
     for (int r = j + 1; r < 8; ++r) a[pk8(r, j)] *= sj;
+    if (j + 1 < 8) a[pk8(j + 1, j + 1)] = fma(-a[pk8(j + 1, j)], a[pk8(j + 1, j)], a[pk8(j + 1, j + 1)]);
 #pragma unroll
     for (int c = j + 1; c < 8; ++c)
 #pragma unroll
-      for (int r = c; r < 8; ++r) a[pk8(r, c)] = fma(-a[pk8(r, j)], a[pk8(c, j)], a[pk8(r, c)]);
-  }
-  // Z = L^-1: Z_cc = 1 / L_cc = s_c, Z_rc = -s_r sum_{t=c}^{r-1} L_rt Z_tc
-  double z[36];
+      for (int r = c; r < 8; ++r)
+        if (!(c == j + 1 && r == c)) a[pk8(r, c)] = fma(-a[pk8(r, j)], a[pk8(c, j)], a[pk8(r, c)]);
 #pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    z[pk8(c, c)] = s[c];
+    for (int c = 0; c < j; ++c) z[pk8(j, c)] = -z[pk8(j, c)] * sj;
+    z[pk8(j, j)] = sj;
 #pragma unroll
-    for (int r = c + 1; r < 8; ++r) {
-      double acc = 0.0;
+    for (int r = j + 1; r < 8; ++r)
 #pragma unroll
-      for (int t = c; t < r; ++t) acc = fma(a[pk8(r, t)], z[pk8(t, c)], acc);
-      z[pk8(r, c)] = -acc * s[r];
-    }
+      for (int c = 0; c <= j; ++c) z[pk8(r, c)] = fma(a[pk8(r, j)], z[pk8(j, c)], c == j ? 0.0 : z[pk8(r, c)]);
   }
   if ((threadIdx.x & 31) == 0) {
 #pragma unroll

@@ -509,15 +509,17 @@ int v3dba_rotations_create(int n_views, int n_pairs, const double* relative_rota
     return V3DBA_ERR_INVALID_ARGUMENT;
   *out = nullptr;
   if ((long)n_pairs * 2 > 0x7fffffffL || (long)n_views * 9 > 0x7fffffffL) return V3DBA_ERR_UNSUPPORTED;
-  for (long t = 0; t < 2L * n_pairs; ++t)
-    if (view_pairs[t] < 0 || view_pairs[t] >= n_views) return V3DBA_ERR_INVALID_INPUT;
-  if (!all_finite(relative_rotations, 9 * (size_t)n_pairs) || !all_finite(rotations, 9 * (size_t)n_views))
-    return V3DBA_ERR_INVALID_INPUT;
   int ndev = 0;
-  if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) {
-    cudaGetLastError();
-    return V3DBA_ERR_NO_DEVICE;
+  const bool device = cudaGetDeviceCount(&ndev) == cudaSuccess && ndev > 0;
+  if (!device) cudaGetLastError();
+  const bool verify = device && (int64_t)n_pairs + n_views >= kDeviceCheckMin;   // on the device, below
+  if (!verify) {
+    for (long t = 0; t < 2L * n_pairs; ++t)
+      if (view_pairs[t] < 0 || view_pairs[t] >= n_views) return V3DBA_ERR_INVALID_INPUT;
+    if (!all_finite(relative_rotations, 9 * (size_t)n_pairs) || !all_finite(rotations, 9 * (size_t)n_views))
+      return V3DBA_ERR_INVALID_INPUT;
   }
+  if (!device) return V3DBA_ERR_NO_DEVICE;
   v3dba_rotations h = new (std::nothrow) v3dba_rotations_s;
   if (!h) return V3DBA_ERR_OUT_OF_MEMORY;
   h->N = n_views;
@@ -582,6 +584,21 @@ int v3dba_rotations_create(int n_views, int n_pairs, const double* relative_rota
   int* keys = reinterpret_cast<int*>(b + o_keys);
   h->state = reinterpret_cast<RotState*>(b + o_state);
   TRY(copy_up({{h->rel, relative_rotations, 72 * P}, {h->pairs, view_pairs, 8 * P}, {h->R0, rotations, 72 * N}}, h->st));
+  if (verify) {
+    int* flag = reinterpret_cast<int*>(h->state);   // (written by a run only)
+    int bad = 0;
+    CTRY(cudaMemsetAsync(flag, 0, sizeof(int), h->st));
+    TRY(check_device({{h->pairs, 2 * (int64_t)P, kCheckIndex, n_views},
+                      {h->rel, 9 * (int64_t)P, kCheckDouble, 0},
+                      {h->R0, 9 * (int64_t)N, kCheckDouble, 0}},
+                     flag, h->st));
+    CTRY(cudaMemcpyAsync(&bad, flag, sizeof(int), cudaMemcpyDeviceToHost, h->st));
+    CTRY(cudaStreamSynchronize(h->st));
+    if (bad) {
+      release(h);
+      return V3DBA_ERR_INVALID_INPUT;
+    }
+  }
   if (N > 0) {
     CTRY(cudaMemcpyAsync(h->R[0], h->R0, 72 * N, cudaMemcpyDeviceToDevice, h->st));
   }

@@ -119,15 +119,20 @@ int copy_params(const ParamSet& dst, const ParamSet& src, const v3dba_handle h, 
   return V3DBA_OK;
 }
 
-int upload_params(v3dba_handle h, const ParamSet& P, const double* K, const double* R, const double* T,
-                  const double* dist, const double* X) {
+int copy_params_up(v3dba_handle h, const ParamSet& P, const double* K, const double* R, const double* T,
+                   const double* dist, const double* X) {
   const Dims& D = h->s.d;
-  const int rc = copy_up({{P.K, K, sizeof(double) * h->nK},
+  return copy_up({{P.K, K, sizeof(double) * h->nK},
                           {P.R, R, sizeof(double) * 9 * (size_t)D.N},
                           {P.T, T, sizeof(double) * 3 * (size_t)D.N},
                           {P.dist, dist, sizeof(double) * h->nD},
                           {P.X, X, sizeof(double) * 3 * (size_t)D.M}},
                          h->stream);
+}
+
+int upload_params(v3dba_handle h, const ParamSet& P, const double* K, const double* R, const double* T,
+                  const double* dist, const double* X) {
+  const int rc = copy_params_up(h, P, K, R, T, dist, X);
   if (rc) return rc;
   V3DBA_CUDA_TRY(cudaStreamSynchronize(h->stream));
   return V3DBA_OK;
@@ -354,8 +359,6 @@ int v3dba_create(const v3dba_problem* p, v3dba_handle* out) {
     if (nrig < 0 || (K > 0 && (nrig == 0 || !p->subcamera)) ||
         (nrig > 0 && (!p->rig_K || !p->rig_R || !p->rig_T)))
       return V3DBA_ERR_INVALID_ARGUMENT;
-    for (int k = 0; k < K; ++k)
-      if (p->subcamera[k] < 0 || p->subcamera[k] >= nrig) return V3DBA_ERR_INVALID_INPUT;
     if (!all_finite(p->rig_K, (size_t)9 * nrig) || !all_finite(p->rig_R, (size_t)9 * nrig) ||
         !all_finite(p->rig_T, (size_t)3 * nrig))
       return V3DBA_ERR_INVALID_INPUT;
@@ -363,22 +366,26 @@ int v3dba_create(const v3dba_problem* p, v3dba_handle* out) {
       if (p->rig_K[9 * l] == 0.0) return V3DBA_ERR_INVALID_INPUT;   // f divides the aspect ratio
   }
   if (!(p->inlier_threshold > 0.0) || !std::isfinite(p->inlier_threshold)) return V3DBA_ERR_INVALID_INPUT;
-  for (int k = 0; k < K; ++k)
-    if (p->view[k] < 0 || p->view[k] >= N || p->point[k] < 0 || p->point[k] >= M) return V3DBA_ERR_INVALID_INPUT;
   const size_t nK = stereo ? 0 : (p->model == V3DBA_MODEL_COMMON) ? 9 : (size_t)9 * N;
   const size_t nD = (p->model == V3DBA_MODEL_COMMON) ? 4 : (p->model == V3DBA_MODEL_VARYING ? (size_t)4 * N : 0);
   if (!all_finite(p->K, nK) || !all_finite(p->R, (size_t)9 * N) || !all_finite(p->T, (size_t)3 * N) ||
-      !all_finite(p->X, (size_t)3 * M) || !all_finite(p->measurements, (size_t)2 * K) ||
       (nD && !all_finite(p->dist, nD)))
     return V3DBA_ERR_INVALID_INPUT;
   if (p->model == V3DBA_MODEL_COMMON && p->K[0] == 0.0) return V3DBA_ERR_INVALID_INPUT;
-
-  trace.mark("validate");
   int ndev = 0;
-  if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) {
-    cudaGetLastError();
-    return V3DBA_ERR_NO_DEVICE;
+  const bool device = cudaGetDeviceCount(&ndev) == cudaSuccess && ndev > 0;
+  if (!device) cudaGetLastError();
+  // what there is one of per point or observation: on the device where that is the faster way
+  const bool verify = device && (int64_t)K + M >= kDeviceCheckMin;
+  if (!verify) {
+    for (int k = 0; k < K; ++k)
+      if (p->view[k] < 0 || p->view[k] >= N || p->point[k] < 0 || p->point[k] >= M ||
+          (stereo && (p->subcamera[k] < 0 || p->subcamera[k] >= nrig)))
+        return V3DBA_ERR_INVALID_INPUT;
+    if (!all_finite(p->X, (size_t)3 * M) || !all_finite(p->measurements, (size_t)2 * K)) return V3DBA_ERR_INVALID_INPUT;
   }
+  trace.mark("validate");
+  if (!device) return V3DBA_ERR_NO_DEVICE;
 
   v3dba_handle h = new (std::nothrow) v3dba_handle_s();
   if (!h) return V3DBA_ERR_OUT_OF_MEMORY;
@@ -395,9 +402,9 @@ int v3dba_create(const v3dba_problem* p, v3dba_handle* out) {
   double pl = 0.0;
   for (int i = 0; i < N; ++i)
     pl += p->T[3 * i] * p->T[3 * i] + p->T[3 * i + 1] * p->T[3 * i + 1] + p->T[3 * i + 2] * p->T[3 * i + 2] + 3.0;
-  for (int j = 0; j < M; ++j)
-    pl += p->X[3 * j] * p->X[3 * j] + p->X[3 * j + 1] * p->X[3 * j + 1] + p->X[3 * j + 2] * p->X[3 * j + 2];
-  h->param_length = std::sqrt(pl);
+  if (!verify)
+    for (int j = 0; j < M; ++j)
+      pl += p->X[3 * j] * p->X[3 * j] + p->X[3 * j + 1] * p->X[3 * j + 1] + p->X[3 * j + 2] * p->X[3 * j + 2];
 
 #define TRY(x) do { if ((rc = (x)) != V3DBA_OK) { free_handle(h); return rc; } } while (0)
 #define CTRY(x) do { cudaError_t _e = (x); if (_e != cudaSuccess) { cudaGetLastError(); free_handle(h); \
@@ -410,9 +417,32 @@ int v3dba_create(const v3dba_problem* p, v3dba_handle* out) {
   h->h_scalars = h->res.pinned;
 
   trace.mark("stream");
+  TRY(alloc_params(h, s.cur, N, M));
+  TRY(alloc_params(h, s.trial, N, M));
+  TRY(alloc_params(h, s.init, N, M));
+  TRY(copy_params_up(h, s.cur, p->K, p->R, p->T, p->dist, p->X));
+  TRY(copy_params(s.init, s.cur, h, h->stream));
+  TRY(copy_params(s.trial, s.cur, h, h->stream));
+  int* sub_in = nullptr;
+  if (stereo) {
+    TRY(dalloc(h, &sub_in, (size_t)std::max(K, 1)));
+    if (K > 0) CTRY(cudaMemcpyAsync(sub_in, p->subcamera, sizeof(int) * K, cudaMemcpyHostToDevice, h->stream));
+  }
+  std::vector<CheckSeg> segs;
+  if (verify) {
+    segs.push_back({s.cur.X, 3 * (int64_t)M, kCheckDouble, 0});
+    if (stereo) segs.push_back({sub_in, K, kCheckIndex, nrig});
+    double* part;
+    TRY(dalloc(h, &part, (size_t)kSumBlocks + 1));
+    TRY(sum_squares_device(s.cur.X, 3 * (int64_t)M, part, part + kSumBlocks, h->stream));
+    CTRY(cudaMemcpyAsync(h->h_scalars, part + kSumBlocks, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+  }
+  trace.mark("params", h->stream);
   DeviceStructure ds;
   const DevAlloc alloc = [h](void** q, size_t bytes) { return dalloc(h, reinterpret_cast<char**>(q), bytes); };
-  TRY(build_structure_device(p, alloc, h->stream, ds));
+  TRY(build_structure_device(p, alloc, h->stream, ds, verify ? &segs : nullptr));
+  if (verify) pl += h->h_scalars[0];   // (the stream was waited for)
+  h->param_length = std::sqrt(pl);
   s.o_cam = ds.o_cam;
   s.o_pt = ds.o_pt;
   s.o_orig = ds.o_orig;
@@ -445,11 +475,8 @@ int v3dba_create(const v3dba_problem* p, v3dba_handle* out) {
       std::memcpy(&rig[(size_t)l * kRigStride + 18], p->rig_T + 3 * l, 3 * sizeof(double));
     }
     TRY(upload(h, &s.rig, rig));
-    int* sub_in;
-    TRY(dalloc(h, &sub_in, (size_t)std::max(K, 1)));
     TRY(dalloc(h, &s.o_sub, (size_t)std::max(K, 1)));
     if (K > 0) {
-      CTRY(cudaMemcpyAsync(sub_in, p->subcamera, sizeof(int) * K, cudaMemcpyHostToDevice, h->stream));
       k_gather_sub<<<(K + 255) / 256, 256, 0, h->stream>>>(sub_in, s.o_orig, K, s.o_sub);
       note_launches(1);
       CTRY(cudaPeekAtLastError());
@@ -471,9 +498,6 @@ int v3dba_create(const v3dba_problem* p, v3dba_handle* out) {
   TRY(dalloc(h, &s.part_bc, (size_t)std::max(s.nch_blk, 1) * block_chunk_values(dA)));
 
   trace.mark("chunks", h->stream);
-  TRY(alloc_params(h, s.cur, N, M));
-  TRY(alloc_params(h, s.trial, N, M));
-  TRY(alloc_params(h, s.init, N, M));
   const size_t Kz = std::max(K, 1), Mz = std::max(M, 1), Nz = std::max(N, 1);
   // 8-byte slots per block, sized for the larger (FP32, 4-float vectors) of the two strides that
   // lm_kernels.cu uses for each block
@@ -531,11 +555,8 @@ int v3dba_create(const v3dba_problem* p, v3dba_handle* out) {
   h->blk_l = ds.h_b_l;
 
   trace.mark("pattern");
-  TRY(upload_params(h, s.cur, p->K, p->R, p->T, p->dist, p->X));
-  TRY(copy_params(s.init, s.cur, h, h->stream));
-  TRY(copy_params(s.trial, s.cur, h, h->stream));
   CTRY(cudaStreamSynchronize(h->stream));
-  trace.mark("params");
+  trace.mark("end");
 #undef TRY
 #undef CTRY
   *out = h;

@@ -219,6 +219,46 @@ __global__ void k_run_starts(const int* __restrict__ flag_scan, const int* __res
   b_l[b] = o_cam[pm[q]];
 }
 
+// ---- checks of the caller's arrays -------------------------------------------------------------
+
+struct CheckList {
+  CheckSeg s[kCheckSegs];
+  int n;
+};
+__global__ void __launch_bounds__(256) k_check(CheckList c, int* flag) {
+  bool bad = false;
+  const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+  for (int q = 0; q < c.n; ++q) {
+    const CheckSeg& g = c.s[q];
+    if (g.kind == kCheckIndex) {
+      const int* p = static_cast<const int*>(g.p);
+      for (int64_t i = t0; i < g.n; i += step) bad |= (unsigned)p[i] >= (unsigned)g.hi;
+    } else if (g.kind == kCheckDouble) {
+      const double* p = static_cast<const double*>(g.p);
+      for (int64_t i = t0; i < g.n; i += step) bad |= !isfinite(p[i]);
+    } else {
+      const float* p = static_cast<const float*>(g.p);
+      for (int64_t i = t0; i < g.n; i += step) bad |= !isfinite(p[i]);
+    }
+  }
+  if (bad) atomicOr(flag, 1);
+}
+
+__global__ void __launch_bounds__(256) k_sum_squares(const double* __restrict__ x, int64_t n, double* part) {
+  __shared__ double red[8];
+  double v[1] = {0.0};
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    v[0] += x[i] * x[i];
+  block_reduce<1, 1>(v, red);
+  if (threadIdx.x == 0) part[blockIdx.x] = v[0];
+}
+__global__ void __launch_bounds__(kSumBlocks) k_sum_parts(const double* __restrict__ part, int n, double* out) {
+  __shared__ double red[kSumBlocks / 32];
+  double v[1] = {(int)threadIdx.x < n ? part[threadIdx.x] : 0.0};
+  block_reduce<1, 1>(v, red);
+  if (threadIdx.x == 0) *out = v[0];
+}
+
 // ---- groups of points with the same cameras --------------------------------------------------
 
 // Sort key of a point's camera sequence; tracks without observations come last.
@@ -453,7 +493,33 @@ __global__ void k_cps_inplace(const int* __restrict__ ptr, const int* __restrict
 
 }  // namespace
 
-int build_structure_device(const v3dba_problem* p, const DevAlloc& alloc, cudaStream_t st, DeviceStructure& S) {
+int check_device(const std::vector<CheckSeg>& segs, int* d_flag, cudaStream_t st) {
+  CheckList c;
+  c.n = 0;
+  int64_t most = 0;
+  if (segs.size() > (size_t)kCheckSegs) return V3DBA_ERR_INVALID_ARGUMENT;
+  for (const CheckSeg& g : segs)
+    if (g.n > 0) {
+      c.s[c.n++] = g;
+      most = std::max(most, g.n);
+    }
+  if (c.n == 0) return V3DBA_OK;
+  k_check<<<(int)std::min<int64_t>((most + 255) / 256, 1184), 256, 0, st>>>(c, d_flag);   // 8 blocks on each of 148 SMs
+  V3DBA_LAUNCH_CHECK();
+  return V3DBA_OK;
+}
+
+int sum_squares_device(const double* x, int64_t n, double* part, double* out, cudaStream_t st) {
+  const int g = (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, kSumBlocks));
+  k_sum_squares<<<g, 256, 0, st>>>(x, n, part);
+  V3DBA_LAUNCH_CHECK();
+  k_sum_parts<<<1, kSumBlocks, 0, st>>>(part, g, out);
+  V3DBA_LAUNCH_CHECK();
+  return V3DBA_OK;
+}
+
+int build_structure_device(const v3dba_problem* p, const DevAlloc& alloc, cudaStream_t st, DeviceStructure& S,
+                           const std::vector<CheckSeg>* verify) {
   const int N = p->n_cameras, M = p->n_points, K = p->n_measurements;
   Scratch sc;
   sc.st = st;
@@ -471,6 +537,20 @@ int build_structure_device(const v3dba_problem* p, const DevAlloc& alloc, cudaSt
                      {d_meas, p->measurements, sizeof(double) * 2 * (size_t)K}},
                     st)))
     return rc;
+  if (verify) {
+    int* d_flag;
+    int flag = 0;
+    if ((rc = sc.get(&d_flag, 1))) return rc;
+    V3DBA_CUDA_TRY(cudaMemsetAsync(d_flag, 0, sizeof(int), st));
+    std::vector<CheckSeg> segs = *verify;
+    segs.push_back({d_view, K, kCheckIndex, N});
+    segs.push_back({d_point, K, kCheckIndex, M});
+    segs.push_back({d_meas, 2 * (int64_t)K, kCheckDouble, 0});
+    if ((rc = check_device(segs, d_flag, st))) return rc;
+    V3DBA_CUDA_TRY(cudaMemcpyAsync(&flag, d_flag, sizeof(int), cudaMemcpyDeviceToHost, st));
+    V3DBA_CUDA_TRY(cudaStreamSynchronize(st));
+    if (flag) return V3DBA_ERR_INVALID_INPUT;
+  }
   const int gK = cdiv(std::max(K, 1), 256);
   // 1. point-major permutation
   uint32_t *ka, *kb;
@@ -785,9 +865,9 @@ void down_add(std::vector<HostCopy>& list, T* h, const T* d, size_t n) {
 
 bool valid_track_ptr(const int* ptr, int n) {
   if (ptr[0] != 0) return false;
-  for (int j = 0; j < n; ++j)
-    if (ptr[j + 1] < ptr[j]) return false;
-  return true;
+  int bad = 0;   // no early exit, so that the loop runs on vectors
+  for (int j = 0; j < n; ++j) bad |= ptr[j + 1] < ptr[j];
+  return bad == 0;
 }
 
 }  // namespace
