@@ -64,6 +64,7 @@ struct DevState {
   int* blk_bc_ptr = nullptr;  // [nb+1] chunks of block b
   // Schur complement by groups of points that the same cameras see (FP64 blocks; build_schur_groups):
   // chunks of points of one group, each with a partial sum for every pair of its cameras
+  bool repeats = false;       // tracks see a camera more than once (pairs of a camera with itself >= 1.5 K)
   int gr_n = 0;               // chunks; 0: the pair lists are used
   int* gr_desc = nullptr;     // [gr_n][4] first point in gr_pt, points, first partial sum, cameras
   int* gr_pt = nullptr;       // [M] points in group order
@@ -148,6 +149,10 @@ enum LmStage {
   kStageTrialFinalize = 13, // {new cost, |delta|^2, delta . g}
   kNumLmStages = 14
 };
+
+// Work chunks over the camera observation lists and the pair lists: one warp each.
+constexpr int kCamChunk = 64;     // observations per camera work chunk
+constexpr int kPairChunk = 128;   // observation pairs per camera-pair work chunk
 
 // partial sizes (doubles) of the chunk kernels for the worst case dims (dA = 13 / dC = 7)
 size_t camera_chunk_values(int DA, int DC);

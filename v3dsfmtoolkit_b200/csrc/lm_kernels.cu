@@ -89,26 +89,50 @@ __device__ __forceinline__ void vstore(double* p, const double (&v)[N]) {
   for (int t = 0; t < N / 2; ++t) q[t] = make_double2(v[2 * t], v[2 * t + 1]);
 }
 
-// Deterministically folds the NV per-block partials of `nblk` blocks (first NS summed, the rest
-// maxed), stored value-major: part[t * nblk + b] (see store_partials).  Warp w folds values w,
-// w + nwarps, ...: lane l reads blocks l, l + 32, ... in order (coalesced), then a fixed shuffle
-// tree.  Every thread receives the results in out[0..NV); smem needs NV doubles.
+// One warp's fold of n partials (summed or maxed) in a fixed order, eight loads in flight per lane; every
+// lane receives the result.
+template <bool SUM>
+__device__ __forceinline__ double warp_fold(const double* __restrict__ p, int n) {
+  constexpr double kNone = SUM ? 0.0 : -1e30;
+  const int lane = threadIdx.x & 31;
+  double acc = kNone;
+  for (int b = lane; b < n; b += 256) {
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = b + 32 * u < n ? p[b + 32 * u] : kNone;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) acc = SUM ? acc + v[u] : fmax(acc, v[u]);
+  }
+  return SUM ? warp_sum(acc) : warp_max(acc);
+}
+
+// The single-block folds run on kFoldWarps warps: the blocks of a value are cut into as many contiguous
+// segments as there are warps for it.  Folds NV values of nblk partials each (the first NS summed, the
+// rest maxed), stored value-major: part[t * nblk + b] (see store_partials).  Every thread receives the
+// results; smem needs NV * fold_segs(NV) doubles.  One warp per value took 53 and 96 us where 2,000 cameras
+// and 1M points leave 15,600 and 21,300 partials; see k_relin_finalize and k_trial_finalize for the rest.
+constexpr int kFoldWarps = 32;
+__host__ __device__ constexpr int fold_segs(int nv) { return nv >= kFoldWarps ? 1 : kFoldWarps / nv; }
 template <int NV, int NS>
 __device__ void fold_partials(const double* __restrict__ part, int nblk, double (&out)[NV], double* smem) {
+  constexpr int SEG = fold_segs(NV);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int t = wid; t < NV; t += nw) {
-    const bool sum = t < NS;
-    double acc = sum ? 0.0 : -1e30;
-    for (int b = lane; b < nblk; b += 32) {
-      const double u = part[(size_t)t * nblk + b];
-      acc = sum ? acc + u : fmax(acc, u);
-    }
-    acc = sum ? warp_sum(acc) : warp_max(acc);
-    if (lane == 0) smem[t] = acc;
+  const int len = (nblk + SEG - 1) / SEG;
+  for (int q = wid; q < NV * SEG; q += nw) {
+    const int t = q / SEG, b0 = min((q - t * SEG) * len, nblk);
+    const double* p = part + (size_t)t * nblk + b0;
+    const int n = min(len, nblk - b0);
+    const double v = t < NS ? warp_fold<true>(p, n) : warp_fold<false>(p, n);
+    if (lane == 0) smem[q] = v;
   }
   __syncthreads();
 #pragma unroll
-  for (int t = 0; t < NV; ++t) out[t] = smem[t];
+  for (int t = 0; t < NV; ++t) {
+    double v = smem[t * SEG];
+#pragma unroll
+    for (int u = 1; u < SEG; ++u) v = t < NS ? v + smem[t * SEG + u] : fmax(v, smem[t * SEG + u]);
+    out[t] = v;
+  }
   __syncthreads();   // smem may be reused right away
 }
 
@@ -173,6 +197,24 @@ struct SchurV {
   static constexpr int VP = round32(NV);
 };
 
+// sum[t] += values lane + 32 t of the partials [c0, c1) of VP values each, in order, eight partials in
+// flight (one after another, a camera's 24 partials took 7 us).
+template <int PER, int VP>
+__device__ __forceinline__ void sum_chunks(double (&sum)[PER], const double* __restrict__ part, int c0, int c1, int lane) {
+  constexpr int U = PER <= 2 ? 8 : 4;
+  for (int c = c0; c < c1; c += U) {
+    double v[U][PER];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int t = 0; t < PER; ++t) v[u][t] = c + u < c1 ? part[(size_t)(c + u) * VP + lane + 32 * t] : 0.0;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int t = 0; t < PER; ++t) sum[t] += v[u][t];
+  }
+}
+
 // row / column of the packed upper-triangle index u of a DA x DA matrix
 template <int DA>
 __device__ __forceinline__ void unpack_sym(int u, int& r, int& c) {
@@ -180,6 +222,49 @@ __device__ __forceinline__ void unpack_sym(int u, int& r, int& c) {
   int start = 0;
   while (u >= start + (DA - r)) { start += DA - r; ++r; }
   c = r + (u - start);
+}
+
+// ---- staged blocks ---------------------------------------------------------------------------
+// The chunk kernels contract small blocks over long lists (observations of a camera, observation pairs of
+// a camera pair).  A lane that loads its own blocks touches a cache line per lane and instruction, and the
+// L1's wavefronts, not bandwidth, set the time.  So a warp copies the blocks of 32 list entries to shared
+// memory together, consecutive lanes on consecutive 16 bytes of a block, and contracts them with DMMA where
+// the sums are FP64: two doubles of accumulator per lane and tile instead of 28 to 112.
+
+// 16 bytes global -> shared; zeros when !use.
+__device__ __forceinline__ void cp16(void* dst, const void* src, bool use) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(use ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_join() {
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
+  __syncwarp();
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+// All copies but those of the last group have arrived.
+__device__ __forceinline__ void cp_join_but_last() {
+  asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+  __syncwarp();
+}
+
+// Copies block `idx` (each lane's own; negative: zeros) of STRIDE values for the warp's 32 pairs:
+// dst[pair * STRIDE + t] = src[idx(pair) * STRIDE + t].
+template <int STRIDE, typename T>
+__device__ __forceinline__ void stage_blocks(T* dst, const T* __restrict__ src, int idx, int lane) {
+  constexpr int E = 16 / sizeof(T), V = STRIDE / E;   // values per copy, copies per block
+  static_assert(STRIDE % E == 0, "blocks are whole 16-byte vectors");
+#pragma unroll
+  for (int t = 0; t < V; ++t) {
+    const int e = lane + 32 * t, rec = e / V, off = e - rec * V;
+    const int k = __shfl_sync(0xffffffffu, idx, rec);
+    cp16(dst + E * e, src + (size_t)max(k, 0) * STRIDE + E * off, k >= 0);
+  }
+}
+
+__device__ __forceinline__ void dmma884(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
 }
 
 // ---- relinearisation --------------------------------------------------------------------
@@ -379,50 +464,91 @@ __global__ void __launch_bounds__(kPtThreads) k_linearize(DevState s, double* __
   store_partials(part, v);
 }
 
+// Shared memory of a warp of k_camera_chunks, in bytes.
+template <int DA, int DC, typename Real>
+__host__ __device__ constexpr int camera_stage_bytes() {
+  using L = Lay<DA, DC, Real>;
+  return 32 * ((L::SA + (DC > 0 ? L::SC : 0)) * (int)sizeof(Real) + L::SG * (int)sizeof(double));
+}
+
 // One warp per chunk of a camera's observation list: partial U = sum A^T A, ga = sum A^T r,
-// X = sum A^T C (FP64 sums); the partials of a camera are folded in chunk order afterwards.
+// X = sum A^T C (FP64 sums); the partials of a camera are folded in chunk order afterwards.  The inner
+// dimension of the products is the residual rows of 32 observations (of ga, the observations).
+// 200 cameras, 375,000 observations, DC = 7: FP32 blocks 25 -> 13.7 us, FP64 35 -> 21 (216 registers held 7
+// warps on an SM); the copies' latency bounds it, at 4.5 TB/s.
 template <int DA, int DC, typename Real>
 __global__ void __launch_bounds__(kCamWarps * 32) k_camera_chunks(DevState s, double* __restrict__ part) {
   pdl_wait();      // the previous stage's writes are visible
   pdl_trigger();   // the next stage may be scheduled once all blocks of this one are resident
   using L = Lay<DA, DC, Real>;
   using CV = CamV<DA, DC>;
-  constexpr int DCc = L::DCc;
-  const int lane = threadIdx.x & 31;
-  const int ch = blockIdx.x * kCamWarps + (threadIdx.x >> 5);
+  constexpr int DCc = L::DCc, NT = (DA + 7) / 8;
+  extern __shared__ double stage_sm[];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, r = lane >> 2, kk = lane & 3;
+  const int ch = blockIdx.x * kCamWarps + w;
   if (ch >= s.nch_cam) return;
-  double acc[CV::VP];
+  char* sm = reinterpret_cast<char*>(stage_sm) + w * camera_stage_bytes<DA, DC, Real>();
+  double* G = reinterpret_cast<double*>(sm);
+  Real* A = reinterpret_cast<Real*>(G + 32 * L::SG);
+  Real* C = A + 32 * L::SA;
+  double u[NT][NT][2], g[NT][2], x[NT][2];
 #pragma unroll
-  for (int t = 0; t < CV::VP; ++t) acc[t] = 0.0;
-  const Real* oA = reinterpret_cast<const Real*>(s.o_A);
-  const Real* oC = reinterpret_cast<const Real*>(s.o_C);
-  for (int idx = s.cc_beg[ch] + lane; idx < s.cc_end[ch]; idx += 32) {
-    const int k = s.c_obs[idx];
-    Real a[L::SA];
-    vload(oA + (size_t)k * L::SA, a);
-    double g[L::SG];
-    vload(s.o_ga + (size_t)k * L::SG, g);
-    int u = 0;
+  for (int a = 0; a < NT; ++a) {
+    g[a][0] = g[a][1] = x[a][0] = x[a][1] = 0.0;
 #pragma unroll
-    for (int r = 0; r < DA; ++r) {
-      acc[CV::NU + r] += g[r];
+    for (int c = 0; c < NT; ++c) u[a][c][0] = u[a][c][1] = 0.0;
+  }
+  constexpr int RD = kCamChunk / 32;
+  const int beg = s.cc_beg[ch], n = s.cc_end[ch] - beg;
+  int ks[RD];   // the chunk's indices first
 #pragma unroll
-      for (int c = r; c < DA; ++c)
-        acc[u++] += double(a[r]) * double(a[c]) + double(a[DA + r]) * double(a[DA + c]);
+  for (int v = 0; v < RD; ++v) ks[v] = 32 * v + lane < n ? s.c_obs[beg + 32 * v + lane] : -1;
+#pragma unroll
+  for (int v = 0; v < RD; ++v) {
+    if (32 * v >= n) break;
+    const int k = ks[v];
+    stage_blocks<L::SA>(A, reinterpret_cast<const Real*>(s.o_A), k, lane);
+    stage_blocks<L::SG>(G, (const double*)s.o_ga, k, lane);
+    if (DC > 0) stage_blocks<L::SC>(C, reinterpret_cast<const Real*>(s.o_C), k, lane);
+    cp_join();
+#pragma unroll
+    for (int st = 0; st < 16; ++st) {   // two observations a step
+      const int q = 2 * st + (kk >> 1), rr = kk & 1;
+      double a[NT];
+#pragma unroll
+      for (int t = 0; t < NT; ++t) a[t] = 8 * t + r < DA ? double(A[q * L::SA + rr * DA + 8 * t + r]) : 0.0;
+#pragma unroll
+      for (int ta = 0; ta < NT; ++ta)
+#pragma unroll
+        for (int tc = ta; tc < NT; ++tc) dmma884(u[ta][tc], a[ta], a[tc]);
+      if (DC > 0) {
+        const double c = r < DC ? double(C[q * L::SC + rr * DCc + r]) : 0.0;
+#pragma unroll
+        for (int ta = 0; ta < NT; ++ta) dmma884(x[ta], a[ta], c);
+      }
     }
-    if (DC > 0) {
-      Real cv[L::SC];
-      vload(oC + (size_t)k * L::SC, cv);
 #pragma unroll
-      for (int r = 0; r < DA; ++r)
+    for (int st = 0; st < 8; ++st)      // four observations a step, against ones
 #pragma unroll
-        for (int c = 0; c < DCc; ++c)
-          acc[CV::NU + DA + r * DCc + c] += double(a[r]) * double(cv[c]) + double(a[DA + r]) * double(cv[DCc + c]);
+      for (int t = 0; t < NT; ++t) dmma884(g[t], 8 * t + r < DA ? G[(4 * st + kk) * L::SG + 8 * t + r] : 0.0, 1.0);
+    __syncwarp();
+  }
+  double* out = part + (size_t)ch * CV::VP;
+#pragma unroll
+  for (int ta = 0; ta < NT; ++ta) {
+    const int R = 8 * ta + r;
+    if (R >= DA) continue;
+    if (kk == 0) out[CV::NU + R] = g[ta][0];
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      if (DC > 0 && 2 * kk + t < DC) out[CV::NU + DA + R * DCc + 2 * kk + t] = x[ta][t];
+#pragma unroll
+      for (int tc = ta; tc < NT; ++tc) {
+        const int Cc = 8 * tc + 2 * kk + t;
+        if (Cc < DA && R <= Cc) out[R * DA - R * (R - 1) / 2 + (Cc - R)] = u[ta][tc][t];
+      }
     }
   }
-  warp_reduce_transpose(acc);
-#pragma unroll
-  for (int t = 0; t < CV::VP / 32; ++t) part[(size_t)ch * CV::VP + lane * (CV::VP / 32) + t] = acc[t];
 }
 
 // One warp per camera: folds its chunk partials in order and stores U_i, ga_i, X_i; gradient
@@ -445,9 +571,7 @@ __global__ void __launch_bounds__(kCamWarps * 32) k_camera_finish(DevState s, co
     double sum[PER];
 #pragma unroll
     for (int t = 0; t < PER; ++t) sum[t] = 0.0;
-    for (int ch = s.cam_cc_ptr[i]; ch < s.cam_cc_ptr[i + 1]; ++ch)
-#pragma unroll
-      for (int t = 0; t < PER; ++t) sum[t] += cpart[(size_t)ch * CV::VP + lane + 32 * t];
+    sum_chunks<PER, CV::VP>(sum, cpart, s.cam_cc_ptr[i], s.cam_cc_ptr[i + 1], lane);
     Real* cU = reinterpret_cast<Real*>(s.c_U) + (size_t)i * L::SU;
     Real* cX = reinterpret_cast<Real*>(s.c_X) + (size_t)i * L::SX;
     double gm = 0.0, dm = -1e30;
@@ -481,14 +605,14 @@ __global__ void __launch_bounds__(kCamWarps * 32) k_camera_finish(DevState s, co
 
 // Sums the relinearisation partials: cost, Z, gc, gradient max, max diagonal, initial lambda.
 template <int DC>
-__global__ void __launch_bounds__(256) k_relin_finalize(DevState s, const double* __restrict__ part_pt, int nbp,
+__global__ void __launch_bounds__(32 * kFoldWarps) k_relin_finalize(DevState s, const double* __restrict__ part_pt, int nbp,
                                                         const double* __restrict__ part_cam, int nbc,
                                                         int init_lambda, double tau) {
   pdl_wait();      // the previous stage's writes are visible
   pdl_trigger();   // the next stage may be scheduled once all blocks of this one are resident
   constexpr int NS = RelinNV<DC>::NS, NV = RelinNV<DC>::NV, NZ = nsym(DC);
   constexpr int DCc = DC > 0 ? DC : 1;
-  __shared__ double red[8 * (NV > 2 ? NV : 2)];
+  __shared__ double red[NV * fold_segs(NV) > kFoldWarps ? NV * fold_segs(NV) : kFoldWarps];
   double a[NV];
   fold_partials<NV, NS>(part_pt, nbp, a, red);
   double b[2];
@@ -542,12 +666,66 @@ __device__ __forceinline__ bool inv3(const double a[6], double o[6]) {
   return true;
 }
 
-// One thread per point: Vinv_j = (V_j + lambda I)^-1, q_j = Vinv gb, Vinv Y_j and, with FP32
-// blocks, T_k = W_k Vinv_j for its observations; Y^T Vinv Y and Y^T q go to per-block partials.
+// T_k = W_k Vinv_j of the FP32 blocks for kPtThreads consecutive observations, one per thread.  The blocks
+// move through shared memory, so that all global accesses are whole lines; a thread inverts its point's
+// V + lambda I itself (as k_point_eliminate's point blocks do, the same bits), which costs less than waiting
+// for them.  One thread per point walking its track's blocks took 23 us for 375,000 observations and 368
+// for 5.5M (2.1 of the copy's 6.5 TB/s); with these blocks in the same launch 19.5
+// and about 140.
+template <int DA, int DC>
+__device__ __forceinline__ void products_body(const DevState& s, int bid) {
+  using L = Lay<DA, DC, float>;
+  __shared__ float4 sm[kPtThreads * L::SW / 4];
+  const int tid = threadIdx.x, k0 = bid * kPtThreads, n = min(kPtThreads, s.d.K - k0), nv = n * L::SW / 4;
+  const float4* src = reinterpret_cast<const float4*>(s.o_W + (size_t)k0 * L::SW);
+  for (int e = tid; e < nv; e += kPtThreads) sm[e] = __ldg(src + e);
+  double vi[6] = {0, 0, 0, 0, 0, 0};
+  if (tid < n) {
+    const int j = s.o_pt[k0 + tid];
+    const double lam = *s.d_lambda;
+    float vv[L::SV];
+    vload(reinterpret_cast<const float*>(s.p_V) + (size_t)j * L::SV, vv);
+    const double a[6] = {double(vv[0]) + lam, double(vv[1]), double(vv[2]), double(vv[3]) + lam, double(vv[4]),
+                         double(vv[5]) + lam};
+    if (j < s.d.nnB || !inv3(a, vi)) vi[0] = vi[1] = vi[2] = vi[3] = vi[4] = vi[5] = 0.0;
+  }
+  __syncthreads();
+  if (tid < n) {
+    float w[L::SW], t[L::SW];
+    float4* own = sm + tid * (L::SW / 4);
+#pragma unroll
+    for (int q = 0; q < L::SW / 4; ++q) {
+      const float4 x = own[q];
+      w[4 * q] = x.x; w[4 * q + 1] = x.y; w[4 * q + 2] = x.z; w[4 * q + 3] = x.w;
+    }
+#pragma unroll
+    for (int x = 0; x < L::SW; ++x) t[x] = 0.f;
+#pragma unroll
+    for (int r = 0; r < DA; ++r)
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        t[r * 3 + c] = float(double(w[r * 3]) * vi[s3(0, c)] + double(w[r * 3 + 1]) * vi[s3(1, c)] +
+                             double(w[r * 3 + 2]) * vi[s3(2, c)]);
+#pragma unroll
+    for (int q = 0; q < L::SW / 4; ++q) own[q] = make_float4(t[4 * q], t[4 * q + 1], t[4 * q + 2], t[4 * q + 3]);
+  }
+  __syncthreads();
+  float4* dst = reinterpret_cast<float4*>(s.o_T + (size_t)k0 * L::SW);
+  for (int e = tid; e < nv; e += kPtThreads) dst[e] = sm[e];
+}
+
+// One thread per point: Vinv_j = (V_j + lambda I)^-1, q_j = Vinv gb, Vinv Y_j; Y^T Vinv Y and Y^T q go to
+// per-block partials.  With FP32 blocks, the blocks from nbp on form the observations' T_k.
 template <int DA, int DC, typename Real>
-__global__ void __launch_bounds__(kPtThreads) k_point_eliminate(DevState s, double* __restrict__ part) {
+__global__ void __launch_bounds__(kPtThreads) k_point_eliminate(DevState s, double* __restrict__ part, int nbp) {
   pdl_wait();      // the previous stage's writes are visible
   pdl_trigger();   // the next stage may be scheduled once all blocks of this one are resident
+  if constexpr (stores_products<Real>()) {
+    if ((int)blockIdx.x >= nbp) {
+      products_body<DA, DC>(s, blockIdx.x - nbp);
+      return;
+    }
+  }
   using L = Lay<DA, DC, Real>;
   constexpr int DCc = L::DCc;
   constexpr int NV = ElimNV<DC>::NV;
@@ -606,91 +784,204 @@ __global__ void __launch_bounds__(kPtThreads) k_point_eliminate(DevState s, doub
       for (int c = 0; c < DCc; ++c)
         v[nsym(DC) + c] = double(yv[c]) * q[0] + double(yv[DCc + c]) * q[1] + double(yv[2 * DCc + c]) * q[2];
     }
-    if constexpr (stores_products<Real>()) {
-      for (int k = s.p_ptr[j]; k < s.p_ptr[j + 1]; ++k) {
-        float w[L::SW];
-        vload(s.o_W + (size_t)k * L::SW, w);
-        float t[L::SW];
-#pragma unroll
-        for (int x = 0; x < L::SW; ++x) t[x] = 0.f;
-#pragma unroll
-        for (int r = 0; r < DA; ++r)
-#pragma unroll
-          for (int c = 0; c < 3; ++c)
-            t[r * 3 + c] = float(double(w[r * 3]) * vi[s3(0, c)] + double(w[r * 3 + 1]) * vi[s3(1, c)] +
-                                 double(w[r * 3 + 2]) * vi[s3(2, c)]);
-        vstore(s.o_T + (size_t)k * L::SW, t);
-      }
-    }
   }
   block_reduce<NV, NV>(v, red);
-  store_partials(part, v);
+  store_partials(part, v, (int)blockIdx.x, nbp);
 }
 
-// One warp per chunk of a camera-pair block's observation pairs: partial sum T_k W_m^T (FP32
-// blocks: the stored T_k and W_m; FP64 blocks: A_k^T (B_k Vinv_j B_m^T) A_m).
+// ---- Schur sums over the pair lists ------------------------------------------------------------
+// One warp per chunk of a camera-pair block's observation pairs: partial sum T_k W_m^T (FP32 blocks: the
+// stored T_k and W_m; FP64 blocks: A_k^T (B_k Vinv_j B_m^T) A_m).  The blocks of 32 pairs are copied to
+// shared memory by the warp together, consecutive lanes on consecutive 16 bytes of a block.  Loads of a
+// lane's own blocks touch a cache line per lane and instruction: the L1's wavefronts were 82% busy, at 5.1
+// TB/s from L2 and 16% of the FP64 pipe.  Staged, FP32 blocks read at 8 TB/s from L2, which is the bound: the
+// launch with the rhs chunks went 1,487 -> 929 us on 2,000 cameras (35M pairs), the sums alone 60 -> 48 us on
+// 200 (1.8M pairs, FP64 118 -> 103).
+
+// Shared memory of a warp, in bytes.
 template <int DA, typename Real>
-__device__ __forceinline__ void schur_chunks_body(DevState s, double* __restrict__ part, int bid, int nblk) {
+__host__ __device__ constexpr int schur_stage_bytes() {
   using L = Lay<DA, 0, Real>;
+  return stores_products<Real>() ? 2 * 32 * 2 * L::SW * (int)sizeof(float)
+                                 : 32 * (2 * L::SA + 2 * kSB + L::SV + 4) * (int)sizeof(double);
+}
+
+template <int DA>
+__device__ __forceinline__ void schur_chunk_fp32(const DevState& s, double* __restrict__ part, float* sm, int ch, int lane) {
+  using L = Lay<DA, 0, float>;
   using SV = SchurV<DA>;
-  const int lane = threadIdx.x & 31;
-  const int ch = bid * 4 + (threadIdx.x >> 5);
-  if (ch >= s.nch_blk) return;
-  Real acc[SV::VP];
+  float acc[SV::VP];
 #pragma unroll
-  for (int t = 0; t < SV::VP; ++t) acc[t] = Real(0);
-  const int end = s.bc_end[ch];
-  if constexpr (!stores_products<Real>()) {
-    // FP64 blocks: T_k W_m^T = A_k^T (B_k Vinv_j B_m^T) A_m, 126 FMAs per pair
-    const double* oA = reinterpret_cast<const double*>(s.o_A);
-    for (int p = s.bc_beg[ch] + lane; p < end; p += 32) {
-      const int k = s.pr_k[p], m = s.pr_m[p];
-      const int j = s.o_pt[k];
-      double Ak[L::SA], Am[L::SA], Bk[kSB], Bm[kSB], vi[L::SV];
-      vload(oA + (size_t)k * L::SA, Ak);
-      vload(s.o_B + (size_t)k * kSB, Bk);
-      vload(oA + (size_t)m * L::SA, Am);
-      vload(s.o_B + (size_t)m * kSB, Bm);
-      vload(reinterpret_cast<const double*>(s.p_Vinv) + (size_t)j * L::SV, vi);
-      double Q[2][3];   // B_k Vinv_j
+  for (int t = 0; t < SV::VP; ++t) acc[t] = 0.f;
+  // the chunk's indices first, then the blocks of the next 32 pairs in flight during the current ones
+  constexpr int R = kPairChunk / 32, kBuf = 32 * 2 * L::SW;
+  const int beg = s.bc_beg[ch], n = s.bc_end[ch] - beg;
+  int k[R], m[R];
 #pragma unroll
-      for (int r = 0; r < 2; ++r)
+  for (int u = 0; u < R; ++u) {
+    const bool in = 32 * u + lane < n;
+    k[u] = in ? s.pr_k[beg + 32 * u + lane] : -1;
+    m[u] = in ? s.pr_m[beg + 32 * u + lane] : -1;
+  }
+  auto fetch = [&](int u) {
+    float* b = sm + (u & 1) * kBuf;
+    stage_blocks<L::SW>(b, (const float*)s.o_T, k[u], lane);
+    stage_blocks<L::SW>(b + 32 * L::SW, (const float*)s.o_W, m[u], lane);
+    cp_commit();
+  };
+  fetch(0);
 #pragma unroll
-        for (int c = 0; c < 3; ++c)
-          Q[r][c] = Bk[3 * r] * vi[s3(0, c)] + Bk[3 * r + 1] * vi[s3(1, c)] + Bk[3 * r + 2] * vi[s3(2, c)];
-      double Mx[2][2];  // B_k Vinv_j B_m^T
+  for (int u = 0; u < R; ++u) {
+    if (32 * u >= n) break;
+    if (u + 1 < R && 32 * (u + 1) < n) {
+      fetch(u + 1);
+      cp_join_but_last();
+    } else {
+      cp_join();
+    }
+    if (32 * u + lane < n) {
+      const float* b = sm + (u & 1) * kBuf + lane * L::SW;
+      float t[L::SW], w[L::SW];
 #pragma unroll
-      for (int r = 0; r < 2; ++r)
+      for (int q = 0; q < L::SW / 4; ++q) {
+        const float4 x = reinterpret_cast<const float4*>(b)[q], y = reinterpret_cast<const float4*>(b + 32 * L::SW)[q];
+        t[4 * q] = x.x; t[4 * q + 1] = x.y; t[4 * q + 2] = x.z; t[4 * q + 3] = x.w;
+        w[4 * q] = y.x; w[4 * q + 1] = y.y; w[4 * q + 2] = y.z; w[4 * q + 3] = y.w;
+      }
 #pragma unroll
-        for (int t = 0; t < 2; ++t) Mx[r][t] = Q[r][0] * Bm[3 * t] + Q[r][1] * Bm[3 * t + 1] + Q[r][2] * Bm[3 * t + 2];
+      for (int a = 0; a < DA; ++a)
 #pragma unroll
-      for (int c = 0; c < DA; ++c) {
-        const double n0 = Mx[0][0] * Am[c] + Mx[0][1] * Am[DA + c];
-        const double n1 = Mx[1][0] * Am[c] + Mx[1][1] * Am[DA + c];
+        for (int c = 0; c < DA; ++c)
+          acc[a * DA + c] += t[a * 3] * w[c * 3] + t[a * 3 + 1] * w[c * 3 + 1] + t[a * 3 + 2] * w[c * 3 + 2];
+    }
+    __syncwarp();
+  }
+  warp_reduce_transpose(acc);
 #pragma unroll
-        for (int a = 0; a < DA; ++a) acc[a * DA + c] += Ak[a] * n0 + Ak[DA + a] * n1;
+  for (int t = 0; t < SV::VP / 32; ++t) part[(size_t)ch * SV::VP + lane * (SV::VP / 32) + t] = double(acc[t]);
+}
+
+// With the residual rows of the 32 pairs as the inner dimension, sum A_k^T M A_m on DMMA, M = B_k Vinv_j
+// B_m^T from a lane's own pair.
+template <int DA>
+__device__ __forceinline__ void schur_chunk_fp64(const DevState& s, double* __restrict__ part, double* sm, int ch, int lane) {
+  using L = Lay<DA, 0, double>;
+  using SV = SchurV<DA>;
+  constexpr int NT = (DA + 7) / 8, SA = L::SA;
+  double* Ak = sm;
+  double* Am = Ak + 32 * SA;
+  double* Bk = Am + 32 * SA;
+  double* Bm = Bk + 32 * kSB;
+  double* Vi = Bm + 32 * kSB;
+  double* Mx = Vi + 32 * L::SV;    // [32][2][2]
+  double acc[2][NT][NT][2];        // two sets, for even and odd steps (shorter DMMA chains)
+#pragma unroll
+  for (int u = 0; u < 2; ++u)
+#pragma unroll
+    for (int a = 0; a < NT; ++a)
+#pragma unroll
+      for (int c = 0; c < NT; ++c) acc[u][a][c][0] = acc[u][a][c][1] = 0.0;
+  const int beg = s.bc_beg[ch], n = s.bc_end[ch] - beg, r = lane >> 2, kk = lane & 3;
+  constexpr int R = kPairChunk / 32;
+  int ks[R], ms[R], js[R];   // the chunk's indices first
+#pragma unroll
+  for (int u = 0; u < R; ++u) {
+    const bool in = 32 * u + lane < n;
+    ks[u] = in ? s.pr_k[beg + 32 * u + lane] : -1;
+    ms[u] = in ? s.pr_m[beg + 32 * u + lane] : -1;
+  }
+#pragma unroll
+  for (int u = 0; u < R; ++u) js[u] = ks[u] >= 0 ? s.o_pt[ks[u]] : -1;
+#pragma unroll
+  for (int u = 0; u < R; ++u) {
+    if (32 * u >= n) break;
+    const int k = ks[u], m = ms[u], j = js[u];
+    stage_blocks<SA>(Ak, reinterpret_cast<const double*>(s.o_A), k, lane);
+    stage_blocks<kSB>(Bk, (const double*)s.o_B, k, lane);
+    stage_blocks<SA>(Am, reinterpret_cast<const double*>(s.o_A), m, lane);
+    stage_blocks<kSB>(Bm, (const double*)s.o_B, m, lane);
+    stage_blocks<L::SV>(Vi, reinterpret_cast<const double*>(s.p_Vinv), j, lane);
+    cp_join();
+    {
+      double bk[6], bm[6], vi[6];
+#pragma unroll
+      for (int t = 0; t < 3; ++t) {
+        const double2 x = reinterpret_cast<const double2*>(Bk + kSB * lane)[t], y = reinterpret_cast<const double2*>(Bm + kSB * lane)[t],
+                      z = reinterpret_cast<const double2*>(Vi + L::SV * lane)[t];
+        bk[2 * t] = x.x; bk[2 * t + 1] = x.y;
+        bm[2 * t] = y.x; bm[2 * t + 1] = y.y;
+        vi[2 * t] = z.x; vi[2 * t + 1] = z.y;
+      }
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        double Q[3];   // row q of B_k Vinv_j
+#pragma unroll
+        for (int c = 0; c < 3; ++c) Q[c] = bk[3 * q] * vi[s3(0, c)] + bk[3 * q + 1] * vi[s3(1, c)] + bk[3 * q + 2] * vi[s3(2, c)];
+        reinterpret_cast<double2*>(Mx)[2 * lane + q] =
+            make_double2(Q[0] * bm[0] + Q[1] * bm[1] + Q[2] * bm[2], Q[0] * bm[3] + Q[1] * bm[4] + Q[2] * bm[5]);
       }
     }
-  } else {
-  const float* oT = s.o_T;
-  const float* oW = s.o_W;
-  // FP32 blocks: a lane takes its pairs p and p + 32 in one trip, so both pairs' gathers are in
-  // flight together (same summation order as one pair per trip), except with 13 unknowns per
-  // camera, whose blocks already fill the register file.
-  constexpr int U = DA <= 11 ? 2 : 1;
-  for (int p = s.bc_beg[ch] + lane; p < end; p += 32 * U) {
-    int k[U], m[U];
+    __syncwarp();
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int q = p + 32 * u < end ? p + 32 * u : p;   // a missing second pair re-reads the first
-      k[u] = s.pr_k[q];
-      m[u] = s.pr_m[q];
+    for (int st = 0; st < 16; ++st) {   // two pairs a step: inner index kk = 2 (pair) + (residual row)
+      const int q = 2 * st + (kk >> 1);
+      const double2 mm = reinterpret_cast<const double2*>(Mx)[2 * q + (kk & 1)];
+      double a[NT], z[NT];
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        const int row = 8 * t + r;
+        const bool ok = row < DA;
+        const double* am = Am + q * SA + (ok ? row : 0);
+        a[t] = ok ? Ak[q * SA + (kk & 1) * DA + row] : 0.0;
+        z[t] = ok ? mm.x * am[0] + mm.y * am[DA] : 0.0;
+      }
+#pragma unroll
+      for (int ta = 0; ta < NT; ++ta)
+#pragma unroll
+        for (int tc = 0; tc < NT; ++tc) dmma884(acc[st & 1][ta][tc], a[ta], z[tc]);
     }
+    __syncwarp();
+  }
+#pragma unroll
+  for (int ta = 0; ta < NT; ++ta)
+#pragma unroll
+    for (int tc = 0; tc < NT; ++tc)
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        const int row = 8 * ta + r, col = 8 * tc + 2 * kk + t;
+        if (row < DA && col < DA) part[(size_t)ch * SV::VP + row * DA + col] = acc[0][ta][tc][t] + acc[1][ta][tc][t];
+      }
+}
+
+// The same sums from a lane's own loads (DIRECT): where tracks see a camera more than once (a rig's two
+// cameras in one pose), neighbouring pairs share their blocks, and the shared lines and the L1 serve them
+// (300 rig poses, 3.2M pairs, FP32 blocks: 64 us, staged 68); and for a launch of a single wave, where a
+// chunk's latency counts and the copies add to it (20 cameras, 268 chunks, FP64: 7.1 us, staged 8.7).
+constexpr int kDirectChunks = 1184;   // two blocks of four chunks on each of 148 SMs
+// (the direct FP64 sums of more than 9 unknowns per camera spill their accumulators)
+template <int DA, typename Real>
+__host__ __device__ constexpr bool has_direct() { return stores_products<Real>() || DA <= 9; }
+template <int DA, typename Real>
+bool schur_direct(const DevState& s) { return has_direct<DA, Real>() && (s.repeats || s.nch_blk <= kDirectChunks); }
+
+// FP32 blocks: the sums in the same order as schur_chunk_fp32.  Two pairs a trip, so both pairs' gathers
+// are in flight, except with 13 unknowns per camera, whose blocks already fill the register file.
+template <int DA>
+__device__ __forceinline__ void schur_chunk_fp32_direct(const DevState& s, double* __restrict__ part, int ch, int lane) {
+  using L = Lay<DA, 0, float>;
+  using SV = SchurV<DA>;
+  constexpr int U = DA <= 11 ? 2 : 1;
+  float acc[SV::VP];
+#pragma unroll
+  for (int t = 0; t < SV::VP; ++t) acc[t] = 0.f;
+  const int end = s.bc_end[ch];
+  for (int p = s.bc_beg[ch] + lane; p < end; p += 32 * U) {
     float t[U][L::SW], w[U][L::SW];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      vload(oT + (size_t)k[u] * L::SW, t[u]);
-      vload(oW + (size_t)m[u] * L::SW, w[u]);
+      const int q = p + 32 * u < end ? p + 32 * u : p;   // a missing second pair re-reads the first
+      vload(s.o_T + (size_t)s.pr_k[q] * L::SW, t[u]);
+      vload(s.o_W + (size_t)s.pr_m[q] * L::SW, w[u]);
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -703,16 +994,66 @@ __device__ __forceinline__ void schur_chunks_body(DevState s, double* __restrict
                              t[u][a * 3 + 2] * w[u][c * 3 + 2];
     }
   }
-  }
   warp_reduce_transpose(acc);
 #pragma unroll
   for (int t = 0; t < SV::VP / 32; ++t) part[(size_t)ch * SV::VP + lane * (SV::VP / 32) + t] = double(acc[t]);
 }
 
-__device__ __forceinline__ void dmma884(double (&c)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(c[0]), "+d"(c[1])
-               : "d"(a), "d"(b));
+template <int DA>
+__device__ __forceinline__ void schur_chunk_fp64_direct(const DevState& s, double* __restrict__ part, int ch, int lane) {
+  using L = Lay<DA, 0, double>;
+  using SV = SchurV<DA>;
+  double acc[SV::VP];
+#pragma unroll
+  for (int t = 0; t < SV::VP; ++t) acc[t] = 0.0;
+  const double* oA = reinterpret_cast<const double*>(s.o_A);
+  const int end = s.bc_end[ch];
+  for (int p = s.bc_beg[ch] + lane; p < end; p += 32) {
+    const int k = s.pr_k[p], m = s.pr_m[p];
+    const int j = s.o_pt[k];
+    double Ak[L::SA], Am[L::SA], Bk[kSB], Bm[kSB], vi[L::SV];
+    vload(oA + (size_t)k * L::SA, Ak);
+    vload(s.o_B + (size_t)k * kSB, Bk);
+    vload(oA + (size_t)m * L::SA, Am);
+    vload(s.o_B + (size_t)m * kSB, Bm);
+    vload(reinterpret_cast<const double*>(s.p_Vinv) + (size_t)j * L::SV, vi);
+    double Q[2][3];   // B_k Vinv_j
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        Q[r][c] = Bk[3 * r] * vi[s3(0, c)] + Bk[3 * r + 1] * vi[s3(1, c)] + Bk[3 * r + 2] * vi[s3(2, c)];
+    double Mx[2][2];  // B_k Vinv_j B_m^T
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int t = 0; t < 2; ++t) Mx[r][t] = Q[r][0] * Bm[3 * t] + Q[r][1] * Bm[3 * t + 1] + Q[r][2] * Bm[3 * t + 2];
+#pragma unroll
+    for (int c = 0; c < DA; ++c) {
+      const double n0 = Mx[0][0] * Am[c] + Mx[0][1] * Am[DA + c];
+      const double n1 = Mx[1][0] * Am[c] + Mx[1][1] * Am[DA + c];
+#pragma unroll
+      for (int a = 0; a < DA; ++a) acc[a * DA + c] += Ak[a] * n0 + Ak[DA + a] * n1;
+    }
+  }
+  warp_reduce_transpose(acc);
+#pragma unroll
+  for (int t = 0; t < SV::VP / 32; ++t) part[(size_t)ch * SV::VP + lane * (SV::VP / 32) + t] = acc[t];
+}
+
+template <int DA, typename Real, bool DIRECT>
+__device__ __forceinline__ void schur_chunks_body(DevState s, double* __restrict__ part, int bid, int nblk) {
+  extern __shared__ double stage_sm[];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, ch = bid * 4 + w;
+  if (ch >= s.nch_blk) return;
+  if constexpr (DIRECT && has_direct<DA, Real>()) {
+    if constexpr (stores_products<Real>()) schur_chunk_fp32_direct<DA>(s, part, ch, lane);
+    else schur_chunk_fp64_direct<DA>(s, part, ch, lane);
+  } else {
+    char* sm = reinterpret_cast<char*>(stage_sm) + w * schur_stage_bytes<DA, Real>();
+    if constexpr (stores_products<Real>()) schur_chunk_fp32<DA>(s, part, reinterpret_cast<float*>(sm), ch, lane);
+    else schur_chunk_fp64<DA>(s, part, reinterpret_cast<double*>(sm), ch, lane);
+  }
 }
 
 // FP64 blocks, points grouped by their cameras: one block per chunk of up to 32 points that the same L
@@ -727,13 +1068,11 @@ __device__ __forceinline__ void dmma884(double (&c)[2], double a, double b) {
 // latency of a chunk (pattern, blocks, product): the DMMAs are 14 us of it.
 constexpr int kGroupThreads = 256;
 template <int DA>
-__global__ void __launch_bounds__(kGroupThreads, DA <= 9 ? 3 : 2) k_schur_groups(DevState s) {
-  pdl_wait();
-  pdl_trigger();
+__device__ __forceinline__ void schur_group_body(const DevState& s, int ch) {
   using L_ = Lay<DA, 0, double>;
   extern __shared__ double group_sm[];
   const int tid = threadIdx.x, lane = tid & 31;
-  const int4 d = reinterpret_cast<const int4*>(s.gr_desc)[blockIdx.x];
+  const int4 d = reinterpret_cast<const int4*>(s.gr_desc)[ch];
   const int p0 = d.x, np = d.y, e0 = d.z, L = d.w;
   const int rows = DA * L, ld = group_ld(rows), K = (3 * np + 3) / 4 * 4;
   double* Gs = group_sm;
@@ -835,11 +1174,18 @@ __global__ void __launch_bounds__(kGroupThreads, DA <= 9 ? 3 : 2) k_schur_groups
     }
 }
 
-template <int DA, typename Real>
+template <int DA>
+__global__ void __launch_bounds__(kGroupThreads, DA <= 9 ? 3 : 2) k_schur_groups(DevState s) {
+  pdl_wait();
+  pdl_trigger();
+  schur_group_body<DA>(s, blockIdx.x);
+}
+
+template <int DA, typename Real, bool DIRECT>
 __global__ void __launch_bounds__(128) k_schur_chunks(DevState s, double* __restrict__ part) {
   pdl_wait();      // the previous stage's writes are visible
   pdl_trigger();   // the next stage may be scheduled once all blocks of this one are resident
-  schur_chunks_body<DA, Real>(s, part, blockIdx.x, gridDim.x);
+  schur_chunks_body<DA, Real, DIRECT>(s, part, blockIdx.x, gridDim.x);
 }
 
 // One warp per camera-pair block (i <= l): S_il = delta_il (U_i + lambda I) - sum of its chunk
@@ -894,9 +1240,7 @@ __device__ __forceinline__ void schur_finish_body(DevState s, const double* __re
 #pragma unroll
     for (int t = 0; t < PER; ++t) sum[t] += ws[0][lane + 32 * t] + ws[1][lane + 32 * t] + ws[2][lane + 32 * t];
   } else {
-    for (int ch = s.blk_bc_ptr[b]; ch < s.blk_bc_ptr[b + 1]; ++ch)
-#pragma unroll
-      for (int t = 0; t < PER; ++t) sum[t] += part[(size_t)ch * SV::VP + lane + 32 * t];
+    sum_chunks<PER, SV::VP>(sum, part, s.blk_bc_ptr[b], s.blk_bc_ptr[b + 1], lane);
   }
   const double lam = *s.d_lambda;
   const Real* cU = reinterpret_cast<const Real*>(s.c_U) + (size_t)i * L::SU;
@@ -924,27 +1268,45 @@ __global__ void __launch_bounds__(128) k_schur_finish(DevState s, const double* 
   schur_finish_body<DA, Real>(s, part, blockIdx.x, gridDim.x);
 }
 
-// One warp per chunk of a camera's observations: partial sum_k W_k q_j(k) and sum_k T_k Y_j(k),
-// the latter as sum_k W_k (Vinv Y)_j(k) (FP64 blocks: W_k x as A_k^T (B_k x)).
+// Whether the rhs chunks are staged: FP64 blocks stay with a lane's own loads where the sums are 32 values
+// or less and the tile mostly padding: few border columns (158 cameras, DC = 1: 8.2 us against 12.5
+// staged), or more unknowns than a tile's eight rows (30 cameras, DA = 11: 188 us an iteration against 198).
 template <int DA, int DC, typename Real>
+__host__ __device__ constexpr bool rhs_staged() {
+  return stores_products<Real>() || RhsV<DA, DC>::VP > 32 || (DC == 0 && DA <= 8);
+}
+// Shared memory of a warp of the rhs chunks, in bytes.
+template <int DA, int DC, typename Real>
+__host__ __device__ constexpr int rhs_stage_bytes() {
+  using L = Lay<DA, DC, Real>;
+  return !rhs_staged<DA, DC, Real>() ? 0 : 32 * (4 * (int)sizeof(double) + (DC > 0 ? L::SY * (int)sizeof(Real) : 0) +
+               (stores_products<Real>() ? L::SW * (int)sizeof(float) : (L::SA + kSB) * (int)sizeof(double)));
+}
+
+// One warp per chunk of a camera's observations: partial sum_k W_k q_j(k) and sum_k T_k Y_j(k),
+// the latter as sum_k W_k (Vinv Y)_j(k), together the product of the W_k with the 1 + DC <= 8 columns
+// [q Vinv Y] of their points: with FP32 blocks the inner dimension is the points' three coordinates (four
+// observations in three DMMA steps), with FP64 blocks the residual rows (W_k x = A_k^T (B_k x)).  200 cameras,
+// DC = 7: FP32 blocks 25 -> 14 us, FP64 32 -> 26.
+template <int DA, int DC, typename Real, int WARPS = kCamWarps>
 __device__ __forceinline__ void rhs_chunks_body(DevState s, double* __restrict__ part, int bid, int nblk) {
   using L = Lay<DA, DC, Real>;
   using RV = RhsV<DA, DC>;
-  constexpr int DCc = L::DCc;
-  const int lane = threadIdx.x & 31;
-  const int ch = bid * kCamWarps + (threadIdx.x >> 5);
-  if (ch >= s.nch_cam) return;
-  double acc[RV::VP];
+  constexpr int DCc = L::DCc, NT = (DA + 7) / 8;
+  static_assert(DC <= 7, "the right-hand side and the border are eight columns");
+  extern __shared__ double stage_sm[];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, r = lane >> 2, kk = lane & 3;
+  const int ch = bid * WARPS + w;
+  if (w >= WARPS || ch >= s.nch_cam) return;
+  if constexpr (!rhs_staged<DA, DC, Real>()) {
+    double acc[RV::VP];
 #pragma unroll
-  for (int t = 0; t < RV::VP; ++t) acc[t] = 0.0;
-  for (int idx = s.cc_beg[ch] + lane; idx < s.cc_end[ch]; idx += 32) {
-    const int k = s.c_obs[idx];
-    const int j = s.o_pt[k];
-    double q[4];
-    vload(s.p_q + (size_t)j * 4, q);
-    if constexpr (!stores_products<Real>()) {
-      // W_k x = A_k^T (B_k x)
-      double A[L::SA], B[kSB];
+    for (int t = 0; t < RV::VP; ++t) acc[t] = 0.0;
+    for (int idx = s.cc_beg[ch] + lane; idx < s.cc_end[ch]; idx += 32) {
+      const int k = s.c_obs[idx];
+      const int j = s.o_pt[k];
+      double q[4], A[L::SA], B[kSB];
+      vload(s.p_q + (size_t)j * 4, q);
       vload(reinterpret_cast<const double*>(s.o_A) + (size_t)k * L::SA, A);
       vload(s.o_B + (size_t)k * kSB, B);
       const double bq0 = B[0] * q[0] + B[1] * q[1] + B[2] * q[2];
@@ -962,27 +1324,83 @@ __device__ __forceinline__ void rhs_chunks_body(DevState s, double* __restrict__
           for (int a = 0; a < DA; ++a) acc[DA + a * DCc + c] += A[a] * by0 + A[DA + a] * by1;
         }
       }
-      continue;
     }
-    float w[L::SW];
-    vload(s.o_W + (size_t)k * L::SW, w);
+    warp_reduce_transpose(acc);
 #pragma unroll
-    for (int a = 0; a < DA; ++a) acc[a] += double(w[a * 3]) * q[0] + double(w[a * 3 + 1]) * q[1] + double(w[a * 3 + 2]) * q[2];
-    if (DC > 0) {
-      // T_k Y_j = W_k (Vinv_j Y_j): the point's Vinv Y is already stored, so no T_k gather
-      Real yv[L::SY];
-      vload(reinterpret_cast<const Real*>(s.p_YV) + (size_t)j * L::SY, yv);
+    for (int t = 0; t < RV::VP / 32; ++t) part[(size_t)ch * RV::VP + lane * (RV::VP / 32) + t] = acc[t];
+    return;
+  }
+  char* sm = reinterpret_cast<char*>(stage_sm) + w * rhs_stage_bytes<DA, DC, Real>();
+  double* Q = reinterpret_cast<double*>(sm);
+  Real* Y = reinterpret_cast<Real*>(Q + 32 * 4);
+  char* rest = reinterpret_cast<char*>(Y + (DC > 0 ? 32 * L::SY : 0));
+  float* W = reinterpret_cast<float*>(rest);           // FP32 blocks
+  double* A = reinterpret_cast<double*>(rest);         // FP64 blocks
+  double* B = A + 32 * L::SA;
+  double acc[2][NT][2];   // two sets in turn (shorter DMMA chains)
 #pragma unroll
-      for (int a = 0; a < DA; ++a)
+  for (int v = 0; v < 2; ++v)
 #pragma unroll
-        for (int c = 0; c < DCc; ++c)
-          acc[DA + a * DCc + c] += double(w[a * 3]) * double(yv[c]) + double(w[a * 3 + 1]) * double(yv[DCc + c]) +
-                                   double(w[a * 3 + 2]) * double(yv[2 * DCc + c]);
+    for (int a = 0; a < NT; ++a) acc[v][a][0] = acc[v][a][1] = 0.0;
+  // element c of column r of an entry's [q Vinv Y]
+  auto column = [&](int q, int c) -> double {
+    return r == 0 ? Q[4 * q + c] : (DC > 0 && r <= DC) ? double(Y[q * L::SY + c * DCc + r - 1]) : 0.0;
+  };
+  constexpr int RD = kCamChunk / 32;
+  const int beg = s.cc_beg[ch], n = s.cc_end[ch] - beg;
+  int ks[RD], js[RD];   // the chunk's indices first
+#pragma unroll
+  for (int v = 0; v < RD; ++v) ks[v] = 32 * v + lane < n ? s.c_obs[beg + 32 * v + lane] : -1;
+#pragma unroll
+  for (int v = 0; v < RD; ++v) js[v] = ks[v] >= 0 ? s.o_pt[ks[v]] : -1;
+#pragma unroll
+  for (int v = 0; v < RD; ++v) {
+    if (32 * v >= n) break;
+    const int k = ks[v], j = js[v];
+    stage_blocks<4>(Q, (const double*)s.p_q, j, lane);
+    if (DC > 0) stage_blocks<L::SY>(Y, reinterpret_cast<const Real*>(s.p_YV), j, lane);
+    if constexpr (stores_products<Real>()) {
+      stage_blocks<L::SW>(W, (const float*)s.o_W, k, lane);
+    } else {
+      stage_blocks<L::SA>(A, reinterpret_cast<const double*>(s.o_A), k, lane);
+      stage_blocks<kSB>(B, (const double*)s.o_B, k, lane);
+    }
+    cp_join();
+    if constexpr (stores_products<Real>()) {
+#pragma unroll
+      for (int st = 0; st < 24; ++st) {
+        const int i = 4 * (st % 3) + kk, q = 4 * (st / 3) + i / 3, c = i % 3;
+        const double z = column(q, c);
+#pragma unroll
+        for (int t = 0; t < NT; ++t)
+          dmma884(acc[st & 1][t], 8 * t + r < DA ? double(W[q * L::SW + (8 * t + r) * 3 + c]) : 0.0, z);
+      }
+    } else {
+#pragma unroll
+      for (int st = 0; st < 16; ++st) {
+        const int q = 2 * st + (kk >> 1), rr = kk & 1;
+        const double* b = B + kSB * q + 3 * rr;
+        const double z = b[0] * column(q, 0) + b[1] * column(q, 1) + b[2] * column(q, 2);
+#pragma unroll
+        for (int t = 0; t < NT; ++t)
+          dmma884(acc[st & 1][t], 8 * t + r < DA ? A[q * L::SA + rr * DA + 8 * t + r] : 0.0, z);
+      }
+    }
+    __syncwarp();
+  }
+  double* out = part + (size_t)ch * RV::VP;
+#pragma unroll
+  for (int ta = 0; ta < NT; ++ta) {
+    const int R = 8 * ta + r;
+    if (R >= DA) continue;
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      const int col = 2 * kk + t;
+      const double v = acc[0][ta][t] + acc[1][ta][t];
+      if (col == 0) out[R] = v;
+      else if (DC > 0 && col <= DC) out[DA + R * DCc + col - 1] = v;
     }
   }
-  warp_reduce_transpose(acc);
-#pragma unroll
-  for (int t = 0; t < RV::VP / 32; ++t) part[(size_t)ch * RV::VP + lane * (RV::VP / 32) + t] = acc[t];
 }
 
 template <int DA, int DC, typename Real>
@@ -1020,9 +1438,7 @@ __device__ __forceinline__ void rhs_finish_body(DevState s, const double* __rest
   double sum[PER];
 #pragma unroll
   for (int t = 0; t < PER; ++t) sum[t] = 0.0;
-  for (int ch = s.cam_cc_ptr[i]; ch < s.cam_cc_ptr[i + 1]; ++ch)
-#pragma unroll
-    for (int t = 0; t < PER; ++t) sum[t] += cpart[(size_t)ch * RV::VP + lane + 32 * t];
+  sum_chunks<PER, RV::VP>(sum, cpart, s.cam_cc_ptr[i], s.cam_cc_ptr[i + 1], lane);
   const Real* cX = reinterpret_cast<const Real*>(s.c_X) + (size_t)i * L::SX;
 #pragma unroll
   for (int t = 0; t < PER; ++t) {
@@ -1044,33 +1460,35 @@ __global__ void __launch_bounds__(kCamWarps * 32) k_rhs_finish(DevState s, const
   rhs_finish_body<DA, DC, Real>(s, cpart, blockIdx.x, gridDim.x);
 }
 
-// Global block: S_cc = Z + lambda I - sum_j Y_j^T Vinv_j Y_j, rhs_c = gc - sum_j Y_j^T q_j.
+// Global block: S_cc = Z + lambda I - sum_j Y_j^T Vinv_j Y_j, rhs_c = gc - sum_j Y_j^T q_j.  One warp per
+// value (the elements are independent): global_blocks(DC) blocks of four warps instead of one block for
+// all 35 values of DC = 7, whose fold was the longest part of the finishing launch.
+__host__ __device__ constexpr int global_blocks(int DC) { return DC > 0 ? (nsym(DC) + DC + 3) / 4 : 0; }
 template <int DA, int DC>
 __device__ __forceinline__ void global_block_body(DevState s, const double* __restrict__ part, int nbp, int bid, int nblk) {
   constexpr int NV = ElimNV<DC>::NV;
   constexpr int DCc = DC > 0 ? DC : 1;
-  __shared__ double red[8 * NV];
-  double a[NV];
-  fold_partials<NV, NV>(part, nbp, a, red);
-  if (threadIdx.x == 0 && DC > 0) {
-    const Dims& D = s.d;
-    const double lam = *s.d_lambda;
-    const int c0 = D.N * DA;
-    const size_t ld = s.ld;
-    int z = 0;
-    for (int r = 0; r < DCc; ++r)
-      for (int c = r; c < DCc; ++c, ++z) {
-        double val;
-        if (r < D.nnC || c < D.nnC) val = (r == c) ? 1.0 : 0.0;
-        else val = s.g_Z[r * DCc + c] - a[z] + (r == c ? lam : 0.0);
-        s.S[(size_t)(c0 + r) * ld + (c0 + c)] = val;   // row c0+c >= col c0+r
-      }
-    for (int c = 0; c < DCc; ++c) s.rhs[(size_t)(c0 + c) * s.rhs_stride] = (c < D.nnC) ? 0.0 : s.g_gc[c] - a[nsym(DC) + c];
+  const int t = 4 * bid + (threadIdx.x >> 5);
+  if (DC == 0 || t >= NV) return;
+  const double a = warp_fold<true>(part + (size_t)t * nbp, nbp);
+  if ((threadIdx.x & 31) != 0) return;
+  const Dims& D = s.d;
+  const int c0 = D.N * DA;
+  if (t < nsym(DC)) {
+    int r, c;
+    unpack_sym<DCc>(t, r, c);
+    double val;
+    if (r < D.nnC || c < D.nnC) val = (r == c) ? 1.0 : 0.0;
+    else val = s.g_Z[r * DCc + c] - a + (r == c ? *s.d_lambda : 0.0);
+    s.S[(size_t)(c0 + r) * s.ld + (c0 + c)] = val;   // row c0+c >= col c0+r
+  } else {
+    const int c = t - nsym(DC);
+    s.rhs[(size_t)(c0 + c) * s.rhs_stride] = (c < D.nnC) ? 0.0 : s.g_gc[c] - a;
   }
 }
 
 template <int DA, int DC>
-__global__ void __launch_bounds__(256) k_global_block(DevState s, const double* __restrict__ part, int nbp) {
+__global__ void __launch_bounds__(128) k_global_block(DevState s, const double* __restrict__ part, int nbp) {
   pdl_wait();      // the previous stage's writes are visible
   pdl_trigger();   // the next stage may be scheduled once all blocks of this one are resident
   global_block_body<DA, DC>(s, part, nbp, blockIdx.x, gridDim.x);
@@ -1257,16 +1675,31 @@ __global__ void __launch_bounds__(128) k_camera_update(DevState s, double* __res
 // stage's own kernel (block index and count of its range), so the results are the same bits.
 
 // Schur chunks (blocks [0, g1)) and reduced-rhs chunks: both read only the elimination's output.
-template <int DA, int DC, typename Real>
+template <int DA, int DC, typename Real, bool DIRECT>
 __global__ void __launch_bounds__(128) k_chunks_merged(DevState s, int g1, int g2) {
   pdl_wait();
   pdl_trigger();
-  if ((int)blockIdx.x < g1) schur_chunks_body<DA, Real>(s, s.part_bc, blockIdx.x, g1);
+  if ((int)blockIdx.x < g1) schur_chunks_body<DA, Real, DIRECT>(s, s.part_bc, blockIdx.x, g1);
   else rhs_chunks_body<DA, DC, Real>(s, s.part_cc, blockIdx.x - g1, g2);
 }
 
+// Grouped Schur sums (blocks [0, g1)) and reduced-rhs chunks, FP64 blocks.  A block of rhs chunks uses the
+// first warps that find room for their tiles in the shared memory of a group.
+template <int DA, int DC>
+__host__ __device__ constexpr int group_rhs_warps() {
+  constexpr int bytes = rhs_stage_bytes<DA, DC, double>(), most = kGroupThreads / 32;
+  return bytes * most <= kGroupSmem ? most : kGroupSmem / (bytes > 0 ? bytes : 1);
+}
+template <int DA, int DC>
+__global__ void __launch_bounds__(kGroupThreads, DA <= 9 ? 3 : 2) k_groups_merged(DevState s, int g1, int g2) {
+  pdl_wait();
+  pdl_trigger();
+  if ((int)blockIdx.x < g1) schur_group_body<DA>(s, blockIdx.x);
+  else rhs_chunks_body<DA, DC, double, group_rhs_warps<DA, DC>()>(s, s.part_cc, blockIdx.x - g1, g2);
+}
+
 // Schur finish (blocks [0, g1)), rhs / border finish ([g1, g1 + g2)) and, with global
-// parameters, the global block (the last block): they write disjoint parts of S and rhs.
+// parameters, the global block (the last blocks): they write disjoint parts of S and rhs.
 template <int DA, int DC, typename Real>
 __global__ void __launch_bounds__(128) k_finish_merged(DevState s, int g1, int g2, const double* __restrict__ pelim,
                                                        int nbp) {
@@ -1275,7 +1708,7 @@ __global__ void __launch_bounds__(128) k_finish_merged(DevState s, int g1, int g
   const int b = blockIdx.x;
   if (b < g1) schur_finish_body<DA, Real>(s, s.part_bc, b, g1, true);
   else if (b < g1 + g2) rhs_finish_body<DA, DC, Real>(s, s.part_cc, b - g1, g2);
-  else global_block_body<DA, DC>(s, pelim, nbp, 0, 1);
+  else global_block_body<DA, DC>(s, pelim, nbp, b - g1 - g2, global_blocks(DC));
 }
 
 // Camera (and global) update (blocks [0, g1)) and point back-substitution: both read the
@@ -1314,26 +1747,38 @@ __global__ void __launch_bounds__(256) k_obs_cost(DevState s, ParamSet P, int re
   if (threadIdx.x == 0) part[blockIdx.x] = v[0];
 }
 
-__global__ void __launch_bounds__(256) k_trial_finalize(DevState s, const double* __restrict__ pb, int nbp,
-                                                        const double* __restrict__ pc, int nbc,
-                                                        const double* __restrict__ po, int nbo) {
+// The trial's scalars: the points' |db|^2 and db.gb (two values of nbp partials), the cameras' (two of
+// nbc) and the cost (nbo), folded side by side by eight, one and fourteen warps a value.
+__global__ void __launch_bounds__(32 * kFoldWarps) k_trial_finalize(DevState s, const double* __restrict__ pb, int nbp,
+                                                                    const double* __restrict__ pc, int nbc,
+                                                                    const double* __restrict__ po, int nbo) {
   pdl_wait();      // the previous stage's writes are visible
   pdl_trigger();   // the next stage may be scheduled once all blocks of this one are resident
-  __shared__ double red[8 * 2];
-  double a[2], b[2], c[1];
-  fold_partials<2, 2>(pb, nbp, a, red);
-  fold_partials<2, 2>(pc, nbc, b, red);
-  fold_partials<1, 1>(po, nbo, c, red);
+  __shared__ double red[kFoldWarps];
+  const int w = threadIdx.x >> 5;
+  const double* p = w < 16 ? pb + (size_t)(w >> 3) * nbp : w < 18 ? pc + (size_t)(w - 16) * nbc : po;
+  const int n = w < 16 ? nbp : w < 18 ? nbc : nbo, segs = w < 16 ? 8 : w < 18 ? 1 : 14;
+  const int at = w < 16 ? (w & 7) : w < 18 ? 0 : w - 18;
+  const int len = (n + segs - 1) / segs, b0 = min(at * len, n);
+  const double v = warp_fold<true>(p + b0, min(len, n - b0));
+  if ((threadIdx.x & 31) == 0) red[w] = v;
+  __syncthreads();
   if (threadIdx.x == 0) {
-    s.d_trial[0] = c[0];
-    s.d_trial[1] = a[0] + b[0];
-    s.d_trial[2] = a[1] + b[1];
+    double d2 = 0.0, dg = 0.0, c = 0.0;
+    for (int u = 0; u < 8; ++u) {
+      d2 += red[u];
+      dg += red[8 + u];
+    }
+    for (int u = 18; u < kFoldWarps; ++u) c += red[u];
+    s.d_trial[0] = c;
+    s.d_trial[1] = d2 + red[16];
+    s.d_trial[2] = dg + red[17];
     s.d_trial[3] = *s.d_fail != 0 ? 1.0 : 0.0;   // every kernel that can fail ran before this one
   }
 }
 
-__global__ void __launch_bounds__(256) k_sum_to(const double* __restrict__ po, int nbo, double* out) {
-  __shared__ double red[8];
+__global__ void __launch_bounds__(32 * kFoldWarps) k_sum_to(const double* __restrict__ po, int nbo, double* out) {
+  __shared__ double red[kFoldWarps];
   double c[1];
   fold_partials<1, 1>(po, nbo, c, red);
   if (threadIdx.x == 0) *out = c[0];
@@ -1368,22 +1813,38 @@ inline PartLayout part_layout(const DevState& s) {
 
 template <int MODEL, int DA, int DC, typename Real>
 struct Ops {
-  static bool grouped(const DevState& s) { return !stores_products<Real>() && s.gr_n > 0; }
-  static cudaError_t launch_groups(const DevState& s, cudaStream_t st) {
-    // the groups' shared memory, allowed on the current device the first time it is used there
+  // Shared memory of the staged kernels, allowed on the current device the first time it is asked for.
+  static constexpr size_t kCamSmem = (size_t)kCamWarps * camera_stage_bytes<DA, DC, Real>();
+  static constexpr size_t kRhsSmem = (size_t)kCamWarps * rhs_stage_bytes<DA, DC, Real>();
+  static constexpr size_t kSchurSmem = (size_t)4 * schur_stage_bytes<DA, Real>();
+  static constexpr size_t kBothSmem = kRhsSmem > kSchurSmem ? kRhsSmem : kSchurSmem;
+  static void allow_stages() {
     static std::atomic<uint64_t> allowed{0};
     int dev = 0;
     cudaGetDevice(&dev);
     const uint64_t bit = 1ull << (dev & 63);
-    if (!(allowed.load() & bit)) {
-      const cudaError_t e = cudaFuncSetAttribute(k_schur_groups<DA>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGroupSmem);
-      if (e != cudaSuccess) return e;
-      allowed.fetch_or(bit);
+    if (allowed.load() & bit) return;
+    constexpr auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaFuncSetAttribute(k_camera_chunks<DA, DC, Real>, attr, (int)kCamSmem);
+    cudaFuncSetAttribute(k_rhs_chunks<DA, DC, Real>, attr, (int)kRhsSmem);
+    cudaFuncSetAttribute(k_schur_chunks<DA, Real, false>, attr, (int)kSchurSmem);
+    cudaFuncSetAttribute(k_chunks_merged<DA, DC, Real, false>, attr, (int)kBothSmem);
+    cudaFuncSetAttribute(k_chunks_merged<DA, DC, Real, true>, attr, (int)kRhsSmem);
+    if (!stores_products<Real>()) {
+      cudaFuncSetAttribute(k_schur_groups<DA>, attr, kGroupSmem);
+      cudaFuncSetAttribute(k_groups_merged<DA, DC>, attr, kGroupSmem);
     }
-    return launch_pdl(k_schur_groups<DA>, dim3(s.gr_n), dim3(kGroupThreads), (size_t)s.gr_smem, st, s);
+    allowed.fetch_or(bit);
+  }
+  static bool grouped(const DevState& s) { return !stores_products<Real>() && s.gr_n > 0; }
+  // shared memory of the grouped launches: a group's, or the rhs chunks' of one block if that is more
+  static size_t group_smem(const DevState& s) {
+    constexpr size_t rhs = (size_t)group_rhs_warps<DA, DC>() * rhs_stage_bytes<DA, DC, double>();
+    return std::max((size_t)s.gr_smem, rhs);
   }
   // Launches one stage of the LM iteration (see LmStage in lm.cuh).
   static int stage(DevState& s, int id, int init_lambda, double tau, cudaStream_t st) {
+    allow_stages();
     const PartLayout pl = part_layout<DA, DC>(s);
     const int bp = cdiv(std::max(s.d.M, 1), kPtThreads);                  // one lane per point
     const int bl = lane_blocks(s.d.M, kLinLanes);                          // the linearisation
@@ -1398,7 +1859,7 @@ struct Ops {
         break;
       case kStageCameraChunks:
         if (s.nch_cam == 0) return V3DBA_OK;
-        e = launch_pdl(k_camera_chunks<DA, DC, Real>, dim3(cdiv(s.nch_cam, kCamWarps)), dim3(kCamWarps * 32), 0, st, s,
+        e = launch_pdl(k_camera_chunks<DA, DC, Real>, dim3(cdiv(s.nch_cam, kCamWarps)), dim3(kCamWarps * 32), kCamSmem, st, s,
                        s.part_cc);
         break;
       case kStageCameraFinish:
@@ -1406,19 +1867,25 @@ struct Ops {
                        s.part + pl.relin_cam);
         break;
       case kStageRelinFinalize:
-        e = launch_pdl(k_relin_finalize<DC>, dim3(1), dim3(256), 0, st, s, (const double*)(s.part + pl.relin_pt), bl,
+        e = launch_pdl(k_relin_finalize<DC>, dim3(1), dim3(32 * kFoldWarps), 0, st, s, (const double*)(s.part + pl.relin_pt), bl,
                        (const double*)(s.part + pl.relin_cam), bc, init_lambda, tau);
         break;
       case kStagePointEliminate:
-        e = launch_pdl(k_point_eliminate<DA, DC, Real>, dim3(bp), dim3(kPtThreads), 0, st, s, s.part + pl.elim);
+        e = launch_pdl(k_point_eliminate<DA, DC, Real>,
+                       dim3(bp + (stores_products<Real>() ? cdiv(s.d.K, kPtThreads) : 0)), dim3(kPtThreads), 0, st, s,
+                       s.part + pl.elim, bp);
         break;
       case kStageSchurChunks:
         if (grouped(s)) {
-          e = launch_groups(s, st);
+          e = launch_pdl(k_schur_groups<DA>, dim3(s.gr_n), dim3(kGroupThreads), (size_t)s.gr_smem, st, s);
           break;
         }
         if (s.nch_blk == 0) return V3DBA_OK;
-        e = launch_pdl(k_schur_chunks<DA, Real>, dim3(cdiv(s.nch_blk, 4)), dim3(128), 0, st, s, s.part_bc);
+        if (schur_direct<DA, Real>(s))
+          e = launch_pdl(k_schur_chunks<DA, Real, true>, dim3(cdiv(s.nch_blk, 4)), dim3(128), 0, st, s, s.part_bc);
+        else
+          e = launch_pdl(k_schur_chunks<DA, Real, false>, dim3(cdiv(s.nch_blk, 4)), dim3(128), kSchurSmem, st, s,
+                         s.part_bc);
         break;
       case kStageSchurFinish:
         if (s.nb == 0) return V3DBA_OK;
@@ -1427,7 +1894,7 @@ struct Ops {
         break;
       case kStageRhsChunks:
         if (s.nch_cam == 0) return V3DBA_OK;
-        e = launch_pdl(k_rhs_chunks<DA, DC, Real>, dim3(cdiv(s.nch_cam, kCamWarps)), dim3(kCamWarps * 32), 0, st, s,
+        e = launch_pdl(k_rhs_chunks<DA, DC, Real>, dim3(cdiv(s.nch_cam, kCamWarps)), dim3(kCamWarps * 32), kRhsSmem, st, s,
                        s.part_cc);
         break;
       case kStageRhsFinish:
@@ -1435,7 +1902,7 @@ struct Ops {
         break;
       case kStageGlobalBlock:
         if (DC == 0) return V3DBA_OK;
-        e = launch_pdl(k_global_block<DA, DC>, dim3(1), dim3(256), 0, st, s, (const double*)(s.part + pl.elim), bp);
+        e = launch_pdl(k_global_block<DA, DC>, dim3(global_blocks(DC)), dim3(128), 0, st, s, (const double*)(s.part + pl.elim), bp);
         break;
       case kStagePointBacksub:
         e = launch_pdl(k_point_backsub<DA, DC, Real>, dim3(bb), dim3(kPtThreads), 0, st, s, s.part + pl.backsub);
@@ -1447,7 +1914,7 @@ struct Ops {
         e = launch_pdl(k_obs_cost<MODEL>, dim3(bo), dim3(256), 0, st, s, (ParamSet)s.trial, 0, s.part + pl.obs);
         break;
       case kStageTrialFinalize:
-        e = launch_pdl(k_trial_finalize, dim3(1), dim3(256), 0, st, s, (const double*)(s.part + pl.backsub), bb,
+        e = launch_pdl(k_trial_finalize, dim3(1), dim3(32 * kFoldWarps), 0, st, s, (const double*)(s.part + pl.backsub), bb,
                        (const double*)(s.part + pl.camupd), bu, (const double*)(s.part + pl.obs), bo);
         break;
       default:
@@ -1486,14 +1953,23 @@ struct Ops {
     int rc = stage(s, kStagePointEliminate, 0, 0.0, st);
     if (rc) return rc;
     const PartLayout pl = part_layout<DA, DC>(s);
-    if (grouped(s) && (rc = launched(launch_groups(s, st)))) return rc;
-    const int g1 = !grouped(s) && s.nch_blk > 0 ? cdiv(s.nch_blk, 4) : 0, g2 = s.nch_cam > 0 ? cdiv(s.nch_cam, kCamWarps) : 0;
-    if (g1 + g2 > 0 && (rc = launched(launch_pdl(k_chunks_merged<DA, DC, Real>, dim3(g1 + g2), dim3(128), 0, st, s,
-                                                 g1, g2))))
-      return rc;
+    if (grouped(s)) {
+      const int g2 = cdiv(s.nch_cam, group_rhs_warps<DA, DC>());
+      if ((rc = launched(launch_pdl(k_groups_merged<DA, DC>, dim3(s.gr_n + g2), dim3(kGroupThreads), group_smem(s), st, s,
+                                    s.gr_n, g2))))
+        return rc;
+    } else {
+      const int g1 = s.nch_blk > 0 ? cdiv(s.nch_blk, 4) : 0, g2 = s.nch_cam > 0 ? cdiv(s.nch_cam, kCamWarps) : 0;
+      const bool direct = g1 == 0 || schur_direct<DA, Real>(s);   // (without Schur chunks, the smaller shared memory)
+      const cudaError_t e =
+          g1 + g2 == 0 ? cudaSuccess
+          : direct ? launch_pdl(k_chunks_merged<DA, DC, Real, true>, dim3(g1 + g2), dim3(128), kRhsSmem, st, s, g1, g2)
+                   : launch_pdl(k_chunks_merged<DA, DC, Real, false>, dim3(g1 + g2), dim3(128), kBothSmem, st, s, g1, g2);
+      if (g1 + g2 > 0 && (rc = launched(e))) return rc;
+    }
     const int f1 = grouped(s) ? s.nb : s.nb > 0 ? cdiv(s.nb, 4) : 0, f2 = cdiv(std::max(s.d.N, 1), kCamWarps);
     const int bp = cdiv(std::max(s.d.M, 1), kPtThreads);
-    return launched(launch_pdl(k_finish_merged<DA, DC, Real>, dim3(f1 + f2 + (DC > 0 ? 1 : 0)), dim3(128), 0, st, s,
+    return launched(launch_pdl(k_finish_merged<DA, DC, Real>, dim3(f1 + f2 + global_blocks(DC)), dim3(128), 0, st, s,
                                f1, f2, (const double*)(s.part + pl.elim), bp));
   }
   // camera update and point back-substitution in one launch, then the trial cost and the step
@@ -1511,7 +1987,7 @@ struct Ops {
     const int bo = cdiv(std::max(s.d.K, 1), 256);
     k_obs_cost<MODEL><<<bo, 256, 0, st>>>(s, P, 1, s.part + pl.obs);
     V3DBA_LAUNCH_CHECK();
-    k_sum_to<<<1, 256, 0, st>>>(s.part + pl.obs, bo, d_out);
+    k_sum_to<<<1, 32 * kFoldWarps, 0, st>>>(s.part + pl.obs, bo, d_out);
     V3DBA_LAUNCH_CHECK();
     return V3DBA_OK;
   }

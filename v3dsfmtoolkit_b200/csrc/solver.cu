@@ -272,9 +272,6 @@ struct Chunks {
   std::vector<int> cc_beg, cc_end, cam_cc_ptr, bc_beg, bc_end, blk_bc_ptr;
 };
 
-constexpr int kCamChunk = 64;     // observations per camera work chunk
-constexpr int kPairChunk = 128;   // observation pairs per camera-pair work chunk
-
 void build_chunks(const std::vector<int>& c_ptr, const std::vector<int>& b_ptr, int N, Chunks& S) {
   S.cam_cc_ptr.assign(1, 0);
   for (int i = 0; i < N; ++i) {
@@ -467,6 +464,10 @@ int v3dba_create(const v3dba_problem* p, v3dba_handle* out) {
   s.b_ptr = ds.b_ptr;
   s.pr_k = ds.pr_k;
   s.pr_m = ds.pr_m;
+  int64_t own = 0;
+  for (int b = 0; b < s.nb; ++b)
+    if (ds.h_b_i[b] == ds.h_b_l[b]) own += ds.h_b_ptr[b + 1] - ds.h_b_ptr[b];
+  s.repeats = 2 * own >= 3 * (int64_t)K;
   if (stereo) {   // rig cameras, and the rig camera of every point-major observation
     std::vector<double> rig((size_t)std::max(nrig, 1) * kRigStride, 0.0);
     for (int l = 0; l < nrig; ++l) {

@@ -735,7 +735,7 @@ int build_schur_groups(DevState& s, const DevAlloc& alloc, cudaStream_t st) {
   V3DBA_CUDA_TRY(cudaMemcpyAsync(&head[1], info, sizeof(int), cudaMemcpyDeviceToHost, st));
   V3DBA_CUDA_TRY(cudaStreamSynchronize(st));
   const int G = head[0];
-  if (head[1] > kGroupTrack || (!force && (int64_t)4 * G > M)) return V3DBA_OK;
+  if (head[1] > kGroupTrack || (!force && (int64_t)8 * G > M)) return V3DBA_OK;
   if ((rc = sc.get(&info, 2 * (size_t)G))) return rc;
   k_group_info<<<g, 256, 0, st>>>(flag, gid, va, s.p_ptr, s.o_cam, M, info);
   V3DBA_LAUNCH_CHECK();
@@ -764,10 +764,10 @@ int build_schur_groups(DevState& s, const DevAlloc& alloc, cudaStream_t st) {
     }
   }
   // A partial sum is written and read back where a pair gathers 340 bytes, and a chunk pays for 8 x 8
-  // tiles and whole DMMA steps: the two are level at about four pairs a sum (200 cameras, pairs against
-  // groups with their finish: 4,000 points 20.7 / 26.6 us, 8,000 points (4.2 pairs a sum) 30.0 / 30.1,
-  // 16,000 points 48.0 / 34.5, 50,000 points 122.9 / 54.8).
-  if (chunks.empty() || entries > 0x3fffffff || (!force && 4 * entries > s.P)) return V3DBA_OK;
+  // tiles and whole DMMA steps: worth it from about ten pairs a sum on (158 cameras, us per iteration, pairs
+  // against groups: 9,981 points, 6 pairs a sum, 308 / 314; 16,000 points, 10 pairs, 319 / 326; 24,000
+  // points, 14 pairs, 363 / 337).
+  if (chunks.empty() || entries > 0x3fffffff || (!force && 10 * entries > s.P)) return V3DBA_OK;
   // the costly chunks first, so that the last ones to run are short
   std::stable_sort(chunks.begin(), chunks.end(),
                    [](const Chunk& a, const Chunk& b) { return a.L * a.L * a.points > b.L * b.L * b.points; });
