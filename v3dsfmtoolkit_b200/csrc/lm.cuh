@@ -17,6 +17,7 @@ struct ParamSet {
   double* T = nullptr;     // N*3
   double* dist = nullptr;  // COMMON: 4, VARYING: N*4, STD: 4 (unused)
   double* X = nullptr;     // M*3
+  double* pack = nullptr;  // N packed records (cam_stride) of K, R, T, dist: written with them
 };
 
 struct Dims {
@@ -167,6 +168,8 @@ struct LmOps {
   int (*build_reduced)(DevState&, cudaStream_t);
   // back-substitution, trial parameters and their cost with frozen weights -> d_trial
   int (*finish_trial)(DevState&, cudaStream_t);
+  // packs the cameras of the given parameters (after K, R, T or dist were written from outside)
+  int (*pack)(DevState&, const ParamSet&, cudaStream_t);
   // cost with Huber weights recomputed at the given parameters -> out[0]
   int (*cost)(DevState&, const ParamSet&, double* d_out, cudaStream_t);
   // one stage by id (LmStage)

@@ -106,6 +106,7 @@ int alloc_params(v3dba_handle h, ParamSet& P, int N, int M) {
   if ((rc = dalloc(h, &P.T, (size_t)N * 3))) return rc;
   if ((rc = dalloc(h, &P.dist, std::max<size_t>(h->nD, 4)))) return rc;
   if ((rc = dalloc(h, &P.X, (size_t)M * 3))) return rc;
+  if ((rc = dalloc(h, &P.pack, (size_t)N * cam_stride(h->s.d.model)))) return rc;
   return V3DBA_OK;
 }
 
@@ -116,18 +117,23 @@ int copy_params(const ParamSet& dst, const ParamSet& src, const v3dba_handle h, 
   V3DBA_CUDA_TRY(cudaMemcpyAsync(dst.T, src.T, sizeof(double) * 3 * D.N, cudaMemcpyDeviceToDevice, st));
   if (h->nD) V3DBA_CUDA_TRY(cudaMemcpyAsync(dst.dist, src.dist, sizeof(double) * h->nD, cudaMemcpyDeviceToDevice, st));
   V3DBA_CUDA_TRY(cudaMemcpyAsync(dst.X, src.X, sizeof(double) * 3 * D.M, cudaMemcpyDeviceToDevice, st));
+  V3DBA_CUDA_TRY(cudaMemcpyAsync(dst.pack, src.pack, sizeof(double) * cam_stride(D.model) * (size_t)D.N,
+                                 cudaMemcpyDeviceToDevice, st));
   return V3DBA_OK;
 }
 
 int copy_params_up(v3dba_handle h, const ParamSet& P, const double* K, const double* R, const double* T,
                    const double* dist, const double* X) {
   const Dims& D = h->s.d;
-  return copy_up({{P.K, K, sizeof(double) * h->nK},
+  const int rc = copy_up({{P.K, K, sizeof(double) * h->nK},
                           {P.R, R, sizeof(double) * 9 * (size_t)D.N},
                           {P.T, T, sizeof(double) * 3 * (size_t)D.N},
                           {P.dist, dist, sizeof(double) * h->nD},
                           {P.X, X, sizeof(double) * 3 * (size_t)D.M}},
                          h->stream);
+  if (rc) return rc;
+  const LmOps* ops = lm_ops(D.model, D.DA, D.DC, true);
+  return ops ? ops->pack(h->s, P, h->stream) : V3DBA_ERR_UNSUPPORTED;
 }
 
 int upload_params(v3dba_handle h, const ParamSet& P, const double* K, const double* R, const double* T,
