@@ -19,6 +19,7 @@
 #include <cstdio>
 
 #include "common.cuh"
+#include "async_copy.cuh"
 #include "lm.cuh"
 #include "model.cuh"
 
@@ -230,22 +231,6 @@ __device__ __forceinline__ void unpack_sym(int u, int& r, int& c) {
 // L1's wavefronts, not bandwidth, set the time.  So a warp copies the blocks of 32 list entries to shared
 // memory together, consecutive lanes on consecutive 16 bytes of a block, and contracts them with DMMA where
 // the sums are FP64: two doubles of accumulator per lane and tile instead of 28 to 112.
-
-// 16 bytes global -> shared; zeros when !use.
-__device__ __forceinline__ void cp16(void* dst, const void* src, bool use) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(use ? 16 : 0) : "memory");
-}
-__device__ __forceinline__ void cp_join() {
-  asm volatile("cp.async.wait_all;\n" ::: "memory");
-  __syncwarp();
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-// All copies but those of the last group have arrived.
-__device__ __forceinline__ void cp_join_but_last() {
-  asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-  __syncwarp();
-}
 
 // Copies block `idx` (each lane's own; negative: zeros) of STRIDE values for the warp's 32 pairs:
 // dst[pair * STRIDE + t] = src[idx(pair) * STRIDE + t].

@@ -39,10 +39,12 @@ struct GnnGraph {
   int* lo_e = nullptr;
   int* up_ptr = nullptr;   // [N+1] edges (a, b) with a == node, ordered by b
   int* up_e = nullptr;
-  int* tri_ptr = nullptr;  // [ne+1] two-hop products of each edge
-  int* tri_1 = nullptr;
-  int* tri_2 = nullptr;
-  unsigned char* tri_t = nullptr;   // 0: F(e1) F(e2); 1: F(e1) F(e2)^T
+  int* tri_ptr = nullptr;  // [ne+1] two-hop products of each edge (a, b): first F(e1) F(e2),
+  int* tri_mid = nullptr;  // [ne] from here on F(e1) F(e2)^T
+  int* tri_1 = nullptr;    // place of e1 in the lower list of b
+  int* tri_2 = nullptr;    // e2
+  int nhop = 0, max_lo = 0;
+  int2* hop = nullptr;     // [nhop] up to 40 edges of one lower list: (b, first place)
 };
 
 int gnn_graph_build(GnnGraph& g, int N, const std::vector<int>& b_i, const std::vector<int>& b_l);

@@ -33,6 +33,7 @@
 #include <random>
 #include <vector>
 
+#include "async_copy.cuh"
 #include "common.cuh"
 #include "lm.cuh"
 #include "precond.cuh"
@@ -41,6 +42,9 @@ namespace v3dba {
 namespace {
 
 inline int cdiv(long a, long b) { return (int)((a + b - 1) / b); }
+
+// k_gnn_two_hop: edges per warp and per block, products in flight per edge, blocks of a row held in shared memory
+constexpr int kHopGroups = 5, kHopWarps = 8, kHopEdges = kHopGroups * kHopWarps, kHopDepth = 4, kHopRow = 256;
 
 template <typename T>
 int upload_vec(T** d, const std::vector<T>& h) {
@@ -80,8 +84,7 @@ int gnn_graph_build(GnnGraph& g, int N, const std::vector<int>& b_i, const std::
   // two-hop products of edge (a, b), the lower position (b, a):
   //   (F F)_(b,a)   = sum over a < k < b of F_(b,k) F_(k,a): edges (k, b) and (a, k)
   //   (F F^T)_(b,a) = sum over k < a of F_(b,k) F_(a,k)^T:  edges (k, b) and (k, a)
-  std::vector<int> tri_ptr(1, 0), t1, t2;
-  std::vector<unsigned char> tt;
+  std::vector<int> tri_ptr(1, 0), tri_mid, t1, t2;
   for (int e = 0; e < ne; ++e) {
     const int a = ea[e], b = eb[e];
     int p = up_ptr[a], q = lo_ptr[b];
@@ -90,33 +93,43 @@ int gnn_graph_build(GnnGraph& g, int N, const std::vector<int>& b_i, const std::
       if (kp < kq) ++p;
       else if (kq < kp) ++q;
       else {
-        if (kp < b) { t1.push_back(lo_e[q]); t2.push_back(up_e[p]); tt.push_back(0); }
+        if (kp < b) { t1.push_back(q - lo_ptr[b]); t2.push_back(up_e[p]); }
         ++p; ++q;
       }
     }
+    tri_mid.push_back((int)t1.size());
     p = lo_ptr[a]; q = lo_ptr[b];
     while (p < lo_ptr[a + 1] && q < lo_ptr[b + 1]) {
       const int kp = ea[lo_e[p]], kq = ea[lo_e[q]];
       if (kp < kq) ++p;
       else if (kq < kp) ++q;
-      else { t1.push_back(lo_e[q]); t2.push_back(lo_e[p]); tt.push_back(1); ++p; ++q; }
+      else { t1.push_back(q - lo_ptr[b]); t2.push_back(lo_e[p]); ++p; ++q; }
     }
     tri_ptr.push_back((int)t1.size());
   }
+  std::vector<int2> hop;
+  int max_lo = 0;
+  for (int b = 0; b < N; ++b) {
+    const int n = lo_ptr[b + 1] - lo_ptr[b];
+    max_lo = std::max(max_lo, n);
+    for (int q = 0; q < n; q += kHopEdges) hop.push_back(make_int2(b, q));
+  }
   gnn_graph_free(g);
+  g.nhop = (int)hop.size(); g.max_lo = max_lo;
   g.N = N; g.ne = ne; g.ntri = (int)t1.size();
   int rc;
   if ((rc = upload_vec(&g.ea, ea)) || (rc = upload_vec(&g.eb, eb)) || (rc = upload_vec(&g.eblk, eblk)) ||
       (rc = upload_vec(&g.lo_ptr, lo_ptr)) || (rc = upload_vec(&g.lo_e, lo_e)) || (rc = upload_vec(&g.up_ptr, up_ptr)) ||
       (rc = upload_vec(&g.up_e, up_e)) || (rc = upload_vec(&g.tri_ptr, tri_ptr)) || (rc = upload_vec(&g.tri_1, t1)) ||
-      (rc = upload_vec(&g.tri_2, t2)) || (rc = upload_vec(&g.tri_t, tt)))
+      (rc = upload_vec(&g.tri_2, t2)) || (rc = upload_vec(&g.tri_mid, tri_mid)) || (rc = upload_vec(&g.hop, hop)))
     return rc;
   return V3DBA_OK;
 }
 
 void gnn_graph_free(GnnGraph& g) {
   cudaFree(g.ea); cudaFree(g.eb); cudaFree(g.eblk); cudaFree(g.lo_ptr); cudaFree(g.lo_e); cudaFree(g.up_ptr);
-  cudaFree(g.up_e); cudaFree(g.tri_ptr); cudaFree(g.tri_1); cudaFree(g.tri_2); cudaFree(g.tri_t);
+  cudaFree(g.up_e); cudaFree(g.tri_ptr); cudaFree(g.tri_1); cudaFree(g.tri_2); cudaFree(g.tri_mid);
+  cudaFree(g.hop);
   g = GnnGraph();
 }
 
@@ -126,38 +139,72 @@ namespace {
 // normalisation and input features
 // --------------------------------------------------------------------------------------------
 
+// A 6x6 block in registers, in 16-byte loads and stores.
+__device__ __forceinline__ void load36(float (&v)[36], const float* p) {
+#pragma unroll
+  for (int t = 0; t < 9; ++t) {
+    const float4 x = reinterpret_cast<const float4*>(p)[t];
+    v[4 * t] = x.x; v[4 * t + 1] = x.y; v[4 * t + 2] = x.z; v[4 * t + 3] = x.w;
+  }
+}
+__device__ __forceinline__ void load36(double (&v)[36], const double* p) {
+#pragma unroll
+  for (int t = 0; t < 18; ++t) {
+    const double2 x = reinterpret_cast<const double2*>(p)[t];
+    v[2 * t] = x.x; v[2 * t + 1] = x.y;
+  }
+}
+__device__ __forceinline__ void store36(float* p, const float (&v)[36]) {
+#pragma unroll
+  for (int t = 0; t < 9; ++t) reinterpret_cast<float4*>(p)[t] = make_float4(v[4 * t], v[4 * t + 1], v[4 * t + 2], v[4 * t + 3]);
+}
+
 // C_i^-1 of the Cholesky factor of each diagonal block (FP64 arithmetic, stored FP32, lower).
 template <typename Real>
 __global__ void k_gnn_cinv(const Real* __restrict__ Sb, const int* __restrict__ diag_blk, int N, float* cinv,
                            int* fail) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
-  const Real* A = Sb + (size_t)diag_blk[i] * 36;
+  Real A[36];
+  load36(A, Sb + (size_t)diag_blk[i] * 36);
   double L[6][6], X[6][6];
   bool ok = true;
+  // (unrolled: the two blocks stay in registers; a serial chain, so one warp per block of threads)
+#pragma unroll
   for (int j = 0; j < 6; ++j) {
     double d = double(A[j * 6 + j]);
+#pragma unroll
     for (int k = 0; k < j; ++k) d -= L[j][k] * L[j][k];
     if (!(d > 0.0)) { ok = false; d = 1.0; }
     L[j][j] = sqrt(d);
+#pragma unroll
     for (int r = j + 1; r < 6; ++r) {
       double v = double(A[r * 6 + j]);
+#pragma unroll
       for (int k = 0; k < j; ++k) v -= L[r][k] * L[j][k];
       L[r][j] = v / L[j][j];
     }
   }
+#pragma unroll
   for (int c = 0; c < 6; ++c) {
+#pragma unroll
     for (int r = 0; r < c; ++r) X[r][c] = 0.0;
     X[c][c] = 1.0 / L[c][c];
+#pragma unroll
     for (int r = c + 1; r < 6; ++r) {
       double v = 0.0;
+#pragma unroll
       for (int k = c; k < r; ++k) v += L[r][k] * X[k][c];
       X[r][c] = -v / L[r][r];
     }
   }
   if (!ok) *fail = 1;
+  float o[36];
+#pragma unroll
   for (int r = 0; r < 6; ++r)
-    for (int c = 0; c < 6; ++c) cinv[(size_t)i * 36 + r * 6 + c] = float(X[r][c]);
+#pragma unroll
+    for (int c = 0; c < 6; ++c) o[r * 6 + c] = float(X[r][c]);
+  store36(cinv + (size_t)i * 36, o);
 }
 
 // F_e = C_b^-1 S_(b,a) C_a^-T, S_(b,a) the transpose of the stored block (a, b).
@@ -165,47 +212,110 @@ template <typename Real>
 __global__ void k_gnn_edge_norm(const Real* __restrict__ Sb, GnnGraph g, const float* __restrict__ cinv, float* xe) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= g.ne) return;
-  const Real* B = Sb + (size_t)g.eblk[e] * 36;
-  const float* Ca = cinv + (size_t)g.ea[e] * 36;
-  const float* Cb = cinv + (size_t)g.eb[e] * 36;
-  double T[6][6];
-  for (int r = 0; r < 6; ++r)          // T = S_(b,a) C_a^-T:  T[r][c] = sum_k B[k][r] Ca[c][k]
-    for (int c = 0; c < 6; ++c) {
+  Real B[36];
+  float Ca[36], Cb[36], o[36];
+  load36(B, Sb + (size_t)g.eblk[e] * 36);
+  load36(Ca, cinv + (size_t)g.ea[e] * 36);
+  load36(Cb, cinv + (size_t)g.eb[e] * 36);
+#pragma unroll
+  for (int c = 0; c < 6; ++c) {        // T = S_(b,a) C_a^-T:  T[r][c] = sum_k B[k][r] Ca[c][k]
+    double T[6];
+#pragma unroll
+    for (int r = 0; r < 6; ++r) {
       double v = 0.0;
+#pragma unroll
       for (int k = 0; k <= c; ++k) v += double(B[k * 6 + r]) * double(Ca[c * 6 + k]);
-      T[r][c] = v;
+      T[r] = v;
     }
-  for (int r = 0; r < 6; ++r)
-    for (int c = 0; c < 6; ++c) {
+#pragma unroll
+    for (int r = 0; r < 6; ++r) {
       double v = 0.0;
-      for (int k = 0; k <= r; ++k) v += double(Cb[r * 6 + k]) * T[k][c];
-      xe[(size_t)e * kGnnEdgeIn + r * 6 + c] = float(v);
-    }
-}
-
-// Two-hop products of every edge: 72 threads per edge, one per output entry (36 of (F F), 36 of
-// (F F^T)); the threads of an edge walk its triangles together and share their loads.
-__global__ void __launch_bounds__(288) k_gnn_two_hop(GnnGraph g, float* xe) {
-  const int e = blockIdx.x * 4 + threadIdx.y;
-  if (e >= g.ne) return;
-  const int o = threadIdx.x;                 // 0..71
-  const int kind = o >= 36 ? 1 : 0;
-  const int r = (o % 36) / 6, c = o % 6;
-  float acc = 0.f;
-  for (int t = g.tri_ptr[e]; t < g.tri_ptr[e + 1]; ++t) {
-    if (g.tri_t[t] != kind) continue;
-    const float* A = xe + (size_t)g.tri_1[t] * kGnnEdgeIn + r * 6;
-    const float* B = xe + (size_t)g.tri_2[t] * kGnnEdgeIn;
-    if (kind == 0) {
 #pragma unroll
-      for (int k = 0; k < 6; ++k) acc += A[k] * B[k * 6 + c];
-    } else {
-#pragma unroll
-      for (int k = 0; k < 6; ++k) acc += A[k] * B[c * 6 + k];
+      for (int k = 0; k <= r; ++k) v += double(Cb[r * 6 + k]) * T[k];
+      o[r * 6 + c] = float(v);
     }
   }
-  xe[(size_t)e * kGnnEdgeIn + 36 + o] = acc;
+  store36(xe + (size_t)e * kGnnEdgeIn, o);
 }
+
+// Two-hop products of the edges (a, b) of one node b, F F (KIND 0) or F F^T (KIND 1), in the order of the
+// lists.  Six lanes per edge, one row of the 6x6 sum each: a lane holds its row of F_(b,k), which the edges of
+// b share from shared memory, against the whole second block, which the warp copies there for its five edges
+// four products ahead.  The copies of the second blocks, 144 bytes per product from L2, bound it; with one
+// thread per entry of the sums, twelve 4-byte loads per six multiplications, the L1's wavefronts did
+// (44,000 edges of 800 cameras in clusters of about 110: 404 -> 182 us).
+template <int KIND>
+__device__ __forceinline__ void two_hop_body(const GnnGraph& g, float* xe, int row_cap, int tile) {
+  extern __shared__ float4 hop_sm[];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, grp = lane / 6, r = lane - 6 * grp;
+  const int2 d = g.hop[tile];
+  const int lo0 = g.lo_ptr[d.x], nlo = g.lo_ptr[d.x + 1] - lo0;
+  const bool staged = nlo <= row_cap;
+  float* row = reinterpret_cast<float*>(hop_sm);
+  float* ring = row + row_cap * 36 + w * (kHopDepth * kHopGroups * 36);
+  if (staged)
+    for (int t = tid; t < 9 * nlo; t += 32 * kHopWarps)
+      cp16(row + 4 * t, xe + (size_t)g.lo_e[lo0 + t / 9] * kGnnEdgeIn + 4 * (t % 9), true);
+  const int p = d.y + w * kHopGroups + grp;
+  const bool active = grp < kHopGroups && p < nlo;
+  const int e = active ? g.lo_e[lo0 + p] : 0;
+  const int t0 = active ? (KIND ? g.tri_mid[e] : g.tri_ptr[e]) : 0;
+  const int n = active ? (KIND ? g.tri_ptr[e + 1] : g.tri_mid[e]) - t0 : 0;
+  const int steps = __reduce_max_sync(0xffffffffu, n);
+  cp_join();
+  __syncthreads();
+  float acc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  int i1 = 0, i2 = -1;
+  auto copy = [&](int s) {
+    const int s6 = s % 6;
+    if (s6 == 0) i2 = s + r < n ? g.tri_2[t0 + s + r] : -1;
+    float* slot = ring + (s % kHopDepth) * (kHopGroups * 36);
+#pragma unroll
+    for (int v = 0; v < 2; ++v) {
+      const int c = lane + 32 * v, gg = min(c / 9, kHopGroups - 1);
+      const int e2 = __shfl_sync(0xffffffffu, i2, 6 * gg + s6);
+      if (c < 9 * kHopGroups && e2 >= 0) cp16(slot + 4 * c, xe + (size_t)e2 * kGnnEdgeIn + 4 * (c - 9 * gg), true);
+    }
+    cp_commit();
+  };
+#pragma unroll
+  for (int s = 0; s < kHopDepth - 1; ++s) copy(s);
+  for (int s = 0; s < steps; ++s) {
+    copy(s + kHopDepth - 1);
+    const int s6 = s % 6;
+    if (s6 == 0) i1 = s + r < n ? g.tri_1[t0 + s + r] : 0;
+    const int q = __shfl_sync(0xffffffffu, i1, min(6 * grp + s6, 31));
+    cp_join_but<kHopDepth - 1>();
+    if (s < n) {
+      const float2* Ar = reinterpret_cast<const float2*>((staged ? row + 36 * q : xe + (size_t)g.lo_e[lo0 + q] * kGnnEdgeIn) + 6 * r);
+      const float4* Bs = reinterpret_cast<const float4*>(ring + ((s % kHopDepth) * kHopGroups + grp) * 36);
+      float A[6], B[36];
+#pragma unroll
+      for (int t = 0; t < 3; ++t) { const float2 x = Ar[t]; A[2 * t] = x.x; A[2 * t + 1] = x.y; }
+#pragma unroll
+      for (int t = 0; t < 9; ++t) {
+        const float4 x = Bs[t];
+        B[4 * t] = x.x; B[4 * t + 1] = x.y; B[4 * t + 2] = x.z; B[4 * t + 3] = x.w;
+      }
+#pragma unroll
+      for (int k = 0; k < 6; ++k)
+#pragma unroll
+        for (int c = 0; c < 6; ++c) acc[c] += A[k] * (KIND ? B[6 * c + k] : B[6 * k + c]);
+    }
+    __syncwarp();   // this slot is copied to next
+  }
+  if (active) {
+    float2* out = reinterpret_cast<float2*>(xe + (size_t)e * kGnnEdgeIn + 36 + 36 * KIND + 6 * r);
+#pragma unroll
+    for (int t = 0; t < 3; ++t) out[t] = make_float2(acc[2 * t], acc[2 * t + 1]);
+  }
+  cp_join();
+}
+__global__ void __launch_bounds__(32 * kHopWarps) k_gnn_two_hop(GnnGraph g, float* xe, int row_cap) {
+  if (blockIdx.x & 1) two_hop_body<1>(g, xe, row_cap, blockIdx.x >> 1);
+  else two_hop_body<0>(g, xe, row_cap, blockIdx.x >> 1);
+}
+inline size_t hop_smem(int row_cap) { return sizeof(float) * 36 * ((size_t)row_cap + kHopWarps * kHopDepth * kHopGroups); }
 
 __device__ __forceinline__ int node_degree(const GnnGraph& g, int i) {
   return (g.lo_ptr[i + 1] - g.lo_ptr[i]) + (g.up_ptr[i + 1] - g.up_ptr[i]);
@@ -218,6 +328,7 @@ __global__ void k_gnn_node_feat(GnnGraph g, const float* __restrict__ xe, float*
   const int nlo = g.lo_ptr[i + 1] - g.lo_ptr[i];
   const int deg = node_degree(g, i);
   float sum = 0.f, mx = 0.f;
+#pragma unroll 4
   for (int q = lane; q < deg; q += 32) {
     const int e = q < nlo ? g.lo_e[g.lo_ptr[i] + q] : g.up_e[g.up_ptr[i] + q - nlo];
     const float4* F = reinterpret_cast<const float4*>(xe + (size_t)e * kGnnEdgeIn);
@@ -314,6 +425,37 @@ __global__ void __launch_bounds__(256) k_rowgemm(RowGemm g) {
   }
 }
 
+// Up to four outputs from one dense segment: a thread per row, the weights in shared memory (44,000 rows of 64:
+// 9.4 us; k_rowgemm, three of whose 64 columns of threads had work, 28).
+constexpr int kNarrow = 4;
+__global__ void __launch_bounds__(128) k_rows_narrow(RowGemm g) {
+  extern __shared__ float sm[];
+  for (int t = threadIdx.x; t < g.K * g.Nout; t += blockDim.x) {
+    const int k = t / g.Nout, c = t - k * g.Nout;
+    sm[kNarrow * k + c] = g.W[(size_t)k * g.wk + (size_t)c * g.wn];
+  }
+  __syncthreads();
+  const int row = blockIdx.x * blockDim.x + threadIdx.x;
+  if (row >= g.rows) return;
+  const float4* x = reinterpret_cast<const float4*>(g.seg[0].src + (size_t)row * g.seg[0].ld);
+  float acc[kNarrow];
+#pragma unroll
+  for (int c = 0; c < kNarrow; ++c) acc[c] = g.bias && c < g.Nout ? g.bias[c] : 0.f;
+#pragma unroll 8
+  for (int k = 0; k < g.K; k += 4) {
+    const float4 v = x[k / 4];
+    const float in[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int c = 0; c < kNarrow; ++c)
+        if (c < g.Nout) acc[c] += in[u] * sm[kNarrow * (k + u) + c];
+  }
+#pragma unroll
+  for (int c = 0; c < kNarrow; ++c)
+    if (c < g.Nout) g.out[(size_t)row * g.ldo + c] = g.relu ? fmaxf(acc[c], 0.f) : acc[c];
+}
+
 struct WGrad {
   int rows = 0, nseg = 0, K = 0, Nout = 0;
   Seg seg[3];
@@ -389,39 +531,52 @@ __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], const uint32_t (&a
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
-// out = act([segments] W + b) (+ resid) for 64-row tiles; Wt is W^T (64 x Kp, bf16, zero
-// padded).  Four warps, 16 rows each, eight 16x8 output tiles per warp.
-__global__ void __launch_bounds__(128) k_rowgemm_bf16(RowGemm g, const __nv_bfloat16* __restrict__ Wt, int Kp) {
+// out = act([segments] W + b) (+ resid) for 64-row tiles; Wt is W^T (64 x KP, bf16, zero
+// padded).  Four warps, 16 rows each, eight 16x8 output tiles per warp.  One segment of any width, or
+// NSEG of 64 columns.  Bound by the gather of the input rows: eight of a thread's 14 to 24 loads are in flight at
+// a time, their places from compile-time divisors (44,000 rows of 192: 66 -> 28 us).
+template <int KP, int NSEG>
+__global__ void __launch_bounds__(128) k_rowgemm_bf16(RowGemm g, const __nv_bfloat16* __restrict__ Wt) {
   extern __shared__ __align__(16) unsigned char smb[];
-  const int ld = Kp + 8;
+  constexpr int Kp = KP, ld = KP + 8;
+  static_assert(NSEG == 1 || KP == 64 * NSEG, "segments of 64 columns");
   __nv_bfloat16* a_s = reinterpret_cast<__nv_bfloat16*>(smb);
   __nv_bfloat16* b_s = a_s + 64 * ld;
   const int r0 = blockIdx.x * 64;
-  // weights: 8 bf16 per 16-byte copy (Kp is a multiple of 16, rows of b_s 16-byte aligned)
-  const int kq8 = Kp / 8;
-  for (int t = threadIdx.x; t < 64 * kq8; t += blockDim.x) {
-    const int n = t / kq8, k = (t - n * kq8) * 8;
-    *reinterpret_cast<uint4*>(b_s + n * ld + k) = *reinterpret_cast<const uint4*>(Wt + (size_t)n * Kp + k);
+  // weights: 8 bf16 per 16-byte copy (KP is a multiple of 16, rows of b_s 16-byte aligned)
+#pragma unroll
+  for (int v = 0; v < KP / 16; ++v) {
+    const int t = threadIdx.x + 128 * v, n = t / (KP / 8), k = (t - n * (KP / 8)) * 8;
+    cp16(b_s + n * ld + k, Wt + (size_t)n * KP + k, true);
   }
   // inputs: 4 floats per 16-byte load (segment widths and leading dimensions are multiples of 4)
-  const int kq4 = Kp / 4;
-  for (int t = threadIdx.x; t < 64 * kq4; t += blockDim.x) {
-    const int r = t / kq4, k = (t - r * kq4) * 4;
-    const int row = r0 + r;
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (row < g.rows && k < g.K) {
-      int sgi = 0, kk = k;
-      while (sgi + 1 < g.nseg && kk >= g.seg[sgi].width) { kk -= g.seg[sgi].width; ++sgi; }
+  constexpr int Q = KP / 4, PER = Q / 2, U = PER % 8 == 0 ? 8 : 7;
+  static_assert(PER % U == 0, "whole batches");
+#pragma unroll
+  for (int v0 = 0; v0 < PER; v0 += U) {
+    const float* src[U];
+    float4 x[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int t = threadIdx.x + 128 * (v0 + u), r = t / Q, k = (t - r * Q) * 4, row = r0 + r;
+      const int sgi = NSEG == 1 ? 0 : k / 64, kk = NSEG == 1 ? k : k % 64;
       const Seg& sg = g.seg[sgi];
-      const int src_row = sg.idx ? sg.idx[row] : row;
-      v = *reinterpret_cast<const float4*>(sg.src + (size_t)src_row * sg.ld + kk);
+      src[u] = nullptr;
+      if (row < g.rows && k < g.K) src[u] = sg.src + (size_t)(sg.idx ? sg.idx[row] : row) * sg.ld + kk;
     }
-    __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
-    uint2 pk;
-    pk.x = *reinterpret_cast<uint32_t*>(&lo);
-    pk.y = *reinterpret_cast<uint32_t*>(&hi);
-    *reinterpret_cast<uint2*>(a_s + r * ld + k) = pk;
+#pragma unroll
+    for (int u = 0; u < U; ++u) x[u] = src[u] ? *reinterpret_cast<const float4*>(src[u]) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int t = threadIdx.x + 128 * (v0 + u), r = t / Q, k = (t - r * Q) * 4;
+      __nv_bfloat162 lo = __floats2bfloat162_rn(x[u].x, x[u].y), hi = __floats2bfloat162_rn(x[u].z, x[u].w);
+      uint2 pk;
+      pk.x = *reinterpret_cast<uint32_t*>(&lo);
+      pk.y = *reinterpret_cast<uint32_t*>(&hi);
+      *reinterpret_cast<uint2*>(a_s + r * ld + k) = pk;
+    }
   }
+  cp_join();
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gq = lane >> 2, tq = lane & 3;
@@ -448,16 +603,21 @@ __global__ void __launch_bounds__(128) k_rowgemm_bf16(RowGemm g, const __nv_bflo
     }
   }
 #pragma unroll
-  for (int nt = 0; nt < 8; ++nt)
+  for (int h = 0; h < 2; ++h) {
+    const int row = r0 + warp * 16 + gq + 8 * h;
+    if (row >= g.rows) continue;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int row = r0 + warp * 16 + gq + (q >> 1) * 8;
-      const int c = nt * 8 + 2 * tq + (q & 1);
-      if (row >= g.rows) continue;
-      float z = acc[nt][q] + (g.bias ? g.bias[c] : 0.f);
-      if (g.relu) z = fmaxf(z, 0.f);
-      g.out[(size_t)row * g.ldo + c] = g.resid ? g.resid[(size_t)row * g.ldo + c] + z : z;
+    for (int nt = 0; nt < 8; ++nt) {
+      const int c = nt * 8 + 2 * tq;
+      float z0 = acc[nt][2 * h] + (g.bias ? g.bias[c] : 0.f), z1 = acc[nt][2 * h + 1] + (g.bias ? g.bias[c + 1] : 0.f);
+      if (g.relu) { z0 = fmaxf(z0, 0.f); z1 = fmaxf(z1, 0.f); }
+      if (g.resid) {
+        const float2 x = *reinterpret_cast<const float2*>(g.resid + (size_t)row * g.ldo + c);
+        z0 = x.x + z0; z1 = x.y + z1;
+      }
+      *reinterpret_cast<float2*>(g.out + (size_t)row * g.ldo + c) = make_float2(z0, z1);
     }
+  }
 }
 
 // --------------------------------------------------------------------------------------------
@@ -517,8 +677,12 @@ __global__ void k_add_cols(float* dst, const float* __restrict__ src, int lds, i
 
 __device__ __forceinline__ void edge_block(const float* x, const float* cf, float (&E)[36]) {
   const float c0 = 1.f + cf[0], c1 = 1.f + cf[1], c2 = 1.f + cf[2];
+  float x1[36], x2[36];
+  load36(E, x);
+  load36(x1, x + 36);
+  load36(x2, x + 72);
 #pragma unroll
-  for (int t = 0; t < 36; ++t) E[t] = -c0 * x[t] + c1 * x[36 + t] + c2 * x[72 + t];
+  for (int t = 0; t < 36; ++t) E[t] = -c0 * E[t] + c1 * x1[t] + c2 * x2[t];
 }
 
 __global__ void k_gnn_build_E(int ne, const float* __restrict__ xe, const float* __restrict__ coef, float* Em) {
@@ -537,14 +701,18 @@ __global__ void k_gnn_pcg_blocks(GnnGraph g, const float* __restrict__ xe, const
   if (e >= g.ne) return;
   float E[36];
   edge_block(xe + (size_t)e * kGnnEdgeIn, coef + (size_t)e * 3, E);
-  const float* Ca = cinv + (size_t)g.ea[e] * 36;
-  float* o = ehat + (size_t)g.eblk[e] * 36;
+  float Ca[36], o[36];
+  load36(Ca, cinv + (size_t)g.ea[e] * 36);
+#pragma unroll
   for (int r = 0; r < 6; ++r)
+#pragma unroll
     for (int c = 0; c < 6; ++c) {
       float v = 0.f;
+#pragma unroll
       for (int k = c; k < 6; ++k) v += E[r * 6 + k] * Ca[k * 6 + c];
       o[r * 6 + c] = v;
     }
+  store36(ehat + (size_t)g.eblk[e] * 36, o);
 }
 
 // Rademacher probe entry (fmix32 finaliser of MurmurHash3 over the entry index and the seed).
@@ -700,14 +868,17 @@ int gnn_features(const GnnGraph& g, const void* Sb, bool fp64, const int* diag_b
                  int* d_fail, cudaStream_t st) {
   const int N = g.N, ne = g.ne;
   if (reinterpret_cast<uintptr_t>(xe) & 15) return V3DBA_ERR_UNSUPPORTED;   // 16-byte loads of edge rows
-  if (fp64) k_gnn_cinv<double><<<cdiv(N, 128), 128, 0, st>>>((const double*)Sb, diag_blk, N, cinv, d_fail);
-  else k_gnn_cinv<float><<<cdiv(N, 128), 128, 0, st>>>((const float*)Sb, diag_blk, N, cinv, d_fail);
+  if (fp64) k_gnn_cinv<double><<<cdiv(N, 32), 32, 0, st>>>((const double*)Sb, diag_blk, N, cinv, d_fail);
+  else k_gnn_cinv<float><<<cdiv(N, 32), 32, 0, st>>>((const float*)Sb, diag_blk, N, cinv, d_fail);
   V3DBA_LAUNCH_CHECK();
   if (ne > 0) {
     if (fp64) k_gnn_edge_norm<double><<<cdiv(ne, 128), 128, 0, st>>>((const double*)Sb, g, cinv, xe);
     else k_gnn_edge_norm<float><<<cdiv(ne, 128), 128, 0, st>>>((const float*)Sb, g, cinv, xe);
     V3DBA_LAUNCH_CHECK();
-    k_gnn_two_hop<<<cdiv(ne, 4), dim3(72, 4), 0, st>>>(g, xe);
+    const int row_cap = g.max_lo <= kHopRow ? g.max_lo : kHopRow;
+    if (hop_smem(row_cap) > 48 * 1024)
+      V3DBA_CUDA_TRY(cudaFuncSetAttribute(k_gnn_two_hop, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hop_smem(kHopRow)));
+    k_gnn_two_hop<<<2 * g.nhop, 32 * kHopWarps, hop_smem(row_cap), st>>>(g, xe, row_cap);
     V3DBA_LAUNCH_CHECK();
   }
   k_gnn_node_feat<<<cdiv(N, 8), 256, 0, st>>>(g, xe, xn);
@@ -824,6 +995,13 @@ int rowgemm(cudaStream_t st, int rows, std::initializer_list<Seg> in, const floa
   for (const Seg& s : in) { g.seg[g.nseg++] = s; g.K += s.width; }
   g.W = W; g.wk = wk; g.wn = wn; g.bias = bias; g.Nout = Nout; g.out = out; g.ldo = ldo; g.resid = resid;
   g.act_out = act_out; g.relu = relu ? 1 : 0;
+  const Seg& s0 = g.seg[0];
+  if (Nout <= kNarrow && g.nseg == 1 && !s0.idx && !resid && !act_out && !(s0.width & 3) && !(s0.ld & 3) &&
+      !(reinterpret_cast<uintptr_t>(s0.src) & 15)) {
+    k_rows_narrow<<<cdiv(rows, 128), 128, sizeof(float) * kNarrow * g.K, st>>>(g);
+    V3DBA_LAUNCH_CHECK();
+    return V3DBA_OK;
+  }
   const size_t smem = sizeof(float) * ((size_t)kRgRows * (g.K + 1) + (size_t)g.K * Nout);
   k_rowgemm<<<cdiv(rows, kRgRows), 256, smem, st>>>(g);
   V3DBA_LAUNCH_CHECK();
@@ -844,7 +1022,12 @@ int rowgemm_bf16(v3dba_precond_model_s* m, cudaStream_t st, int rows, std::initi
   g.bias = bias; g.Nout = kGnnH; g.out = out; g.ldo = kGnnH; g.resid = resid; g.relu = relu ? 1 : 0;
   const int Kp = kPackK[layer];
   const size_t smem = sizeof(__nv_bfloat16) * 2 * 64 * (size_t)(Kp + 8);
-  k_rowgemm_bf16<<<cdiv(rows, 64), 128, smem, st>>>(g, m->wt + pack_offset(layer), Kp);
+  const __nv_bfloat16* Wt = m->wt + pack_offset(layer);
+  const int nb = cdiv(rows, 64);
+  if (Kp == 192 && g.nseg == 3) k_rowgemm_bf16<192, 3><<<nb, 128, smem, st>>>(g, Wt);
+  else if (Kp == 128 && g.nseg == 2) k_rowgemm_bf16<128, 2><<<nb, 128, smem, st>>>(g, Wt);
+  else if (Kp == 112 && g.nseg == 1) k_rowgemm_bf16<112, 1><<<nb, 128, smem, st>>>(g, Wt);
+  else return V3DBA_ERR_UNSUPPORTED;
   V3DBA_LAUNCH_CHECK();
   return V3DBA_OK;
 }
@@ -874,7 +1057,7 @@ int set_smem_limits() {
   if (done) return V3DBA_OK;
   V3DBA_CUDA_TRY(cudaFuncSetAttribute(k_rowgemm, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
   V3DBA_CUDA_TRY(cudaFuncSetAttribute(k_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
-  V3DBA_CUDA_TRY(cudaFuncSetAttribute(k_rowgemm_bf16, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
+  V3DBA_CUDA_TRY(cudaFuncSetAttribute(k_rowgemm_bf16<192, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
   done = true;
   return V3DBA_OK;
 }
