@@ -246,6 +246,27 @@ __device__ __forceinline__ void stage_blocks(T* dst, const T* __restrict__ src, 
   }
 }
 
+// Writes the lanes' blocks v (of lanes with k >= 0) to dst[k * STRIDE + t], consecutive lanes on consecutive 16
+// bytes of a block (STAGED; buf: 32 blocks of the warp), or every lane its own.
+template <bool STAGED, int STRIDE, typename T>
+__device__ __forceinline__ void put_block(T* __restrict__ dst, void* buf, const T (&v)[STRIDE], int k, int lane) {
+  constexpr int E = 16 / sizeof(T), V = STRIDE / E;
+  if constexpr (!STAGED) {
+    vstore(dst + (size_t)k * STRIDE, v);
+    return;
+  }
+  static_assert(STRIDE % E == 0, "blocks are whole 16-byte vectors");
+  if (k >= 0) vstore(reinterpret_cast<T*>(buf) + lane * STRIDE, v);
+  __syncwarp();
+#pragma unroll
+  for (int t = 0; t < V; ++t) {
+    const int e = lane + 32 * t, rec = e / V, off = e - rec * V;
+    const int kk = __shfl_sync(0xffffffffu, k, rec);
+    if (kk >= 0) reinterpret_cast<float4*>(dst + (size_t)kk * STRIDE)[off] = reinterpret_cast<const float4*>(buf)[e];
+  }
+  __syncwarp();
+}
+
 __device__ __forceinline__ void dmma884(double (&c)[2], double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
                : "+d"(c[0]), "+d"(c[1])
@@ -289,6 +310,18 @@ struct RelinNV {
   static constexpr int NV = NS + 2;        // + max |gb|, max diag V
 };
 
+// 16-byte units of the largest block that k_linearize stores per observation.
+template <int DA, int DC, typename Real>
+__host__ __device__ constexpr int obs_block_units() {
+  using L = Lay<DA, DC, Real>;
+  int m = L::SA * (int)sizeof(Real);
+  const int w = stores_products<Real>() ? L::SW * 4 : kSB * 8, g = L::SG * 8, c = DC > 0 ? L::SC * (int)sizeof(Real) : 0;
+  m = m > w ? m : w;
+  m = m > g ? m : g;
+  m = m > c ? m : c;
+  return m / 16;
+}
+
 // kLinLanes lanes per point: each linearises every kLinLanes-th observation of the track (FP64),
 // stores the weighted blocks, and accumulates its share of V_j, gb_j, Y_j, summed over the group
 // at the end in a fixed order; Z, gc and the cost go to per-block partials.  The cameras come as packed
@@ -302,6 +335,7 @@ __global__ void __launch_bounds__(kPtThreads) k_linearize(DevState s, double* __
   constexpr int DCc = L::DCc;
   constexpr int NS = RelinNV<DC>::NS, NV = RelinNV<DC>::NV, NZ = L::NZ;
   __shared__ double red[(kPtThreads / 32) * NV];
+  constexpr int kBlk = obs_block_units<DA, DC, Real>();
   const Dims& D = s.d;
   const int gt = blockIdx.x * blockDim.x + threadIdx.x;
   const int tp = gt / kLinLanes, lig = gt % kLinLanes;
@@ -316,25 +350,38 @@ __global__ void __launch_bounds__(kPtThreads) k_linearize(DevState s, double* __
     for (int c = 0; c < DCc; ++c) Y[b][c] = 0.0;
   const bool fixB = j < D.nnB;
   int k0 = 0, k1 = 0;
-
+  double X[3] = {0, 0, 0};
   if (j < D.M) {
-    const double X[3] = {s.cur.X[3 * j], s.cur.X[3 * j + 1], s.cur.X[3 * j + 2]};
-    Real* oA = reinterpret_cast<Real*>(s.o_A);
-    Real* oC = reinterpret_cast<Real*>(s.o_C);
+#pragma unroll
+    for (int t = 0; t < 3; ++t) X[t] = s.cur.X[3 * (size_t)j + t];
     k0 = s.p_ptr[j];
     k1 = s.p_ptr[j + 1];
-    for (int k = k0 + lig; k < k1; k += kLinLanes) {
+  }
+  // With FP64 blocks (216 to 340 bytes an observation) the warp writes its 32 observations' blocks together,
+  // through shared memory: 375,000 observations with 7 global intrinsics 64.5 -> 59.4 us, 460,000 of a rig
+  // 42.0 -> 38.3; 5.5M 504 -> 523, and with FP32 blocks the first 48.7 -> 51.9 and the last 501 -> 599 (the
+  // blocks wait in registers for the warp), so those are written lane by lane.
+  constexpr bool STAGED = !stores_products<Real>();
+  __shared__ float4 stage[STAGED ? kPtThreads * kBlk : 1];
+  const int lane = threadIdx.x & 31;
+  float4* buf = stage + (threadIdx.x & ~31) * kBlk;
+  const int own = (k1 - k0 - lig + kLinLanes - 1) / kLinLanes, trips = STAGED ? __reduce_max_sync(0xffffffffu, own) : own;
+  for (int u = 0; u < trips; ++u) {
+    const int kt = k0 + lig + kLinLanes * u, k = !STAGED || kt < k1 ? kt : -1;
+    double A[2][DA], B[2][3], C[2][DCc], r0 = 0.0, r1 = 0.0;
+    if (k >= 0) {
       const int i = s.o_cam[k];
       const bool fixA = i < D.nnA;
       Cam cam;
       load_cam_packed<MODEL>(cam, s.cur.pack, s.cur.K, s.cur.dist, i);
       if (MODEL == kModelStereo) load_rig(cam, s.rig, s.o_sub[k]);
-      double e[2], A[2][DA], B[2][3], C[2][DCc];
+      double e[2];
       linearize_obs<MODEL, DA, DC>(cam, X, s.o_meas[2 * k], s.o_meas[2 * k + 1], D.mode, D.cached_ar, e, A, B, C);
       const double w = huber_weight(D.thr, e);
       s.o_w[k] = w;
       v[0] += w * w * (e[0] * e[0] + e[1] * e[1]);
-      const double r0 = -w * e[0], r1 = -w * e[1];
+      r0 = -w * e[0];
+      r1 = -w * e[1];
       const double wa = fixA ? 0.0 : w, wb = fixB ? 0.0 : w;
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
@@ -344,52 +391,6 @@ __global__ void __launch_bounds__(kPtThreads) k_linearize(DevState s, double* __
         for (int q = 0; q < 3; ++q) B[r][q] *= wb;
 #pragma unroll
         for (int q = 0; q < DCc; ++q) C[r][q] = (DC > 0 && q >= D.nnC) ? C[r][q] * w : 0.0;
-      }
-      // per-observation blocks
-      {
-        Real a[L::SA];
-#pragma unroll
-        for (int t = 0; t < L::SA; ++t) a[t] = Real(0);
-#pragma unroll
-        for (int r = 0; r < 2; ++r)
-#pragma unroll
-          for (int q = 0; q < DA; ++q) a[r * DA + q] = Real(A[r][q]);
-        vstore(oA + (size_t)k * L::SA, a);
-        if constexpr (stores_products<Real>()) {
-          float wv[L::SW];
-#pragma unroll
-          for (int t = 0; t < L::SW; ++t) wv[t] = 0.f;
-#pragma unroll
-          for (int q = 0; q < DA; ++q)
-#pragma unroll
-            for (int b = 0; b < 3; ++b) wv[q * 3 + b] = float(A[0][q] * B[0][b] + A[1][q] * B[1][b]);
-          vstore(s.o_W + (size_t)k * L::SW, wv);
-        } else {
-          double bv[kSB];
-#pragma unroll
-          for (int t = 0; t < kSB; ++t) bv[t] = 0.0;
-#pragma unroll
-          for (int r = 0; r < 2; ++r)
-#pragma unroll
-            for (int b = 0; b < 3; ++b) bv[r * 3 + b] = B[r][b];
-          vstore(s.o_B + (size_t)k * kSB, bv);
-        }
-        if (DC > 0) {
-          Real cv[L::SC];
-#pragma unroll
-          for (int t = 0; t < L::SC; ++t) cv[t] = Real(0);
-#pragma unroll
-          for (int r = 0; r < 2; ++r)
-#pragma unroll
-            for (int q = 0; q < DCc; ++q) cv[r * DCc + q] = Real(C[r][q]);
-          vstore(oC + (size_t)k * L::SC, cv);
-        }
-        double g[L::SG];
-#pragma unroll
-        for (int t = 0; t < L::SG; ++t) g[t] = 0.0;
-#pragma unroll
-        for (int q = 0; q < DA; ++q) g[q] = A[0][q] * r0 + A[1][q] * r1;
-        vstore(s.o_ga + (size_t)k * L::SG, g);
       }
       // point sums
 #pragma unroll
@@ -411,6 +412,54 @@ __global__ void __launch_bounds__(kPtThreads) k_linearize(DevState s, double* __
 #pragma unroll
         for (int c = 0; c < DCc; ++c) v[1 + NZ + c] += C[0][c] * r0 + C[1][c] * r1;
       }
+    }
+    // per-observation blocks
+    {
+      Real a[L::SA];
+#pragma unroll
+      for (int t = 0; t < L::SA; ++t) a[t] = Real(0);
+#pragma unroll
+      for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int q = 0; q < DA; ++q) a[r * DA + q] = Real(A[r][q]);
+      put_block<STAGED, L::SA>(reinterpret_cast<Real*>(s.o_A), buf, a, k, lane);
+    }
+    if constexpr (stores_products<Real>()) {
+      float wv[L::SW];
+#pragma unroll
+      for (int t = 0; t < L::SW; ++t) wv[t] = 0.f;
+#pragma unroll
+      for (int q = 0; q < DA; ++q)
+#pragma unroll
+        for (int b = 0; b < 3; ++b) wv[q * 3 + b] = float(A[0][q] * B[0][b] + A[1][q] * B[1][b]);
+      put_block<STAGED, L::SW>(s.o_W, buf, wv, k, lane);
+    } else {
+      double bv[kSB];
+#pragma unroll
+      for (int t = 0; t < kSB; ++t) bv[t] = 0.0;
+#pragma unroll
+      for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int b = 0; b < 3; ++b) bv[r * 3 + b] = B[r][b];
+      put_block<STAGED, kSB>(s.o_B, buf, bv, k, lane);
+    }
+    if (DC > 0) {
+      Real cv[L::SC];
+#pragma unroll
+      for (int t = 0; t < L::SC; ++t) cv[t] = Real(0);
+#pragma unroll
+      for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int q = 0; q < DCc; ++q) cv[r * DCc + q] = Real(C[r][q]);
+      put_block<STAGED, L::SC>(reinterpret_cast<Real*>(s.o_C), buf, cv, k, lane);
+    }
+    {
+      double g[L::SG];
+#pragma unroll
+      for (int t = 0; t < L::SG; ++t) g[t] = 0.0;
+#pragma unroll
+      for (int q = 0; q < DA; ++q) g[q] = A[0][q] * r0 + A[1][q] * r1;
+      put_block<STAGED, L::SG>(s.o_ga, buf, g, k, lane);
     }
   }
   // the group's sums (every lane takes part in the shuffles)
