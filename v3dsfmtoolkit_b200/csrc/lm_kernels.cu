@@ -1761,9 +1761,12 @@ __global__ void __launch_bounds__(128) k_finish_merged(DevState s, int g1, int g
 }
 
 // Camera (and global) update (blocks [0, g1)) and point back-substitution: both read the
-// reduced solution and the current parameters and write different parts of the trial ones.
+// reduced solution and the current parameters and write different parts of the trial ones.  At most 64
+// registers: the few camera blocks would take 80 to 120 and leave the points, which need 32 to 42 and wait for
+// their loads, half the warps (5.5M observations, the whole iteration 2341 -> 2275 us; 40 registers 2279, and
+// 3 us more on 20 cameras, whose camera blocks then spill on the critical path).
 template <int MODEL, int DA, int DC, typename Real>
-__global__ void __launch_bounds__(128) k_update_merged(DevState s, int g1, int g2, double* __restrict__ pcam,
+__global__ void __launch_bounds__(128, 8) k_update_merged(DevState s, int g1, int g2, double* __restrict__ pcam,
                                                        double* __restrict__ ppt) {
   pdl_wait();
   pdl_trigger();
