@@ -423,22 +423,22 @@ def bundle_point_structure(tracks, n_required=2):
     mpos (K, 2) float32.  Returns dict of points3d, measurements, measurement_ids,
     corresponding_view, corresponding_point, xs_indices."""
     ptr, pos, view, ids, mpos = _tracks_args(tracks)
+    n_required = int(n_required)
+    if not -2**31 <= n_required < 2**31:   # ctypes would pass its low word
+        raise V3dbaError(ERR_INVALID_ARGUMENT, "v3dba_bundle_point_structure")
     n, K = ptr.size - 1, int(ptr[-1])
     npts, nm = C.c_int(), C.c_int()
-    # the kept tracks' counts, so that the results are written where they stay (a list that the call
-    # refuses has lengths that mean nothing: arrays of the largest size then)
-    length = np.diff(ptr)
-    keep = length >= int(n_required) if n_required >= 0 else np.zeros(n, dtype=bool)
-    valid = n == 0 or (ptr[0] == 0 and int(length.min()) >= 0)
-    M, Kk = (int(np.count_nonzero(keep)), int(length[keep].sum())) if valid else (n, max(K, 0))
-    pts, meas = np.zeros((M, 3)), np.zeros((Kk, 2))
-    mid, cv, cp = (np.zeros(Kk, np.int32) for _ in range(3))
-    xs = np.zeros(M, np.int32)
-    check(_lib().v3dba_bundle_point_structure(n, _i(ptr), _d(pos), _i(view), _i(ids), _f32p(mpos), int(n_required),
+    # Arrays of the largest size, whatever the library keeps; the results are their first part, written where
+    # they stay (the pages of the rest are never touched).
+    pts, meas = np.zeros((n, 3)), np.zeros((max(K, 0), 2))
+    mid, cv, cp = (np.zeros(max(K, 0), np.int32) for _ in range(3))
+    xs = np.zeros(n, np.int32)
+    check(_lib().v3dba_bundle_point_structure(n, _i(ptr), _d(pos), _i(view), _i(ids), _f32p(mpos), n_required,
                                               C.byref(npts), C.byref(nm), _d(pts), _d(meas), _i(mid), _i(cv), _i(cp),
                                               _i(xs)), "v3dba_bundle_point_structure")
-    return dict(points3d=pts, measurements=meas, measurement_ids=mid, corresponding_view=cv, corresponding_point=cp,
-                xs_indices=xs)
+    M, Kk = npts.value, nm.value
+    return dict(points3d=pts[:M], measurements=meas[:Kk], measurement_ids=mid[:Kk], corresponding_view=cv[:Kk],
+                corresponding_point=cp[:Kk], xs_indices=xs[:M])
 
 
 def create_point_structure(bps, from_scratch=True, tracks=None):
