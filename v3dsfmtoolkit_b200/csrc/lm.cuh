@@ -120,16 +120,17 @@ struct DevState {
   int trial_blocks_pt = 0, trial_blocks_cam = 0, trial_blocks_obs = 0;
 };
 
-// Limits of a chunk of the grouped Schur complement, and its shared memory: G is [3 points, padded to
-// whole DMMA steps][leading dimension], a row per (camera, unknown); the leading dimension is 4 mod 8
-// doubles, so that the 4 x 4 elements of a fragment load lie in different banks.
+// Limits of a chunk of the grouped Schur complement, and its shared memory: G is [3 points, padded to four
+// points][leading dimension], a row per (camera, unknown); the leading dimension is 4 mod 8 doubles (and
+// three times that too), so that the 4 x 4 elements of a fragment load lie in different banks.
 constexpr int kGroupPoints = 32;    // points per chunk, fewer where the cameras are many
 constexpr int kGroupTrack = 64;     // observations per point
 constexpr int kGroupRows = 360;     // unknowns of the cameras of a group
 constexpr int kGroupSmem = 72 * 1024;   // three blocks per SM
 __host__ __device__ constexpr int group_ld(int rows) { return (rows + 3) / 8 * 8 + 4; }
+__host__ __device__ constexpr int group_pad(int points) { return (points + 3) / 4 * 4; }
 __host__ __device__ constexpr int group_doubles(int points, int rows) {
-  return (3 * points + 3) / 4 * 4 * group_ld(rows) + 8 + 6 * points + (kGroupPoints + 3 * kGroupTrack) / 2;
+  return 3 * group_pad(points) * group_ld(rows) + 8 + 6 * group_pad(points) + (kGroupPoints + 3 * kGroupTrack) / 2;
 }
 
 // Stages of one LM iteration, in launch order.

@@ -1093,9 +1093,12 @@ __device__ __forceinline__ void schur_chunks_body(DevState s, double* __restrict
 }
 
 // FP64 blocks, points grouped by their cameras: one block per chunk of up to 32 points that the same L
-// cameras see.  With (V + lambda I)^-1 = C^-T C^-1 and G_k = A_k^T B_k C^-T, the chunk's part of the
-// whole L x L block matrix is G G^T, G one row per camera unknown and three columns per point, formed in
-// shared memory (observations of a point in the same camera add up first) and multiplied with DMMA.
+// cameras see.  With G_k = A_k^T B_k the chunk's part of the whole L x L block matrix is G Vinv G^T, G one row
+// per camera unknown and three columns per point, formed in shared memory (observations of a point in the
+// same camera add up first) and multiplied with DMMA.  Vinv = (V + lambda I)^-1 is k_point_eliminate's, as for
+// the pair lists, the right-hand side and the step, so that the system is one and the same where rounding
+// decides about it (a Cholesky factor of V + lambda I in its place left a point out, or turned a pivot's sign,
+// that the other parts kept); it multiplies the left fragment, nine FMAs for nine DMMAs.
 // Every observation's blocks are read once per trial instead of once per pair (144 bytes instead of 340
 // times the pairs of its track), the gathers that bound the pair lists: their L2 to L1 traffic was 870
 // MB at 5.8 TB/s (pairs staged through shared memory and multiplied with DMMA reached 9.4 TB/s, and no
@@ -1110,40 +1113,28 @@ __device__ __forceinline__ void schur_group_body(const DevState& s, int ch) {
   const int tid = threadIdx.x, lane = tid & 31;
   const int4 d = reinterpret_cast<const int4*>(s.gr_desc)[ch];
   const int p0 = d.x, np = d.y, e0 = d.z, L = d.w;
-  const int rows = DA * L, ld = group_ld(rows), K = (3 * np + 3) / 4 * 4;
+  const int rows = DA * L, ld = group_ld(rows), nq = group_pad(np);
   double* Gs = group_sm;
-  double* Cs = Gs + K * ld + 8;                          // [np][6] C^-1 (00 10 11 20 21 22)
-  int* first = reinterpret_cast<int*>(Cs + 6 * np);      // [np] first observation of the point
+  double* Vs = Gs + 3 * nq * ld + 8;                     // [nq][6] (V + lambda I)^-1
+  int* first = reinterpret_cast<int*>(Vs + 6 * nq);      // [np] first observation of the point
   int* rank = first + kGroupPoints;                      // [track] rank of the observation's camera
   int* head = rank + kGroupTrack;                        // [L] first observation in the camera ...
   int* next = head + kGroupTrack;                        // [track] ... and the next one, or -1
   if (tid < np) {
     const int j = s.gr_pt[p0 + tid];
     first[tid] = s.p_ptr[j];
-    const double lam = *s.d_lambda;
-    double V[L_::SV], c[6] = {0, 0, 0, 0, 0, 0};
-    vload(reinterpret_cast<const double*>(s.p_V) + (size_t)j * L_::SV, V);
-    // A pivot that rounding made negative (a direction no observation sees, lambda below the last bit)
-    // counts by its size: that direction's G is zero to rounding, whatever the sign.
-    const double d0 = V[0] + lam, i0 = rsqrt(fabs(d0)), l10 = V[1] * i0, l20 = V[2] * i0;
-    const double d1 = V[3] + lam - l10 * l10, i1 = rsqrt(fabs(d1)), l21 = (V[4] - l20 * l10) * i1;
-    const double d2 = V[5] + lam - l20 * l20 - l21 * l21, i2 = rsqrt(fabs(d2));
-    // a singular point contributes nothing here and failed in k_point_eliminate; a fixed one neither
-    if (j >= s.d.nnB && isfinite(i0) && isfinite(i1) && isfinite(i2)) {
-      c[0] = i0;
-      c[1] = -l10 * i0 * i1;
-      c[2] = i1;
-      c[3] = -(l20 * i0 + l21 * c[1]) * i2;
-      c[4] = -l21 * i1 * i2;
-      c[5] = i2;
-    }
+    double V[L_::SV];   // zero for a fixed point and for a singular one (which k_point_eliminate reports)
+    vload(reinterpret_cast<const double*>(s.p_Vinv) + (size_t)j * L_::SV, V);
 #pragma unroll
-    for (int t = 0; t < 6; ++t) Cs[6 * tid + t] = c[t];
+    for (int t = 0; t < 6; ++t) Vs[6 * tid + t] = V[t];
+  } else if (tid < nq) {                                 // the last DMMA steps' padding
+#pragma unroll
+    for (int t = 0; t < 6; ++t) Vs[6 * tid + t] = 0.0;
   } else if (tid >= kGroupThreads - kGroupTrack) {       // two other warps: the pattern
     const int t = tid - (kGroupThreads - kGroupTrack), j = s.gr_pt[p0], k0 = s.p_ptr[j], n = s.p_ptr[j + 1] - k0;
     rank[t] = t < n ? (int)s.gr_rank[k0 + t] : -1;
   }
-  for (int e = 3 * np * ld + tid; e < K * ld; e += kGroupThreads) Gs[e] = 0.0;   // the last DMMA step's padding
+  for (int e = 3 * np * ld + tid; e < 3 * nq * ld; e += kGroupThreads) Gs[e] = 0.0;   // (padding too)
   __syncthreads();
   if (tid < kGroupTrack) {
     int h = -1, nx = -1;
@@ -1160,8 +1151,6 @@ __device__ __forceinline__ void schur_group_body(const DevState& s, int ch) {
   // one column (of three) of a point's rows in one camera per thread
   for (int idx = tid; idx < 3 * np * L; idx += kGroupThreads) {
     const int q = idx / (3 * L), rest = idx - q * 3 * L, sl = rest / 3, u = rest - 3 * sl;
-    const double* c = Cs + 6 * q;
-    const double c0 = u == 0 ? c[0] : u == 1 ? c[1] : c[3], c1 = u == 0 ? 0.0 : u == 1 ? c[2] : c[4], c2 = u == 2 ? c[5] : 0.0;
     double g[DA];
 #pragma unroll
     for (int a = 0; a < DA; ++a) g[a] = 0.0;
@@ -1170,7 +1159,7 @@ __device__ __forceinline__ void schur_group_body(const DevState& s, int ch) {
       double A[L_::SA], B[kSB];
       vload(reinterpret_cast<const double*>(s.o_A) + k * L_::SA, A);
       vload(s.o_B + k * kSB, B);
-      const double h0 = B[0] * c0 + B[1] * c1 + B[2] * c2, h1 = B[3] * c0 + B[4] * c1 + B[5] * c2;   // of B_k C^-T
+      const double h0 = u == 0 ? B[0] : u == 1 ? B[1] : B[2], h1 = u == 0 ? B[3] : u == 1 ? B[4] : B[5];
 #pragma unroll
       for (int a = 0; a < DA; ++a) g[a] += A[a] * h0 + A[DA + a] * h1;
     }
@@ -1179,7 +1168,8 @@ __device__ __forceinline__ void schur_group_body(const DevState& s, int ch) {
     for (int a = 0; a < DA; ++a) out[a] = g[a];
   }
   __syncthreads();
-  // lower tiles of G G^T, up to three of a tile row at a time (they share the row's fragment)
+  // lower tiles of G Vinv G^T, up to three of a tile row at a time (they share the row's fragment); three DMMA
+  // steps take four points, lane kk = 0..3 of a step one column of point kk
   const int T = (rows + 7) / 8, r = lane >> 2, kk = lane & 3;
   int unit = 0;
   for (int ti = T - 1; ti >= 0; --ti)
@@ -1187,14 +1177,20 @@ __device__ __forceinline__ void schur_group_body(const DevState& s, int ch) {
       if (unit % (kGroupThreads / 32) != (tid >> 5)) continue;
       const int nt = min(3, ti - tj + 1);
       double acc[3][2] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
-      const double* ga = Gs + kk * ld + 8 * ti + r;
-      const double* gb = Gs + kk * ld + 8 * tj + r;
-#pragma unroll 2
-      for (int k = 0; k < K; k += 4, ga += 4 * ld, gb += 4 * ld) {
-        const double a = *ga;
-        dmma884(acc[0], a, gb[0]);
-        if (nt > 1) dmma884(acc[1], a, gb[8]);
-        if (nt > 2) dmma884(acc[2], a, gb[16]);
+      const double* ga = Gs + 3 * kk * ld + 8 * ti + r;
+      const double* gb = Gs + 3 * kk * ld + 8 * tj + r;
+      const double2* vp = reinterpret_cast<const double2*>(Vs + 6 * kk);
+      for (int q = 0; q < nq; q += 4, ga += 12 * ld, gb += 12 * ld, vp += 12) {
+        const double2 v0 = vp[0], v1 = vp[1], v2 = vp[2];   // 00 01, 02 11, 12 22
+        const double g0 = ga[0], g1 = ga[ld], g2 = ga[2 * ld];
+        const double a[3] = {v0.x * g0 + v0.y * g1 + v1.x * g2, v0.y * g0 + v1.y * g1 + v2.x * g2,
+                             v1.x * g0 + v2.x * g1 + v2.y * g2};
+#pragma unroll
+        for (int u = 0; u < 3; ++u) {
+          dmma884(acc[0], a[u], gb[u * ld]);
+          if (nt > 1) dmma884(acc[1], a[u], gb[u * ld + 8]);
+          if (nt > 2) dmma884(acc[2], a[u], gb[u * ld + 16]);
+        }
       }
 #pragma unroll
       for (int t = 0; t < 3; ++t) {
