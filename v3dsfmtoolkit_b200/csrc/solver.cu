@@ -215,13 +215,22 @@ int use_pcg(v3dba_handle h) {
   return V3DBA_OK;
 }
 
-// The grouping of the points for the FP64 blocks' Schur complement: made on first use.
+// The grouping of the points for the FP64 blocks' Schur complement: made on first use, after all that a call
+// cannot do without.  Where there is no room for it the pair lists are used, and the next call tries again.
 int use_groups(v3dba_handle h) {
   if (h->groups_ready) return V3DBA_OK;
   const DevAlloc alloc = [h](void** q, size_t bytes) { return dalloc(h, reinterpret_cast<char**>(q), bytes); };
-  const int rc = build_schur_groups(h->s, alloc, h->stream);
-  if (rc) return rc;
-  h->groups_ready = true;
+  const size_t before = h->allocs.size();
+  int rc;
+  try {
+    rc = build_schur_groups(h->s, alloc, h->stream);
+  } catch (const std::bad_alloc&) {
+    rc = V3DBA_ERR_OUT_OF_MEMORY;
+  }
+  h->groups_ready = rc == V3DBA_OK;
+  if (rc != V3DBA_ERR_OUT_OF_MEMORY) return rc;
+  h->s.gr_n = 0;
+  for (; h->allocs.size() > before; h->allocs.pop_back()) cudaFreeAsync(h->allocs.back(), h->stream);
   return V3DBA_OK;
 }
 
@@ -754,12 +763,12 @@ extern "C" int v3dba_minimize(v3dba_handle h, const v3dba_options* opts, v3dba_r
   if (gauge && D.DA != 6) return V3DBA_ERR_UNSUPPORTED;
   {
     int rc0 = pcg ? use_pcg(h) : use_dense(h);
-    if (!rc0 && fp64) rc0 = use_groups(h);
     if (rc0) return rc0;
     if (gauge) {
       const int rc1 = use_gnn(h, learned);
       if (rc1) return rc1;
     }
+    if (fp64 && (rc0 = use_groups(h))) return rc0;
   }
 
   const int nvA = D.N - D.nnA, nvB = D.M - D.nnB, nvC = D.DC - D.nnC;
