@@ -403,7 +403,8 @@ int v3dba_batch_minimize(v3dba_batch_t b, const v3dba_options* opts, v3dba_resul
 /* Restores the parameters the batch was created with. */
 int v3dba_batch_reset(v3dba_batch_t b);
 /* Schedule: the first `split` problems of the size order run with `large_threads` threads per
- * block, the rest with `small_threads` (64, 128 or 256). */
+ * block, the rest with `small_threads` (64, 128 or 256).  A problem's result does not depend on it,
+ * nor on the other problems of the batch. */
 int v3dba_batch_set_schedule(v3dba_batch_t b, int large_threads, int small_threads, int split);
 /* Times candidate schedules on the batch itself (restoring the parameters after each) and keeps
  * the fastest; reports it when the pointers are not NULL. */

@@ -100,9 +100,10 @@ struct BatchLay {
   static constexpr int kA = NC * 6 * kTileLd;    // A_c, column per (point, residual row)
   static constexpr int kZ = 8 * kTileLd;         // right operand of one camera pair
   static constexpr int kWarp = kA + kZ;          // doubles per warp (the A part also holds its sums)
+  static constexpr int kTile = kPairs * 64;      // doubles of a slot's block sums
   static constexpr int kDim = 6 * NC;
   static constexpr int kSld = kDim + 1;
-  static_assert(kPairs * 64 <= kA, "a warp's block sums take the place of its A tiles");
+  static_assert(2 * kTile <= kA, "a warp's block sums, of two slots with four warps, take the place of its A tiles");
 };
 
 __device__ __forceinline__ void dmma884(double& c0, double& c1, double a, double b) {
@@ -190,8 +191,8 @@ __device__ __forceinline__ void store_a(double* Ac, int lane, const double A[2][
 }
 
 // acc += A Z^T over the warp's 32 points: rows 0..5 of the left tile against `rows` rows of the right
-// one; the other rows are read from `zero`.  Four accumulators in turn: a chain of 16 dependent DMMAs
-// would take about 500 cycles, and an SM holds only 12 warps.
+// one; the other rows are read from `zero`.  Four accumulators in turn (one chain of 16 DMMAs measured
+// the same: the other warps of the SM fill it).
 __device__ __forceinline__ void tile_product(const double* Ac, const double* Z, const double* zero, int rows, int lane,
                                              double (&acc)[2]) {
   const int r = lane >> 2, k = lane & 3;
@@ -323,16 +324,19 @@ __device__ __forceinline__ Track<NC> load_track(const BatchDev& b, const double*
   return t;
 }
 
-template <int NT>
-__device__ __forceinline__ double block_sum(double v, double* red) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  v = warp_sum(v);
-  if (lane == 0) red[wid] = v;
-  __syncthreads();
-  double s = 0.0;
-  for (int w = 0; w < NT / 32; ++w) s += red[w];
-  __syncthreads();
-  return s;
+// The sums over a problem's points have one order for every block size: tile c of 32 points belongs to slot
+// c % kSlots, one warp sums a slot's tiles in order, and the slots add up as slots_sum has it.  So a problem's
+// result does not depend on the threads that its batch gets, nor on the problems beside it.
+constexpr int kSlots = 8;   // the warps of the largest block
+
+template <typename F>
+__device__ __forceinline__ double slots_sum(F v) {
+  return (((v(0) + v(2)) + v(4)) + v(6)) + (((v(1) + v(3)) + v(5)) + v(7));
+}
+// A warp's sum of per-lane values of the slots.
+__device__ __forceinline__ double slots_warp_sum(const double (*v)[32]) {
+  const int lane = threadIdx.x & 31;
+  return warp_sum(slots_sum([&](int sl) { return v[sl][lane]; }));
 }
 
 // One thread block per problem at a time.  A pass over the points gives each warp 32 points, one per
@@ -341,17 +345,18 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
 //     sum_p A_i^T (delta_il I - B_i (V + lambda I)^-1 B_l^T) A_l,
 // so one pass builds U, the Schur complement, the reduced rhs (a seventh column r_i - B_i q) and the
 // gradient (an eighth, r_i) from one linearisation of every observation; each warp sums its points in
-// eight-by-eight accumulators and the warps' sums are added in order (deterministic, no atomics).
-// Bound by FP64 latency: 168 registers and 14 KB of operand tiles per warp leave 12 warps per SM, the
-// FP64 pipe is active 24% and the DMMA pipe 16% of the cycles.  Of the 2.2 ms that 4096 triplets of
-// 50-800 points take for 4 iterations the products are 0.8, the step pass 0.5, the solve 0.25 (timed
-// by leaving each out).  A pass per camera pair that linearised each point again for it (39
+// eight-by-eight accumulators and the slots' sums are added in order (deterministic, no atomics).
+// Bound by FP64 latency: 14 KB of operand tiles per warp and 168 registers (a few spill: 28 bytes a thread
+// with three cameras, about 550 with four) leave 12 warps per SM, the FP64 pipe is active 24% and the DMMA
+// pipe 16% of the cycles.  Of the 2.2 ms that 4096 triplets of 50-800 points take for 4 iterations the products
+// are 0.8, the step pass 0.5, the solve 0.25 (timed by leaving each out).  Loading the next tile's tracks
+// during the products took 24 registers more and, with the slots, 2.43 ms.  A pass per camera pair that linearised each point again for it (39
 // linearisations per point and iteration instead of 6) took 6.7 ms; the same for 61 triplets 1.29 ms
 // against 0.17.
 template <int NT, int NC>
 __global__ void __launch_bounds__(NT, NT > 128 ? 1 : 384 / NT) k_batched_lm(BatchDev b, BatchOpts o, int first, int last) {
   using L = BatchLay<NC>;
-  constexpr int NW = NT / 32, ND = L::kDim, LD = L::kSld;
+  constexpr int NW = NT / 32, ND = L::kDim, LD = L::kSld, OWN = kSlots / NW;   // slots of a warp
   extern __shared__ double dyn[];   // [NW][L::kWarp]
   __shared__ CamS cams[NC], tcams[NC];
   __shared__ double S[ND * LD], rhs[ND], da[ND], ga[ND], udiag[ND], colb[64], red[NW], zrow[kTileK];
@@ -360,6 +365,12 @@ __global__ void __launch_bounds__(NT, NT > 128 ? 1 : 384 / NT) k_batched_lm(Batc
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   double* Aw = dyn + wid * L::kWarp;
   double* Zw = Aw + L::kA;
+  double(*part)[kSlots][32] = reinterpret_cast<double(*)[kSlots][32]>(dyn);   // per-lane sums of the slots
+  // The total of what the warps left at v for their slots, one (of several, summed) or two `second` apart.
+  auto slots_total = [&](const double* v, int second) {
+    if (OWN > 2) return v[0] + v[L::kWarp];
+    return slots_sum([&](int sl) { return v[(sl % NW) * L::kWarp + (sl / NW) * second]; });
+  };
   for (int e = tid; e < kTileK; e += NT) zrow[e] = 0.0;   // read after the barrier below
   for (;;) {
     if (tid == 0) {
@@ -384,16 +395,20 @@ __global__ void __launch_bounds__(NT, NT > 128 ? 1 : 384 / NT) k_batched_lm(Batc
     }
     // cached parameter length (v3d_metricbundle.h:37-45)
     {
-      double v = 0.0;
-      for (int j = tid; j < M; j += NT) {
-        const double* X = Xc + 3 * (size_t)(pt0 + j);
-        v += X[0] * X[0] + X[1] * X[1] + X[2] * X[2];
+      for (int sl = wid; sl < kSlots; sl += NW) {
+        double v = 0.0;
+        for (int j = 32 * sl + lane; j < M; j += 32 * kSlots) {
+          const double* X = Xc + 3 * (size_t)(pt0 + j);
+          v += X[0] * X[0] + X[1] * X[1] + X[2] * X[2];
+        }
+        if (sl == 0 && lane < N) {
+          const double* T = b.T + 3 * (size_t)(c0 + lane);
+          v += T[0] * T[0] + T[1] * T[1] + T[2] * T[2] + 3.0;
+        }
+        part[0][sl][lane] = v;
       }
-      if (tid < N) {
-        const double* T = b.T + 3 * (size_t)(c0 + tid);
-        v += T[0] * T[0] + T[1] * T[1] + T[2] * T[2] + 3.0;
-      }
-      const double s = block_sum<NT>(v, red);
+      __syncthreads();
+      const double s = wid == 0 ? slots_warp_sum(part[0]) : 0.0;
       if (tid == 0) {
         sc[6] = sqrt(s);
         sc[1] = 1e-3;   // lambda of a new optimizer object
@@ -412,173 +427,202 @@ __global__ void __launch_bounds__(NT, NT > 128 ? 1 : 384 / NT) k_batched_lm(Batc
         double acc[L::kPairs][2], err = 0.0, gbmax = 0.0, vdmax = -1e30;
 #pragma unroll
         for (int t = 0; t < L::kPairs; ++t) acc[t][0] = acc[t][1] = 0.0;
-        Track<NC> tr = load_track<NC>(b, Xc, pt0, M, 32 * wid + lane);
-        for (int ch = wid; ch < chunks; ch += NW) {
-          const double X[3] = {tr.X[0], tr.X[1], tr.X[2]};
-          const int o0 = tr.o0, n = tr.n;
-          const bool twice = tr.twice;
-          double V[6] = {0, 0, 0, 0, 0, 0}, gb[3] = {0, 0, 0}, B[NC][2][3], r[NC][2];
-          // no branch on the presence of a camera: the cameras' chains of divisions and roots overlap
+        // The sums of the warp's earlier slots, one after another (two warps) or each for itself (four); kept in
+        // memory, as they are touched once a slot.
+        volatile double kept[L::kPairs][2], kept_err;
+#pragma unroll 1
+        for (int sl = wid; sl < kSlots; sl += NW) {
+          if (OWN > 1 && sl > wid && sl < chunks) {
 #pragma unroll
-          for (int c = 0; c < NC; ++c) {
-            if (c >= N) {
+            for (int t = 0; t < L::kPairs; ++t)
 #pragma unroll
-              for (int q = 0; q < 3; ++q) B[c][0][q] = B[c][1][q] = 0.0;
-              r[c][0] = r[c][1] = 0.0;
-              continue;
-            }
-            const bool has = (tr.mask >> c) & 1u;
-            ObsLin ol;
-            project_obs(cams[c], X, tr.m[c].x, tr.m[c].y, ol);
-            const double w = huber_weight(thr, ol.e);
-            if (has) b.w[o0 + (int)((tr.slot >> (4 * c)) & 15u)] = w;
-            weigh(ol, w, r[c]);
-            if (!has) ol.P[0] = ol.P[1] = ol.P[2] = ol.P[3] = r[c][0] = r[c][1] = 0.0;
-            err += r[c][0] * r[c][0] + r[c][1] * r[c][1];
-            point_block(cams[c], ol, B[c]);
-            double A[2][6];
-            camera_block(ol, A);
-            add_point(B[c], r[c], V, gb);
-            store_a(Aw + c * 6 * kTileLd, lane, A);
+              for (int u = 0; u < 2; ++u) {
+                kept[t][u] = OWN > 2 && sl > wid + NW ? kept[t][u] + acc[t][u] : acc[t][u];
+                acc[t][u] = 0.0;
+              }
+            kept_err = OWN > 2 && sl > wid + NW ? kept_err + err : err;
+            err = 0.0;
           }
-          if (tr.mask) {
-            gbmax = fmax(gbmax, fmax(fabs(gb[0]), fmax(fabs(gb[1]), fabs(gb[2]))));
-            vdmax = fmax(vdmax, fmax(V[0], fmax(V[3], V[5])));
-          }
-          tr = load_track<NC>(b, Xc, pt0, M, 32 * (ch + NW) + lane);   // in flight during the products
-          // without the elimination (mode 0) the same product is U, and its right-hand side the gradient
-          double vi[6] = {0, 0, 0, 0, 0, 0}, q[3], det;
-          bool ok = true;
-          if (mode == 1) {
-            ok = invert_point(V, lam, vi, &det);
-            if (!ok && !isfinite(det)) {   // a point at infinity contributes nothing
-              const double zero2[2][6] = {};
+#pragma unroll 1
+          for (int ch = sl; ch < chunks; ch += kSlots) {
+            Track<NC> tr = load_track<NC>(b, Xc, pt0, M, 32 * ch + lane);
+            const double X[3] = {tr.X[0], tr.X[1], tr.X[2]};
+            const int o0 = tr.o0, n = tr.n;
+            const bool twice = tr.twice;
+            double V[6] = {0, 0, 0, 0, 0, 0}, gb[3] = {0, 0, 0}, B[NC][2][3], r[NC][2];
+            // no branch on the presence of a camera (with branches it measured the same)
 #pragma unroll
-              for (int c = 0; c < NC; ++c) {
-                if (c < N) store_a(Aw + c * 6 * kTileLd, lane, zero2);
+            for (int c = 0; c < NC; ++c) {
+              if (c >= N) {
+#pragma unroll
+                for (int q = 0; q < 3; ++q) B[c][0][q] = B[c][1][q] = 0.0;
                 r[c][0] = r[c][1] = 0.0;
+                continue;
               }
+              const bool has = (tr.mask >> c) & 1u;
+              ObsLin ol;
+              project_obs(cams[c], X, tr.m[c].x, tr.m[c].y, ol);
+              const double w = huber_weight(thr, ol.e);
+              if (has) b.w[o0 + (int)((tr.slot >> (4 * c)) & 15u)] = w;
+              weigh(ol, w, r[c]);
+              if (!has) ol.P[0] = ol.P[1] = ol.P[2] = ol.P[3] = r[c][0] = r[c][1] = 0.0;
+              err += r[c][0] * r[c][0] + r[c][1] * r[c][1];
+              point_block(cams[c], ol, B[c]);
+              double A[2][6];
+              camera_block(ol, A);
+              add_point(B[c], r[c], V, gb);
+              store_a(Aw + c * 6 * kTileLd, lane, A);
             }
-          }
-          mul_sym3(vi, gb, q);
-          int pr = 0;
-#pragma unroll
-          for (int i = 0; i < NC; ++i) {
-            double BV[2][3];
-            mul_sym3(vi, B[i][0], BV[0]);
-            mul_sym3(vi, B[i][1], BV[1]);
-#pragma unroll
-            for (int l = i; l < NC; ++l, ++pr) {
-              if (l >= N || (l != i && mode == 0)) continue;
-              store_z(Zw, Aw + l * 6 * kTileLd, lane, BV, B[l], i == l, ok);
-              if (i == l) {
-                const double e0 = r[i][0] - (B[i][0][0] * q[0] + B[i][0][1] * q[1] + B[i][0][2] * q[2]);
-                const double e1 = r[i][1] - (B[i][1][0] * q[0] + B[i][1][1] * q[1] + B[i][1][2] * q[2]);
-                store_row(Zw, 6, lane, ok ? e0 : 0.0, ok ? e1 : 0.0);
-                store_row(Zw, 7, lane, r[i][0], r[i][1]);
-              }
-              __syncwarp();
-              tile_product(Aw + i * 6 * kTileLd, Zw, zrow, i == l ? 8 : 6, lane, acc[pr]);
-              __syncwarp();
+            if (tr.mask) {
+              gbmax = fmax(gbmax, fmax(fabs(gb[0]), fmax(fabs(gb[1]), fabs(gb[2]))));
+              vdmax = fmax(vdmax, fmax(V[0], fmax(V[3], V[5])));
             }
-          }
-          // tracks that name a camera twice: their observation pairs one per round and point
-          if (__any_sync(0xffffffffu, twice)) {
-            double vi[6] = {0, 0, 0, 0, 0, 0}, q[3] = {0, 0, 0};
-            bool ok = false, dead = false;
-            const int nt = twice ? n : 0;
-            {
-              double V2[6] = {0, 0, 0, 0, 0, 0}, gb2[3] = {0, 0, 0}, det;
-              for (int t = 0; t < nt; ++t) {
-                const int k = o0 + t;
-                const CamS& cm = cams[b.cam[k]];
-                ObsLin ol;
-                double rr[2], Bt[2][3];
-                project_obs(cm, X, b.meas[2 * (size_t)k], b.meas[2 * (size_t)k + 1], ol);
-                const double w = huber_weight(thr, ol.e);
-                b.w[k] = w;
-                err += w * w * (ol.e[0] * ol.e[0] + ol.e[1] * ol.e[1]);
-                weigh(ol, w, rr);
-                point_block(cm, ol, Bt);
-                add_point(Bt, rr, V2, gb2);
-              }
-              if (twice) {
-                gbmax = fmax(gbmax, fmax(fabs(gb2[0]), fmax(fabs(gb2[1]), fabs(gb2[2]))));
-                vdmax = fmax(vdmax, fmax(V2[0], fmax(V2[3], V2[5])));
-                ok = invert_point(V2, lam, vi, &det);
-                dead = mode == 1 && !ok && !isfinite(det);
-                mul_sym3(vi, gb2, q);
-              }
-            }
-#pragma unroll 1
-            for (int i = 0; i < N; ++i)
-#pragma unroll 1
-              for (int l = i; l < N; ++l) {
-                if (mode == 0 && l != i) continue;
-                double* Ac = Aw + i * 6 * kTileLd;
-                int t = 0, u = -1;
-                for (;;) {
-                  // the lane's next pair (t, u) of an observation in camera i with one in camera l; the
-                  // diagonal's U term and gradient come with t == u (mode 0 has only those)
-                  bool have = false;
-                  while (!have) {
-                    if (++u >= nt) { u = 0; ++t; }
-                    if (t >= nt) break;
-                    have = b.cam[o0 + t] == i && b.cam[o0 + u] == l && (mode == 1 || t == u);
-                  }
-                  if (!__any_sync(0xffffffffu, have)) break;
-                  double At[2][6] = {}, Z[8][2] = {};
-                  if (have && !dead) {
-                    double Au[2][6], Bt[2][3], Bu[2][3], rt[2], ru[2], BV[2][3];
-                    ObsLin ol;
-                    project_obs(cams[i], X, b.meas[2 * (size_t)(o0 + t)], b.meas[2 * (size_t)(o0 + t) + 1], ol);
-                    weigh(ol, b.w[o0 + t], rt);
-                    point_block(cams[i], ol, Bt);
-                    camera_block(ol, At);
-                    project_obs(cams[l], X, b.meas[2 * (size_t)(o0 + u)], b.meas[2 * (size_t)(o0 + u) + 1], ol);
-                    weigh(ol, b.w[o0 + u], ru);
-                    point_block(cams[l], ol, Bu);
-                    camera_block(ol, Au);
-                    mul_sym3(vi, Bt[0], BV[0]);
-                    mul_sym3(vi, Bt[1], BV[1]);
-                    for (int rr = 0; rr < 2; ++rr) {
-                      double P[2];
-                      for (int cc = 0; cc < 2; ++cc)
-                        P[cc] = ((t == u && rr == cc) ? 1.0 : 0.0) -
-                                (mode == 1 ? BV[rr][0] * Bu[cc][0] + BV[rr][1] * Bu[cc][1] + BV[rr][2] * Bu[cc][2] : 0.0);
-                      const bool use = mode == 0 || ok;
-                      for (int a = 0; a < 6; ++a) Z[a][rr] = use ? P[0] * Au[0][a] + P[1] * Au[1][a] : 0.0;
-                      if (t == u) {
-                        if (mode == 1 && ok) Z[6][rr] = rt[rr] - (Bt[rr][0] * q[0] + Bt[rr][1] * q[1] + Bt[rr][2] * q[2]);
-                        Z[7][rr] = rt[rr];
-                      }
-                    }
-                  }
-                  store_a(Ac, lane, At);
-                  for (int a = 0; a < 8; ++a) store_row(Zw, a, lane, Z[a][0], Z[a][1]);
-                  __syncwarp();
-                  double add[2] = {0.0, 0.0};
-                  tile_product(Ac, Zw, zrow, 8, lane, add);
-                  const int at = i * NC - i * (i - 1) / 2 + (l - i);
+            // without the elimination (mode 0) the same product is U, and its right-hand side the gradient
+            double vi[6] = {0, 0, 0, 0, 0, 0}, q[3], det;
+            bool ok = true;
+            if (mode == 1) {
+              ok = invert_point(V, lam, vi, &det);
+              if (!ok && !isfinite(det)) {   // a point at infinity contributes nothing
+                const double zero2[2][6] = {};
 #pragma unroll
-                  for (int pr = 0; pr < L::kPairs; ++pr)
-                    if (pr == at) { acc[pr][0] += add[0]; acc[pr][1] += add[1]; }
-                  __syncwarp();
+                for (int c = 0; c < NC; ++c) {
+                  if (c < N) store_a(Aw + c * 6 * kTileLd, lane, zero2);
+                  r[c][0] = r[c][1] = 0.0;
                 }
               }
+            }
+            mul_sym3(vi, gb, q);
+            int pr = 0;
+#pragma unroll
+            for (int i = 0; i < NC; ++i) {
+              double BV[2][3];
+              mul_sym3(vi, B[i][0], BV[0]);
+              mul_sym3(vi, B[i][1], BV[1]);
+#pragma unroll
+              for (int l = i; l < NC; ++l, ++pr) {
+                if (l >= N || (l != i && mode == 0)) continue;
+                store_z(Zw, Aw + l * 6 * kTileLd, lane, BV, B[l], i == l, ok);
+                if (i == l) {
+                  const double e0 = r[i][0] - (B[i][0][0] * q[0] + B[i][0][1] * q[1] + B[i][0][2] * q[2]);
+                  const double e1 = r[i][1] - (B[i][1][0] * q[0] + B[i][1][1] * q[1] + B[i][1][2] * q[2]);
+                  store_row(Zw, 6, lane, ok ? e0 : 0.0, ok ? e1 : 0.0);
+                  store_row(Zw, 7, lane, r[i][0], r[i][1]);
+                }
+                __syncwarp();
+                tile_product(Aw + i * 6 * kTileLd, Zw, zrow, i == l ? 8 : 6, lane, acc[pr]);
+                __syncwarp();
+              }
+            }
+            // tracks that name a camera twice: their observation pairs one per round and point
+            if (__any_sync(0xffffffffu, twice)) {
+              double vi[6] = {0, 0, 0, 0, 0, 0}, q[3] = {0, 0, 0};
+              bool ok = false, dead = false;
+              const int nt = twice ? n : 0;
+              {
+                double V2[6] = {0, 0, 0, 0, 0, 0}, gb2[3] = {0, 0, 0}, det;
+                for (int t = 0; t < nt; ++t) {
+                  const int k = o0 + t;
+                  const CamS& cm = cams[b.cam[k]];
+                  ObsLin ol;
+                  double rr[2], Bt[2][3];
+                  project_obs(cm, X, b.meas[2 * (size_t)k], b.meas[2 * (size_t)k + 1], ol);
+                  const double w = huber_weight(thr, ol.e);
+                  b.w[k] = w;
+                  err += w * w * (ol.e[0] * ol.e[0] + ol.e[1] * ol.e[1]);
+                  weigh(ol, w, rr);
+                  point_block(cm, ol, Bt);
+                  add_point(Bt, rr, V2, gb2);
+                }
+                if (twice) {
+                  gbmax = fmax(gbmax, fmax(fabs(gb2[0]), fmax(fabs(gb2[1]), fabs(gb2[2]))));
+                  vdmax = fmax(vdmax, fmax(V2[0], fmax(V2[3], V2[5])));
+                  ok = invert_point(V2, lam, vi, &det);
+                  dead = mode == 1 && !ok && !isfinite(det);
+                  mul_sym3(vi, gb2, q);
+                }
+              }
+#pragma unroll 1
+              for (int i = 0; i < N; ++i)
+#pragma unroll 1
+                for (int l = i; l < N; ++l) {
+                  if (mode == 0 && l != i) continue;
+                  double* Ac = Aw + i * 6 * kTileLd;
+                  int t = 0, u = -1;
+                  for (;;) {
+                    // the lane's next pair (t, u) of an observation in camera i with one in camera l; the
+                    // diagonal's U term and gradient come with t == u (mode 0 has only those)
+                    bool have = false;
+                    while (!have) {
+                      if (++u >= nt) { u = 0; ++t; }
+                      if (t >= nt) break;
+                      have = b.cam[o0 + t] == i && b.cam[o0 + u] == l && (mode == 1 || t == u);
+                    }
+                    if (!__any_sync(0xffffffffu, have)) break;
+                    double At[2][6] = {}, Z[8][2] = {};
+                    if (have && !dead) {
+                      double Au[2][6], Bt[2][3], Bu[2][3], rt[2], ru[2], BV[2][3];
+                      ObsLin ol;
+                      project_obs(cams[i], X, b.meas[2 * (size_t)(o0 + t)], b.meas[2 * (size_t)(o0 + t) + 1], ol);
+                      weigh(ol, b.w[o0 + t], rt);
+                      point_block(cams[i], ol, Bt);
+                      camera_block(ol, At);
+                      project_obs(cams[l], X, b.meas[2 * (size_t)(o0 + u)], b.meas[2 * (size_t)(o0 + u) + 1], ol);
+                      weigh(ol, b.w[o0 + u], ru);
+                      point_block(cams[l], ol, Bu);
+                      camera_block(ol, Au);
+                      mul_sym3(vi, Bt[0], BV[0]);
+                      mul_sym3(vi, Bt[1], BV[1]);
+                      for (int rr = 0; rr < 2; ++rr) {
+                        double P[2];
+                        for (int cc = 0; cc < 2; ++cc)
+                          P[cc] = ((t == u && rr == cc) ? 1.0 : 0.0) -
+                                  (mode == 1 ? BV[rr][0] * Bu[cc][0] + BV[rr][1] * Bu[cc][1] + BV[rr][2] * Bu[cc][2] : 0.0);
+                        const bool use = mode == 0 || ok;
+                        for (int a = 0; a < 6; ++a) Z[a][rr] = use ? P[0] * Au[0][a] + P[1] * Au[1][a] : 0.0;
+                        if (t == u) {
+                          if (mode == 1 && ok) Z[6][rr] = rt[rr] - (Bt[rr][0] * q[0] + Bt[rr][1] * q[1] + Bt[rr][2] * q[2]);
+                          Z[7][rr] = rt[rr];
+                        }
+                      }
+                    }
+                    store_a(Ac, lane, At);
+                    for (int a = 0; a < 8; ++a) store_row(Zw, a, lane, Z[a][0], Z[a][1]);
+                    __syncwarp();
+                    double add[2] = {0.0, 0.0};
+                    tile_product(Ac, Zw, zrow, 8, lane, add);
+                    const int at = i * NC - i * (i - 1) / 2 + (l - i);
+#pragma unroll
+                    for (int pr = 0; pr < L::kPairs; ++pr)
+                      if (pr == at) { acc[pr][0] += add[0]; acc[pr][1] += add[1]; }
+                    __syncwarp();
+                  }
+                }
+            }
           }
         }
-        // the warps' sums, in warp order
+        // the slots' sums
         __syncwarp();
+        const bool more = OWN > 1 && wid + NW < chunks;   // something was kept
 #pragma unroll
-        for (int t = 0; t < L::kPairs; ++t)
-          *reinterpret_cast<double2*>(Aw + t * 64 + (lane >> 2) * 8 + 2 * (lane & 3)) = make_double2(acc[t][0], acc[t][1]);
-        const double errs = block_sum<NT>(err, red);
+        for (int t = 0; t < L::kPairs; ++t) {
+          double2* at = reinterpret_cast<double2*>(Aw + t * 64 + (lane >> 2) * 8 + 2 * (lane & 3));
+          if (OWN == 2) {
+            at[0] = more ? make_double2(kept[t][0], kept[t][1]) : make_double2(acc[t][0], acc[t][1]);
+            at[L::kTile / 2] = more ? make_double2(acc[t][0], acc[t][1]) : make_double2(0.0, 0.0);
+          } else {
+            at[0] = more ? make_double2(kept[t][0] + acc[t][0], kept[t][1] + acc[t][1]) : make_double2(acc[t][0], acc[t][1]);
+          }
+        }
+        if (OWN == 2) {
+          Zw[lane] = more ? kept_err : err;
+          Zw[32 + lane] = more ? err : 0.0;
+        } else {
+          Zw[lane] = more ? kept_err + err : err;
+        }
         const double gm = block_max<NT>(gbmax, red);
         const double vm = block_max<NT>(vdmax, red);
-        for (int e = tid; e < L::kPairs * 64; e += NT) {
-          double s = 0.0;
-          for (int w = 0; w < NW; ++w) s += dyn[w * L::kWarp + e];
+        for (int e = tid; e < L::kTile; e += NT) {
+          const double s = slots_total(dyn + e, L::kTile);
           int i = 0, t = e >> 6;
           while (t >= NC - i) { t -= NC - i; ++i; }
           const int l = i + t, a = (e >> 3) & 7, c = e & 7;
@@ -594,6 +638,7 @@ __global__ void __launch_bounds__(NT, NT > 128 ? 1 : 384 / NT) k_batched_lm(Batc
         }
         __syncthreads();
         if (wid == 0) {
+          const double errs = warp_sum(slots_total(dyn + L::kA + lane, 32));
           double gx = lane < 6 * N ? fabs(ga[lane]) : 0.0, dx = (mode == 0 && lane < 6 * N) ? udiag[lane] : -1e30;
           gx = warp_max(gx);
           dx = warp_max(dx);
@@ -626,59 +671,62 @@ __global__ void __launch_bounds__(NT, NT > 128 ? 1 : 384 / NT) k_batched_lm(Batc
       __syncthreads();
       if (!si[3]) {
         // ---- points: back-substitution, trial points, trial cost with frozen weights ----
-        double nerr = 0.0, d2 = 0.0, dg = 0.0;
-        for (int j = tid; j < M; j += NT) {
-          const size_t g = (size_t)(pt0 + j);
-          const int o0 = b.ptr[g], n = b.ptr[g + 1] - o0;
-          const double X[3] = {Xc[3 * g], Xc[3 * g + 1], Xc[3 * g + 2]};
-          double V[6] = {0, 0, 0, 0, 0, 0}, gb[3] = {0, 0, 0}, s[3] = {0, 0, 0}, vi[6], db[3] = {0, 0, 0}, det;
-          for (int t = 0; t < n; ++t) {
-            const int k = o0 + t;
-            const int c = b.cam[k];
-            const double2 m = *reinterpret_cast<const double2*>(b.meas + 2 * (size_t)k);
-            const CamS& cm = cams[c];
-            ObsLin ol;
-            double r[2], B[2][3];
-            project_obs(cm, X, m.x, m.y, ol);
-            weigh(ol, b.w[k], r);
-            point_block(cm, ol, B);
-            add_point(B, r, V, gb);
-            // A da = P (dT + omega x v)
-            const double* d = da + 6 * c;
-            const double t0 = d[0] + (d[4] * ol.v[2] - d[5] * ol.v[1]);
-            const double t1 = d[1] + (d[5] * ol.v[0] - d[3] * ol.v[2]);
-            const double t2 = d[2] + (d[3] * ol.v[1] - d[4] * ol.v[0]);
-            const double a0 = ol.P[0] * t0 + ol.P[1] * t2, a1 = ol.P[2] * t1 + ol.P[3] * t2;
+        for (int sl = wid; sl < kSlots; sl += NW) {
+          double nerr = 0.0, d2 = 0.0, dg = 0.0;
+          for (int j = 32 * sl + lane; j < M; j += 32 * kSlots) {
+            const size_t g = (size_t)(pt0 + j);
+            const int o0 = b.ptr[g], n = b.ptr[g + 1] - o0;
+            const double X[3] = {Xc[3 * g], Xc[3 * g + 1], Xc[3 * g + 2]};
+            double V[6] = {0, 0, 0, 0, 0, 0}, gb[3] = {0, 0, 0}, s[3] = {0, 0, 0}, vi[6], db[3] = {0, 0, 0}, det;
+            for (int t = 0; t < n; ++t) {
+              const int k = o0 + t;
+              const int c = b.cam[k];
+              const double2 m = *reinterpret_cast<const double2*>(b.meas + 2 * (size_t)k);
+              const CamS& cm = cams[c];
+              ObsLin ol;
+              double r[2], B[2][3];
+              project_obs(cm, X, m.x, m.y, ol);
+              weigh(ol, b.w[k], r);
+              point_block(cm, ol, B);
+              add_point(B, r, V, gb);
+              // A da = P (dT + omega x v)
+              const double* d = da + 6 * c;
+              const double t0 = d[0] + (d[4] * ol.v[2] - d[5] * ol.v[1]);
+              const double t1 = d[1] + (d[5] * ol.v[0] - d[3] * ol.v[2]);
+              const double t2 = d[2] + (d[3] * ol.v[1] - d[4] * ol.v[0]);
+              const double a0 = ol.P[0] * t0 + ol.P[1] * t2, a1 = ol.P[2] * t1 + ol.P[3] * t2;
 #pragma unroll
-            for (int q = 0; q < 3; ++q) s[q] += B[0][q] * a0 + B[1][q] * a1;
-          }
-          if (invert_point(V, lam, vi, &det)) {
+              for (int q = 0; q < 3; ++q) s[q] += B[0][q] * a0 + B[1][q] * a1;
+            }
+            if (invert_point(V, lam, vi, &det)) {
 #pragma unroll
-            for (int q = 0; q < 3; ++q) s[q] = gb[q] - s[q];
-            mul_sym3(vi, s, db);
-            d2 += db[0] * db[0] + db[1] * db[1] + db[2] * db[2];
-            dg += db[0] * gb[0] + db[1] * gb[1] + db[2] * gb[2];
+              for (int q = 0; q < 3; ++q) s[q] = gb[q] - s[q];
+              mul_sym3(vi, s, db);
+              d2 += db[0] * db[0] + db[1] * db[1] + db[2] * db[2];
+              dg += db[0] * gb[0] + db[1] * gb[1] + db[2] * gb[2];
+            }
+            const double Xn[3] = {X[0] + db[0], X[1] + db[1], X[2] + db[2]};
+            Xt[3 * g] = Xn[0];
+            Xt[3 * g + 1] = Xn[1];
+            Xt[3 * g + 2] = Xn[2];
+            for (int t = 0; t < n; ++t) {
+              const int k = o0 + t;
+              const double2 m = *reinterpret_cast<const double2*>(b.meas + 2 * (size_t)k);
+              ObsLin ol;
+              project_obs(tcams[b.cam[k]], Xn, m.x, m.y, ol);
+              const double wk = b.w[k];
+              nerr += wk * wk * (ol.e[0] * ol.e[0] + ol.e[1] * ol.e[1]);
+            }
           }
-          const double Xn[3] = {X[0] + db[0], X[1] + db[1], X[2] + db[2]};
-          Xt[3 * g] = Xn[0];
-          Xt[3 * g + 1] = Xn[1];
-          Xt[3 * g + 2] = Xn[2];
-          for (int t = 0; t < n; ++t) {
-            const int k = o0 + t;
-            const double2 m = *reinterpret_cast<const double2*>(b.meas + 2 * (size_t)k);
-            ObsLin ol;
-            project_obs(tcams[b.cam[k]], Xn, m.x, m.y, ol);
-            const double wk = b.w[k];
-            nerr += wk * wk * (ol.e[0] * ol.e[0] + ol.e[1] * ol.e[1]);
-          }
+          part[0][sl][lane] = nerr;
+          part[1][sl][lane] = d2;
+          part[2][sl][lane] = dg;
         }
-        nerr = block_sum<NT>(nerr, red);
-        d2 = block_sum<NT>(d2, red);
-        dg = block_sum<NT>(dg, red);
+        __syncthreads();
         if (wid == 0) {
           const double dl = lane < 6 * N ? da[lane] : 0.0, gl = lane < 6 * N ? ga[lane] : 0.0;
-          d2 += warp_sum(dl * dl);
-          dg += warp_sum(dl * gl);
+          const double nerr = slots_warp_sum(part[0]);
+          const double d2 = slots_warp_sum(part[1]) + warp_sum(dl * dl), dg = slots_warp_sum(part[2]) + warp_sum(dl * gl);
           if (lane == 0) {
             si[4] = 0;
             if (sqrt(d2) < o.upd_thr * (sc[6] + o.upd_thr)) {
@@ -838,12 +886,25 @@ BatchKernel batch_kernel(int threads, int max_cams) {
   return threads == 64 ? batch_kernel_of<64, 4>() : threads == 128 ? batch_kernel_of<128, 4>() : batch_kernel_of<256, 4>();
 }
 
-// Threads per problem of a batch that sets no schedule.  A problem's passes take time in inverse
-// proportion to its warps, but the 256-thread instance runs one block per SM where the others keep 12
-// warps.  Measured (4 iterations, 50-800 points; ms with 64 / 128 / 256 threads): 61 problems 0.50 /
-// 0.29 / 0.17, 300: 0.61 / 0.34 / 0.26, 600: 0.73 / 0.39 / 0.46, 1200: 0.78 / 0.68 / 0.87, 4096: 2.19 /
-// 2.21 / 2.85 and, with 20-90 points, 0.58 / 0.75 / 1.60.
-int default_threads(int count, int sms) { return count <= 2 * sms ? 256 : count <= 8 * sms ? 128 : 64; }
+// Threads per problem of a batch that sets no schedule; they set the time alone, not the results.  A problem's
+// passes take time in inverse proportion to its warps as far as it has tiles of 32 points for them, but the
+// 256-thread instance runs one block per SM where the others keep 12 warps.  Measured (4 iterations, triplets
+// of 20-90, 50-300 and 50-800 points; ms with 64 / 128 / 256 threads), the lines lie where the best changes:
+//    148 problems  .103 .075 .066   .223 .137 .100   .488 .285 .170
+//    296           .113 .079 .123   .236 .164 .156   .510 .327 .227
+//    420           .130 .089 .177   .270 .186 .217   .578 .378 .325
+//    500           .131 .141 .230   .279 .186 .252   .608 .382 .381
+//   1000           .170 .214 .400   .338 .328 .463   .748 .565 .706
+//   1184           .194 .225 .464   .354 .371 .547   .751 .661 .823
+//   4096           .561 .729 1.57   1.16 1.22 1.88   2.24 2.19 2.88
+// With four cameras the second line is the same, and from 256 points a problem on 256 threads are the best
+// at every count (50-800 points, 600 problems 1.03 .661 .626, 4096 4.16 4.24 3.95).
+int default_threads(int count, int sms, int points, int max_cams) {
+  const int per_sm = (count + sms - 1) / sms;
+  if (points >= 256) return per_sm <= 3 || max_cams > 3 ? 256 : 128;
+  if (points >= 128) return per_sm <= 2 ? 256 : per_sm <= 7 ? 128 : 64;
+  return per_sm <= 1 ? 256 : per_sm <= 3 ? 128 : 64;
+}
 
 int batch_resources(v3dba_batch_t h) {
   const int rc = h->res.acquire();
@@ -858,7 +919,7 @@ int launch_range(v3dba_batch_t h, int threads, int first, int last, const BatchO
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (threads == 0) threads = default_threads(last - first, sms);
+  if (threads == 0) threads = default_threads(last - first, sms, h->total_pts / h->d.count, h->max_cams);
   V3DBA_CUDA_TRY(cudaMemsetAsync(h->d.queue, 0, sizeof(unsigned), h->stream));
   const BatchKernel k = batch_kernel(threads, h->max_cams);
   V3DBA_CUDA_TRY(cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem));
