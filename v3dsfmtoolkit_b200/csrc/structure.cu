@@ -703,13 +703,16 @@ int build_structure_device(const v3dba_problem* p, const DevAlloc& alloc, cudaSt
 }
 
 int build_schur_groups(DevState& s, const DevAlloc& alloc, cudaStream_t st) {
-  // Points below which the plan costs more than a call saves (about 0.1 ms against 20 us an iteration)
-  constexpr int kMinObs = 65536;
   s.gr_n = 0;
   const char* want = std::getenv("V3DBA_SCHUR");
   const bool force = want && !std::strcmp(want, "groups");
   const int M = s.d.M, DA = s.d.DA;
-  if ((want && !std::strcmp(want, "pairs")) || M <= 0 || s.nb <= 0 || (!force && s.d.K < kMinObs)) return V3DBA_OK;
+  // Observations below which the plan (about 0.1 ms) costs more than a call saves, or the groups are the slower
+  // way (us an iteration, pairs / groups; 9 unknowns a camera: 77,000 observations 276 / 276, 132,000 302 / 301,
+  // 263,000 385 / 372; 13 unknowns, whose blocks leave room for two chunks an SM: 132,000 366 / 386, 263,000
+  // 499 / 492, 439,000 744 / 707; 11 unknowns: 132,000 326 / 334, 263,000 446 / 432).
+  const int min_obs = DA <= 9 ? 65536 : 262144;
+  if ((want && !std::strcmp(want, "pairs")) || M <= 0 || s.nb <= 0 || (!force && s.d.K < min_obs)) return V3DBA_OK;
   Scratch sc;
   sc.st = st;
   int rc;
@@ -764,9 +767,9 @@ int build_schur_groups(DevState& s, const DevAlloc& alloc, cudaStream_t st) {
     }
   }
   // A partial sum is written and read back where a pair gathers 340 bytes, and a chunk pays for 8 x 8
-  // tiles and whole DMMA steps: worth it from about ten pairs a sum on (158 cameras, us per iteration, pairs
-  // against groups: 9,981 points, 6 pairs a sum, 308 / 314; 16,000 points, 10 pairs, 319 / 326; 24,000
-  // points, 14 pairs, 363 / 337).
+  // tiles and whole DMMA steps: even from about ten pairs a sum on (158 cameras, us an iteration, pairs / groups,
+  // with and without 7 global unknowns: 6 pairs a sum 316 / 324 and 275 / 276, 8: 327 / 326 and 277 / 277, 9.4:
+  // 328 / 329 and 286 / 278, 11: 335 / 334 and 288 / 278, 13: 363 / 353 and 294 / 290, 21: 426 / 396 and 333 / 312).
   if (chunks.empty() || entries > 0x3fffffff || (!force && 10 * entries > s.P)) return V3DBA_OK;
   // the costly chunks first, so that the last ones to run are short
   std::stable_sort(chunks.begin(), chunks.end(),
