@@ -79,15 +79,17 @@ struct HostCopy {
   const void* src;
   size_t bytes;
 };
-// Copies device -> caller (down) and waits for it.  Large copies (kRingDown bytes and more) go through a
-// ring of pinned slots: the driver's own path to pageable memory copies with one thread, which also takes
+// Copies device -> caller (down) and waits for it.  Large copies to pageable memory (kRingDown bytes and more)
+// go through a ring of pinned slots: the driver's own path to pageable memory copies with one thread, which also takes
 // the page faults of arrays that the caller has just allocated (42 MB of points into new arrays: 5.2 ms
-// against 0.7 ms on the bus), so a few threads copy from the slots instead (3.0 ms).
+// against 0.7 ms on the bus), so a few threads copy from the slots instead (3.0 ms).  Pinned arrays are copied
+// directly (42 MB: 0.87 ms; through the slots 1.08).
 int copy_down(const std::vector<HostCopy>& list, cudaStream_t st);
-// Copies the caller's arrays -> device, from kRingUp bytes on the same way round (67 MB: 6.4 -> 3.3 ms);
-// smaller arrays are often in this thread's cache, and reading them from other cores costs more than it
-// saves (16 MB: 0.8 -> 2.4 ms).  Later work on the stream is ordered after the copies, and the caller's
-// arrays have been read when it returns.
+// Copies the caller's arrays -> device, pageable ones from kRingUp bytes on the same way round (67 MB: 6.4 ->
+// 3.3 ms); smaller arrays are often in this thread's cache, and reading them from other cores costs more than
+// it saves (a rotation problem of 16 MB created: 1.0 -> 1.7 ms with its arrays in cache, 1.8 -> 2.0 out of it).
+// Later work on the stream is ordered after the copies.  Pinned arrays have been read when the stream has been
+// waited for, which every entry point does before it returns.
 int copy_up(const std::vector<HostCopy>& list, cudaStream_t st);
 constexpr size_t kRingDown = (size_t)8 << 20, kRingUp = (size_t)32 << 20;
 

@@ -65,7 +65,7 @@ bool injected_alloc_failure() {
 
 namespace {
 
-// Pinned slots for large downloads, each with the event of its copy.
+// Pinned slots for large copies in either direction, each with the event of its copy.
 struct Ring {
   static constexpr int kSlots = 8;
   static constexpr size_t kSlot = (size_t)2 << 20;
@@ -190,8 +190,16 @@ void CallRes::release() {
 
 namespace {
 
-// A list of copies, the large ones cut into pieces of at most a slot.  The pieces end where a 2 MB page
-// of the caller's memory ends, so that no two threads fault one page.
+// Memory that the DMA engine reads and writes itself: pinned, registered or managed.
+bool direct(const void* host) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, host) == cudaSuccess) return a.type != cudaMemoryTypeUnregistered;
+  cudaGetLastError();
+  return false;
+}
+
+// A list of copies, the large ones to and from pageable memory cut into pieces of at most a slot.  The pieces
+// end where a 2 MB page of the caller's memory ends, so that no two threads fault one page.
 struct Pieces {
   std::vector<HostCopy> p;
   bool staged = false;
@@ -201,12 +209,16 @@ struct Pieces {
   Pieces(const std::vector<HostCopy>& list, bool down, cudaStream_t st) {
     constexpr size_t kPieceMin = (size_t)256 << 10;
     size_t large = 0;
-    for (const HostCopy& c : list)
-      if (c.bytes >= kPieceMin) large += c.bytes;
+    std::vector<char> cut(list.size(), 0);
+    for (size_t i = 0; i < list.size(); ++i) {
+      cut[i] = list[i].bytes >= kPieceMin && !direct(down ? list[i].dst : list[i].src);
+      if (cut[i]) large += list[i].bytes;
+    }
     staged = large >= (down ? kRingDown : kRingUp) && ring_acquire(ring) == V3DBA_OK;
-    for (const HostCopy& c : list) {
+    for (size_t i = 0; i < list.size(); ++i) {
+      const HostCopy& c = list[i];
       if (!c.bytes) continue;
-      if (!staged || c.bytes < kPieceMin) {
+      if (!staged || !cut[i]) {
         if (err == cudaSuccess)
           err = cudaMemcpyAsync(c.dst, c.src, c.bytes, down ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice, st);
         continue;
