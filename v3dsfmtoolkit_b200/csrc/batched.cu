@@ -862,10 +862,8 @@ int bupload(v3dba_batch_t h, T** p, const std::vector<T>& v) {
 
 void batch_free(v3dba_batch_t h) {
   if (!h) return;
-  if (h->stream) {
+  if (h->stream)
     for (void* p : h->allocs) cudaFreeAsync(p, h->stream);
-    cudaStreamSynchronize(h->stream);
-  }
   h->res.release();
   delete h;
 }

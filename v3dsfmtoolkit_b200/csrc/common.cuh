@@ -58,15 +58,16 @@ struct Arena {
 
 // What a call or handle needs from the driver besides memory: a stream, two timing events and a page of
 // pinned memory.  Creating and destroying them took 2.6-3.2 and 0.9 ms per handle (80 ms and more on a
-// busy host), a multiple of a small adjustment, so a few sets are kept per device for the next call.
-// acquire() takes one from the pool or makes one; release() returns it (its stream must be idle), or
-// destroys it when kCallResKept are kept already.  Any thread may call both; a set has one owner at a
-// time.  The kept sets are destroyed at process exit.
+// busy host), a multiple of a small adjustment, so a few sets are kept per context for the next call.
+// acquire() takes one of the current context from the pool or makes one; release() waits for the stream and
+// returns the set, or destroys it when kCallResKept are kept already or the stream reported an error.  A set of
+// a context that has ended (cudaDeviceReset) is never handed out again.  Any thread may call both; a set has
+// one owner at a time.  The kept sets are destroyed at process exit.
 struct CallRes {
   cudaStream_t st = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   double* pinned = nullptr;   // kCallResDoubles doubles
-  int dev = -1;
+  uint64_t ctx = 0;           // the driver's number of its context
   int acquire();
   void release();
 };

@@ -10,6 +10,8 @@
 #include <system_error>
 #include <thread>
 
+#include <cuda.h>
+
 #include "common.cuh"
 
 namespace v3dba {
@@ -71,9 +73,43 @@ struct Ring {
   static constexpr size_t kSlot = (size_t)2 << 20;
   char* mem = nullptr;
   cudaEvent_t ev[kSlots] = {};
-  int dev = -1;
+  uint64_t ctx = 0;
 };
 constexpr int kRingsKept = 2;
+// All that is kept, whatever its context; what a device reset left of one is among it, never used again.
+constexpr size_t kAllKept = 64;
+
+// The driver's number of a context; it is not used again after the context has ended.
+struct Driver {
+  CUresult(CUDAAPI* id)(CUcontext, unsigned long long*) = nullptr;
+  CUresult(CUDAAPI* of_stream)(CUstream, CUcontext*) = nullptr;
+};
+const Driver& driver() {
+  static const Driver d = [] {
+    Driver n;
+    void* f = nullptr;
+    if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault) == cudaSuccess)
+      n.id = reinterpret_cast<decltype(n.id)>(f);
+    if (cudaGetDriverEntryPoint("cuStreamGetCtx", &f, cudaEnableDefault) == cudaSuccess)
+      n.of_stream = reinterpret_cast<decltype(n.of_stream)>(f);
+    cudaGetLastError();
+    return n;
+  }();
+  return d;
+}
+// The current context, and a stream's; 0 where there is none.
+uint64_t current_context() {
+  unsigned long long id = 0;
+  return driver().id && driver().id(nullptr, &id) == CUDA_SUCCESS ? id : 0;
+}
+uint64_t stream_context(cudaStream_t st) {
+  CUcontext c = nullptr;
+  unsigned long long id = 0;
+  return driver().id && driver().of_stream && driver().of_stream(st, &c) == CUDA_SUCCESS &&
+                 driver().id(c, &id) == CUDA_SUCCESS
+             ? id
+             : 0;
+}
 
 void destroy(CallRes& r) {
   if (r.pinned) cudaFreeHost(r.pinned);
@@ -89,8 +125,9 @@ void destroy(Ring& r) {
   r = Ring();
 }
 
-// Never destroyed itself (other threads may be in a call when the process ends); what it keeps is
-// destroyed by a handler that runs before the CUDA runtime's own, registered after its first use.
+// Never destroyed itself (other threads may be in a call when the process ends); what it keeps of the
+// context that is current then is destroyed by a handler that runs before the CUDA runtime's own, registered
+// after its first use.
 struct Kept {
   std::mutex m;
   std::vector<CallRes> res;
@@ -105,8 +142,11 @@ Kept& kept() {
       Kept& k2 = kept();
       std::lock_guard<std::mutex> lock(k2.m);
       k2.closing = true;
-      for (CallRes& r : k2.res) destroy(r);
-      for (Ring& r : k2.rings) destroy(r);
+      const uint64_t ctx = current_context();
+      for (CallRes& r : k2.res)
+        if (r.ctx == ctx) destroy(r);
+      for (Ring& r : k2.rings)
+        if (r.ctx == ctx) destroy(r);
       k2.res.clear();
       k2.rings.clear();
     });
@@ -116,25 +156,34 @@ Kept& kept() {
 }
 
 template <typename T>
-bool take(std::vector<T>& v, int dev, T& out) {
+bool take(std::vector<T>& v, uint64_t ctx, T& out) {
   for (size_t i = v.size(); i-- > 0;)
-    if (v[i].dev == dev) {
+    if (v[i].ctx == ctx) {
       out = v[i];
       v.erase(v.begin() + (long)i);
       return true;
     }
   return false;
 }
+// Keeps x if its context is known and has fewer than `most`; false: the caller destroys it.
+template <typename T>
+bool put(std::vector<T>& v, const T& x, int most) {
+  if (x.ctx == 0 || v.size() >= kAllKept) return false;
+  for (const T& y : v) most -= y.ctx == x.ctx;
+  if (most <= 0) return false;
+  v.push_back(x);
+  return true;
+}
 
+// A ring of the current context.
 int ring_acquire(Ring& r) {
-  int dev = 0;
-  V3DBA_CUDA_TRY(cudaGetDevice(&dev));
-  {
+  const uint64_t ctx = current_context();
+  if (ctx) {
     Kept& k = kept();
     std::lock_guard<std::mutex> lock(k.m);
-    if (take(k.rings, dev, r)) return V3DBA_OK;
+    if (take(k.rings, ctx, r)) return V3DBA_OK;
   }
-  r.dev = dev;
+  r.ctx = ctx;
   cudaError_t e = cudaMallocHost(reinterpret_cast<void**>(&r.mem), Ring::kSlots * Ring::kSlot);
   for (int t = 0; t < Ring::kSlots && e == cudaSuccess; ++t) e = cudaEventCreateWithFlags(&r.ev[t], cudaEventDisableTiming);
   if (e == cudaSuccess) return V3DBA_OK;
@@ -145,25 +194,20 @@ int ring_acquire(Ring& r) {
 void ring_release(Ring& r) {
   Kept& k = kept();
   std::lock_guard<std::mutex> lock(k.m);
-  if ((int)k.rings.size() < kRingsKept && !k.closing) {
-    k.rings.push_back(r);
-    r = Ring();
-  } else {
-    destroy(r);
-  }
+  if (!k.closing && put(k.rings, r, kRingsKept)) r = Ring();
+  else destroy(r);
 }
 
 }  // namespace
 
 int CallRes::acquire() {
-  int d = 0;
-  V3DBA_CUDA_TRY(cudaGetDevice(&d));
-  {
+  V3DBA_CUDA_TRY(cudaFree(nullptr));   // the current context, made if there is none yet or it was reset
+  ctx = current_context();
+  if (ctx) {
     Kept& k = kept();
     std::lock_guard<std::mutex> lock(k.m);
-    if (take(k.res, d, *this)) return V3DBA_OK;
+    if (take(k.res, ctx, *this)) return V3DBA_OK;
   }
-  dev = d;
   cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreate(&ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&ev1);
@@ -176,16 +220,12 @@ int CallRes::acquire() {
 
 void CallRes::release() {
   if (!st) return;
+  const bool sound = cudaStreamSynchronize(st) == cudaSuccess;
+  if (!sound) cudaGetLastError();
   Kept& k = kept();
   std::lock_guard<std::mutex> lock(k.m);
-  int same = 0;
-  for (const CallRes& r : k.res) same += r.dev == dev;
-  if (same < kCallResKept && !k.closing) {
-    k.res.push_back(*this);
-    *this = CallRes();
-  } else {
-    destroy(*this);
-  }
+  if (sound && !k.closing && put(k.res, *this, kCallResKept)) *this = CallRes();
+  else destroy(*this);
 }
 
 namespace {
@@ -214,7 +254,9 @@ struct Pieces {
       cut[i] = list[i].bytes >= kPieceMin && !direct(down ? list[i].dst : list[i].src);
       if (cut[i]) large += list[i].bytes;
     }
-    staged = large >= (down ? kRingDown : kRingUp) && ring_acquire(ring) == V3DBA_OK;
+    // (the slots' events are the current context's and cannot be recorded on another one's stream)
+    staged = large >= (down ? kRingDown : kRingUp) && cudaFree(nullptr) == cudaSuccess &&
+             stream_context(st) == current_context() && ring_acquire(ring) == V3DBA_OK;
     for (size_t i = 0; i < list.size(); ++i) {
       const HostCopy& c = list[i];
       if (!c.bytes) continue;

@@ -34,6 +34,7 @@ struct Dims {
 // (multiple of 16 bytes) so that it moves with vector loads.
 struct DevState {
   Dims d;
+  uint64_t ctx = 0;         // the handle's context (CallRes::ctx)
   // structure
   int* o_cam = nullptr;     // [K] camera of permuted observation k
   int* o_pt = nullptr;      // [K] point of permuted observation k

@@ -1883,17 +1883,14 @@ inline PartLayout part_layout(const DevState& s) {
 
 template <int MODEL, int DA, int DC, typename Real>
 struct Ops {
-  // Shared memory of the staged kernels, allowed on the current device the first time it is asked for.
+  // Shared memory of the staged kernels, allowed in the handle's context the first time it is asked for.
   static constexpr size_t kCamSmem = (size_t)kCamWarps * camera_stage_bytes<DA, DC, Real>();
   static constexpr size_t kRhsSmem = (size_t)kCamWarps * rhs_stage_bytes<DA, DC, Real>();
   static constexpr size_t kSchurSmem = (size_t)4 * schur_stage_bytes<DA, Real>();
   static constexpr size_t kBothSmem = kRhsSmem > kSchurSmem ? kRhsSmem : kSchurSmem;
-  static void allow_stages() {
-    static std::atomic<uint64_t> allowed{0};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    const uint64_t bit = 1ull << (dev & 63);
-    if (allowed.load() & bit) return;
+  static void allow_stages(uint64_t ctx) {
+    static std::atomic<uint64_t> allowed[8];   // contexts, by the last bits of their number
+    if (ctx != 0 && allowed[ctx % 8].load() == ctx) return;
     constexpr auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
     cudaFuncSetAttribute(k_camera_chunks<DA, DC, Real>, attr, (int)kCamSmem);
     cudaFuncSetAttribute(k_rhs_chunks<DA, DC, Real>, attr, (int)kRhsSmem);
@@ -1904,7 +1901,7 @@ struct Ops {
       cudaFuncSetAttribute(k_schur_groups<DA>, attr, kGroupSmem);
       cudaFuncSetAttribute(k_groups_merged<DA, DC>, attr, kGroupSmem);
     }
-    allowed.fetch_or(bit);
+    allowed[ctx % 8].store(ctx);
   }
   static bool grouped(const DevState& s) { return !stores_products<Real>() && s.gr_n > 0; }
   // shared memory of the grouped launches: a group's, or the rhs chunks' of one block if that is more
@@ -1914,7 +1911,7 @@ struct Ops {
   }
   // Launches one stage of the LM iteration (see LmStage in lm.cuh).
   static int stage(DevState& s, int id, int init_lambda, double tau, cudaStream_t st) {
-    allow_stages();
+    allow_stages(s.ctx);
     const PartLayout pl = part_layout<DA, DC>(s);
     const int bp = cdiv(std::max(s.d.M, 1), kPtThreads);                  // one lane per point
     const int bl = lane_blocks(s.d.M, kLinLanes);                          // the linearisation

@@ -443,7 +443,6 @@ void release(v3dba_rotations h) {
   if (!h) return;
   if (h->arena) cudaFreeAsync(h->arena, h->st);
   if (h->trace) cudaFreeAsync(h->trace, h->st);
-  if (h->st) cudaStreamSynchronize(h->st);
   h->res.release();
   delete h;
 }

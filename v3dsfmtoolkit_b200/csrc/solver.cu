@@ -157,10 +157,8 @@ void free_handle(v3dba_handle h) {
   if (!h) return;
   tile_chol_free(h->chol);
   pcg_free(h->pcg);
-  if (h->stream) {
+  if (h->stream)
     for (void* p : h->allocs) cudaFreeAsync(p, h->stream);
-    cudaStreamSynchronize(h->stream);
-  }
   gnn_graph_free(h->gnn);
   h->res.release();
   delete h;
@@ -424,6 +422,7 @@ int v3dba_create(const v3dba_problem* p, v3dba_handle* out) {
 
   TRY(h->res.acquire());
   h->stream = h->res.st;
+  s.ctx = h->res.ctx;
   h->ev0 = h->res.ev0;
   h->ev1 = h->res.ev1;
   h->h_scalars = h->res.pinned;

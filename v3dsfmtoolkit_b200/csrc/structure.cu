@@ -848,7 +848,6 @@ struct CallScope {
   }
   ~CallScope() {
     if (sc) delete sc;   // frees the buffers on the stream
-    if (st) cudaStreamSynchronize(st);
     res.release();
   }
 };
