@@ -1075,7 +1075,8 @@ namespace {
 // The flat arrays straight to the device: the checks, the camera bytes and the point offsets are made
 // there (4096 triplets, 1.7M points: 86 -> 6.5 ms against the host's loops).  Returns V3DBA_OK with
 // *out == nullptr where the host's way has to be taken: an index or value that it then refuses with its
-// own code, or observations that are not in point order.
+// own code, or observations that are not in point order (a look at the first problems, in_point_order, keeps
+// most of those from the upload).
 int batch_create_device(int count, const int* n_cameras, const int* n_points, const int* n_measurements,
                         const double* thr, const double* K, const double* R, const double* T, const double* X,
                         const double* measurements, const int* view, const int* point, v3dba_batch_t* out) {
@@ -1180,6 +1181,21 @@ int batch_create_device(int count, const int* n_cameras, const int* n_points, co
   return V3DBA_OK;
 }
 
+// Whether the first kDeviceCheckMin observations of flat problems are in point order (10 us).  A program's
+// problems mostly are or are not, all alike: without this look 4096 triplets out of order were uploaded for
+// nothing (created in 127-157 ms instead of 121).
+bool in_point_order(int count, const int* n_measurements, const int* point) {
+  int64_t left = kDeviceCheckMin;
+  for (int p = 0; p < count && left > 0; ++p) {
+    const int n = (int)std::min<int64_t>(n_measurements[p], left);
+    for (int k = 1; k < n; ++k)
+      if (point[k] < point[k - 1]) return false;
+    point += n_measurements[p];
+    left -= n;
+  }
+  return true;
+}
+
 }  // namespace
 
 extern "C" {
@@ -1221,7 +1237,8 @@ int v3dba_batch_create_flat(int count, const int* n_cameras, const int* n_points
   int ndev = 0;
   const bool device = cudaGetDeviceCount(&ndev) == cudaSuccess && ndev > 0;
   if (!device) cudaGetLastError();
-  if (usual && device && oo + po >= (size_t)kDeviceCheckMin && oo <= 0x7fffffff && po <= 0x7fffffff - 1) {
+  if (usual && device && oo + po >= (size_t)kDeviceCheckMin && oo <= 0x7fffffff && po <= 0x7fffffff - 1 &&
+      in_point_order(count, n_measurements, point)) {
     const int rc = batch_create_device(count, n_cameras, n_points, n_measurements, inlier_threshold, K, R, T, X,
                                        measurements, view, point, out);
     if (rc || *out) return rc;
