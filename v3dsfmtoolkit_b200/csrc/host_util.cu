@@ -10,7 +10,7 @@
 #include <system_error>
 #include <thread>
 
-#include <cuda.h>
+#include <cudaTypedefs.h>
 
 #include "common.cuh"
 
@@ -79,19 +79,21 @@ constexpr int kRingsKept = 2;
 // All that is kept, whatever its context; what a device reset left of one is among it, never used again.
 constexpr size_t kAllKept = 64;
 
-// The driver's number of a context; it is not used again after the context has ended.
+// The driver's number of a context; it is not used again after the context has ended.  Each function is asked
+// for in the version whose type is named: later ones of cuStreamGetCtx take another argument.
 struct Driver {
-  CUresult(CUDAAPI* id)(CUcontext, unsigned long long*) = nullptr;
-  CUresult(CUDAAPI* of_stream)(CUstream, CUcontext*) = nullptr;
+  PFN_cuCtxGetId_v12000 id = nullptr;
+  PFN_cuStreamGetCtx_v9020 of_stream = nullptr;
 };
 const Driver& driver() {
   static const Driver d = [] {
     Driver n;
     void* f = nullptr;
-    if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault) == cudaSuccess)
-      n.id = reinterpret_cast<decltype(n.id)>(f);
-    if (cudaGetDriverEntryPoint("cuStreamGetCtx", &f, cudaEnableDefault) == cudaSuccess)
-      n.of_stream = reinterpret_cast<decltype(n.of_stream)>(f);
+    if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault) == cudaSuccess)
+      n.id = reinterpret_cast<PFN_cuCtxGetId_v12000>(f);
+    f = nullptr;
+    if (cudaGetDriverEntryPointByVersion("cuStreamGetCtx", &f, 9020, cudaEnableDefault) == cudaSuccess)
+      n.of_stream = reinterpret_cast<PFN_cuStreamGetCtx_v9020>(f);
     cudaGetLastError();
     return n;
   }();
