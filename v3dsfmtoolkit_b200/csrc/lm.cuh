@@ -131,7 +131,7 @@ constexpr int kGroupSmem = 72 * 1024;   // three blocks per SM
 __host__ __device__ constexpr int group_ld(int rows) { return (rows + 3) / 8 * 8 + 4; }
 __host__ __device__ constexpr int group_pad(int points) { return (points + 3) / 4 * 4; }
 __host__ __device__ constexpr int group_doubles(int points, int rows) {
-  return 3 * group_pad(points) * group_ld(rows) + 8 + 6 * group_pad(points) + (kGroupPoints + 3 * kGroupTrack) / 2;
+  return 3 * group_pad(points) * group_ld(rows) + 8 + 12 * group_pad(points) + (kGroupPoints + 3 * kGroupTrack) / 2;
 }
 
 // Stages of one LM iteration, in launch order.

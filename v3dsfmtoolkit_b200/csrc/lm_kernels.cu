@@ -1093,19 +1093,24 @@ __device__ __forceinline__ void schur_chunks_body(DevState s, double* __restrict
 }
 
 // FP64 blocks, points grouped by their cameras: one block per chunk of up to 32 points that the same L
-// cameras see.  With G_k = A_k^T B_k the chunk's part of the whole L x L block matrix is G Vinv G^T, G one row
-// per camera unknown and three columns per point, formed in shared memory (observations of a point in the
-// same camera add up first) and multiplied with DMMA.  Vinv = (V + lambda I)^-1 is k_point_eliminate's, as for
-// the pair lists, the right-hand side and the step, so that the system is one and the same where rounding
-// decides about it (a Cholesky factor of V + lambda I in its place left a point out, or turned a pivot's sign,
-// that the other parts kept); it multiplies the left fragment, nine FMAs for nine DMMAs.
+// cameras see.  With (V + lambda I)^-1 = F N F^T and G_k = A_k^T (B_k F) the chunk's part of the whole L x L
+// block matrix is G N G^T, G one row per camera unknown and three columns per point, formed in shared memory
+// (observations of a point in the same camera add up first) and multiplied with DMMA; N multiplies the left
+// fragment, nine FMAs for nine DMMAs.
+// F is C^-T of the Cholesky factor of V + lambda I and N = I, while every pivot keeps kGroupPivot of its diagonal
+// entry: the rounding of G then counts by B C^-T, whose entries are at most 1, and not by the condition number
+// of V (F = I throughout gave 24-iteration runs of 200 cameras 8% more error).  Below that rounding decides about
+// the pivot, and F = I with N = k_point_eliminate's own inverse, which the pair lists, the right-hand side and
+// the step use: the system stays one and the same.  (C^-T there left a point out, or turned a pivot's sign, that
+// the other parts kept.)
 // Every observation's blocks are read once per trial instead of once per pair (144 bytes instead of 340
 // times the pairs of its track), the gathers that bound the pair lists: their L2 to L1 traffic was 870
 // MB at 5.8 TB/s (pairs staged through shared memory and multiplied with DMMA reached 9.4 TB/s, and no
-// more).  200 cameras, 50,000 points, 1.8M pairs: 118.6 -> 46.3 us (finish 4.3 -> 8.5); 300 rig poses,
-// 40,000 points, 3.2M pairs (two observations per pose): 118 -> 47 us (5.7 -> 7.0).  Bound by the
+// more).  200 cameras, 50,000 points, 1.8M pairs: 118.6 -> 49.6 us (finish 4.3 -> 8.5); 300 rig poses,
+// 40,000 points, 3.2M pairs (two observations per pose): 118 -> 48 us (5.7 -> 6.8).  Bound by the
 // latency of a chunk (pattern, blocks, product): the DMMAs are 14 us of it.
 constexpr int kGroupThreads = 256;
+constexpr double kGroupPivot = 1e-8;
 template <int DA>
 __device__ __forceinline__ void schur_group_body(const DevState& s, int ch) {
   using L_ = Lay<DA, 0, double>;
@@ -1115,21 +1120,34 @@ __device__ __forceinline__ void schur_group_body(const DevState& s, int ch) {
   const int p0 = d.x, np = d.y, e0 = d.z, L = d.w;
   const int rows = DA * L, ld = group_ld(rows), nq = group_pad(np);
   double* Gs = group_sm;
-  double* Vs = Gs + 3 * nq * ld + 8;                     // [nq][6] (V + lambda I)^-1
-  int* first = reinterpret_cast<int*>(Vs + 6 * nq);      // [np] first observation of the point
+  double* Ns = Gs + 3 * nq * ld + 8;                     // [nq][6] N (00 01 02 11 12 22)
+  double* Fs = Ns + 6 * nq;                              // [np][6] F^T (00 10 11 20 21 22)
+  int* first = reinterpret_cast<int*>(Fs + 6 * nq);      // [np] first observation of the point
   int* rank = first + kGroupPoints;                      // [track] rank of the observation's camera
   int* head = rank + kGroupTrack;                        // [L] first observation in the camera ...
   int* next = head + kGroupTrack;                        // [track] ... and the next one, or -1
   if (tid < np) {
     const int j = s.gr_pt[p0 + tid];
     first[tid] = s.p_ptr[j];
-    double V[L_::SV];   // zero for a fixed point and for a singular one (which k_point_eliminate reports)
-    vload(reinterpret_cast<const double*>(s.p_Vinv) + (size_t)j * L_::SV, V);
+    const double lam = *s.d_lambda;
+    double V[L_::SV], vi[L_::SV];   // (vi: zero for a fixed point and a singular one, which k_point_eliminate reports)
+    vload(reinterpret_cast<const double*>(s.p_V) + (size_t)j * L_::SV, V);
+    vload(reinterpret_cast<const double*>(s.p_Vinv) + (size_t)j * L_::SV, vi);
+    const double i0 = rsqrt(V[0] + lam), l10 = V[1] * i0, l20 = V[2] * i0;
+    const double d1 = V[3] + lam - l10 * l10, i1 = rsqrt(d1), l21 = (V[4] - l20 * l10) * i1;
+    const double d2 = V[5] + lam - l20 * l20 - l21 * l21, i2 = rsqrt(d2);
+    const bool plain = V[0] + lam > 0.0 && d1 > kGroupPivot * (V[3] + lam) && d2 > kGroupPivot * (V[5] + lam) &&
+                       isfinite(i0) && isfinite(i1) && isfinite(i2) && vi[0] != 0.0;
+    const double c10 = -l10 * i0 * i1;
+    const double F[6] = {i0, c10, i1, -(l20 * i0 + l21 * c10) * i2, -l21 * i1 * i2, i2};
 #pragma unroll
-    for (int t = 0; t < 6; ++t) Vs[6 * tid + t] = V[t];
+    for (int t = 0; t < 6; ++t) {
+      Fs[6 * tid + t] = plain ? F[t] : (t == 0 || t == 2 || t == 5) ? 1.0 : 0.0;
+      Ns[6 * tid + t] = !plain ? vi[t] : (t == 0 || t == 3 || t == 5) ? 1.0 : 0.0;
+    }
   } else if (tid < nq) {                                 // the last DMMA steps' padding
 #pragma unroll
-    for (int t = 0; t < 6; ++t) Vs[6 * tid + t] = 0.0;
+    for (int t = 0; t < 6; ++t) Ns[6 * tid + t] = 0.0;
   } else if (tid >= kGroupThreads - kGroupTrack) {       // two other warps: the pattern
     const int t = tid - (kGroupThreads - kGroupTrack), j = s.gr_pt[p0], k0 = s.p_ptr[j], n = s.p_ptr[j + 1] - k0;
     rank[t] = t < n ? (int)s.gr_rank[k0 + t] : -1;
@@ -1151,6 +1169,8 @@ __device__ __forceinline__ void schur_group_body(const DevState& s, int ch) {
   // one column (of three) of a point's rows in one camera per thread
   for (int idx = tid; idx < 3 * np * L; idx += kGroupThreads) {
     const int q = idx / (3 * L), rest = idx - q * 3 * L, sl = rest / 3, u = rest - 3 * sl;
+    const double* f = Fs + 6 * q;
+    const double f0 = u == 0 ? f[0] : u == 1 ? f[1] : f[3], f1 = u == 0 ? 0.0 : u == 1 ? f[2] : f[4], f2 = u == 2 ? f[5] : 0.0;
     double g[DA];
 #pragma unroll
     for (int a = 0; a < DA; ++a) g[a] = 0.0;
@@ -1159,7 +1179,7 @@ __device__ __forceinline__ void schur_group_body(const DevState& s, int ch) {
       double A[L_::SA], B[kSB];
       vload(reinterpret_cast<const double*>(s.o_A) + k * L_::SA, A);
       vload(s.o_B + k * kSB, B);
-      const double h0 = u == 0 ? B[0] : u == 1 ? B[1] : B[2], h1 = u == 0 ? B[3] : u == 1 ? B[4] : B[5];
+      const double h0 = B[0] * f0 + B[1] * f1 + B[2] * f2, h1 = B[3] * f0 + B[4] * f1 + B[5] * f2;   // of B_k F
 #pragma unroll
       for (int a = 0; a < DA; ++a) g[a] += A[a] * h0 + A[DA + a] * h1;
     }
@@ -1168,7 +1188,7 @@ __device__ __forceinline__ void schur_group_body(const DevState& s, int ch) {
     for (int a = 0; a < DA; ++a) out[a] = g[a];
   }
   __syncthreads();
-  // lower tiles of G Vinv G^T, up to three of a tile row at a time (they share the row's fragment); three DMMA
+  // lower tiles of G N G^T, up to three of a tile row at a time (they share the row's fragment); three DMMA
   // steps take four points, lane kk = 0..3 of a step one column of point kk
   const int T = (rows + 7) / 8, r = lane >> 2, kk = lane & 3;
   int unit = 0;
@@ -1179,7 +1199,7 @@ __device__ __forceinline__ void schur_group_body(const DevState& s, int ch) {
       double acc[3][2] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
       const double* ga = Gs + 3 * kk * ld + 8 * ti + r;
       const double* gb = Gs + 3 * kk * ld + 8 * tj + r;
-      const double2* vp = reinterpret_cast<const double2*>(Vs + 6 * kk);
+      const double2* vp = reinterpret_cast<const double2*>(Ns + 6 * kk);
       for (int q = 0; q < nq; q += 4, ga += 12 * ld, gb += 12 * ld, vp += 12) {
         const double2 v0 = vp[0], v1 = vp[1], v2 = vp[2];   // 00 01, 02 11, 12 22
         const double g0 = ga[0], g1 = ga[ld], g2 = ga[2 * ld];
