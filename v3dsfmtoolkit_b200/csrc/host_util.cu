@@ -250,15 +250,20 @@ struct Pieces {
 
   Pieces(const std::vector<HostCopy>& list, bool down, cudaStream_t st) {
     constexpr size_t kPieceMin = (size_t)256 << 10;
+    const size_t least = down ? kRingDown : kRingUp;
     size_t large = 0;
+    for (const HostCopy& c : list)
+      if (c.bytes >= kPieceMin) large += c.bytes;
     std::vector<char> cut(list.size(), 0);
-    for (size_t i = 0; i < list.size(); ++i) {
-      cut[i] = list[i].bytes >= kPieceMin && !direct(down ? list[i].dst : list[i].src);
-      if (cut[i]) large += list[i].bytes;
-    }
+    if (large >= least)   // (the look at a pointer takes 3 us)
+      for (size_t i = 0; i < list.size(); ++i) {
+        if (list[i].bytes < kPieceMin) continue;
+        cut[i] = !direct(down ? list[i].dst : list[i].src);
+        if (!cut[i]) large -= list[i].bytes;
+      }
     // (the slots' events are the current context's and cannot be recorded on another one's stream)
-    staged = large >= (down ? kRingDown : kRingUp) && cudaFree(nullptr) == cudaSuccess &&
-             stream_context(st) == current_context() && ring_acquire(ring) == V3DBA_OK;
+    staged = large >= least && cudaFree(nullptr) == cudaSuccess && stream_context(st) == current_context() &&
+             ring_acquire(ring) == V3DBA_OK;
     for (size_t i = 0; i < list.size(); ++i) {
       const HostCopy& c = list[i];
       if (!c.bytes) continue;
