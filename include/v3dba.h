@@ -250,6 +250,11 @@ int v3dba_create_point_structure(int from_scratch, int n_points, int n_measureme
  * host memory).  Returns V3DBA_OK and *fail = 1 when a pivot is not positive. */
 int v3dba_dense_cholesky_solve(int n, const double* S, const double* rhs, double* x, int* fail);
 
+/* With FP64 blocks the Schur sums go over groups of points that the same cameras see, where that is the
+ * faster way, or over the lists of observation pairs: the same system in another order of summation.
+ * V3DBA_SCHUR=groups|pairs in the environment forces either when a handle first solves with FP64 blocks
+ * (for tests; every handle of the process). */
+
 /* Benchmark support (no counterpart in the reference): the same tile Cholesky factor + solve
  * timed alone on the GPU, `reps` times from the same input; *ms receives the mean device time of
  * one factor + solve (CUDA events), x and *fail the result.  trace (may be NULL, up to trace_cap

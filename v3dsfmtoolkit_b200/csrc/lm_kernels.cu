@@ -1779,8 +1779,10 @@ __global__ void __launch_bounds__(128) k_finish_merged(DevState s, int g1, int g
 // Camera (and global) update (blocks [0, g1)) and point back-substitution: both read the
 // reduced solution and the current parameters and write different parts of the trial ones.  At most 64
 // registers: the few camera blocks would take 80 to 120 and leave the points, which need 32 to 42 and wait for
-// their loads, half the warps (5.5M observations, the whole iteration 2341 -> 2275 us; 40 registers 2279, and
-// 3 us more on 20 cameras, whose camera blocks then spill on the critical path).
+// their loads, half the warps (5.5M observations, the whole iteration 2341 -> 2275 us; 375,000, FP64 blocks 497
+// -> 495).  Camera blocks with a K of their own then spill (88 bytes, 120 to 284 with a distortion of their own),
+// which small scenes do not feel: 20 cameras 111 us an iteration, 25 with their own intrinsics 187, either way
+// (at 40 registers 20 cameras took 3 us more).
 template <int MODEL, int DA, int DC, typename Real>
 __global__ void __launch_bounds__(128, 8) k_update_merged(DevState s, int g1, int g2, double* __restrict__ pcam,
                                                        double* __restrict__ ppt) {
