@@ -99,10 +99,14 @@ const Driver& driver() {
   }();
   return d;
 }
-// The current context, and a stream's; 0 where there is none.
-uint64_t current_context() {
+// The current context, made where there is none yet in this thread or it was reset (only then is the runtime
+// asked: another thread may be capturing a graph), and a stream's; 0 where there is none.
+uint64_t current_context(bool make = true) {
   unsigned long long id = 0;
-  return driver().id && driver().id(nullptr, &id) == CUDA_SUCCESS ? id : 0;
+  if (!driver().id) return 0;
+  if (driver().id(nullptr, &id) == CUDA_SUCCESS) return id;
+  if (!make || cudaFree(nullptr) != cudaSuccess) return 0;
+  return driver().id(nullptr, &id) == CUDA_SUCCESS ? id : 0;
 }
 uint64_t stream_context(cudaStream_t st) {
   CUcontext c = nullptr;
@@ -144,7 +148,7 @@ Kept& kept() {
       Kept& k2 = kept();
       std::lock_guard<std::mutex> lock(k2.m);
       k2.closing = true;
-      const uint64_t ctx = current_context();
+      const uint64_t ctx = current_context(false);
       for (CallRes& r : k2.res)
         if (r.ctx == ctx) destroy(r);
       for (Ring& r : k2.rings)
@@ -203,7 +207,6 @@ void ring_release(Ring& r) {
 }  // namespace
 
 int CallRes::acquire() {
-  V3DBA_CUDA_TRY(cudaFree(nullptr));   // the current context, made if there is none yet or it was reset
   ctx = current_context();
   if (ctx) {
     Kept& k = kept();
@@ -262,8 +265,7 @@ struct Pieces {
         if (!cut[i]) large -= list[i].bytes;
       }
     // (the slots' events are the current context's and cannot be recorded on another one's stream)
-    staged = large >= least && cudaFree(nullptr) == cudaSuccess && stream_context(st) == current_context() &&
-             ring_acquire(ring) == V3DBA_OK;
+    staged = large >= least && stream_context(st) == current_context() && ring_acquire(ring) == V3DBA_OK;
     for (size_t i = 0; i < list.size(); ++i) {
       const HostCopy& c = list[i];
       if (!c.bytes) continue;
