@@ -11,7 +11,7 @@ namespace v3dba {
 
 constexpr int kRigStride = 24;   // doubles per rig camera: K 9, R 9, T 3, padding
 
-struct ParamSet {
+struct ParamSet {           // one block that begins with K
   double* K = nullptr;     // STD/VARYING: N*9, COMMON: 9
   double* R = nullptr;     // N*9
   double* T = nullptr;     // N*3
