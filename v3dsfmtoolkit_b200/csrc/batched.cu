@@ -346,7 +346,7 @@ __device__ __forceinline__ double slots_warp_sum(const double (*v)[32]) {
 // so one pass builds U, the Schur complement, the reduced rhs (a seventh column r_i - B_i q) and the
 // gradient (an eighth, r_i) from one linearisation of every observation; each warp sums its points in
 // eight-by-eight accumulators and the slots' sums are added in order (deterministic, no atomics).
-// Bound by FP64 latency: 14 KB of operand tiles per warp and 168 registers (a few spill: 28 bytes a thread
+// Bound by FP64 latency: 14 KB of operand tiles per warp and 168 registers (a few spill: 60 bytes a thread
 // with three cameras, about 550 with four) leave 12 warps per SM, the FP64 pipe is active 24% and the DMMA
 // pipe 16% of the cycles.  Of the 2.2 ms that 4096 triplets of 50-800 points take for 4 iterations the products
 // are 0.8, the step pass 0.5, the solve 0.25 (timed by leaving each out).  Loading the next tile's tracks
@@ -466,7 +466,8 @@ __global__ void __launch_bounds__(NT, NT > 128 ? 1 : 384 / NT) k_batched_lm(Batc
               if (has) b.w[o0 + (int)((tr.slot >> (4 * c)) & 15u)] = w;
               weigh(ol, w, r[c]);
               if (!has) ol.P[0] = ol.P[1] = ol.P[2] = ol.P[3] = r[c][0] = r[c][1] = 0.0;
-              err += r[c][0] * r[c][0] + r[c][1] * r[c][1];
+              const double cost = w * w * (ol.e[0] * ol.e[0] + ol.e[1] * ol.e[1]);
+              err += has ? cost : 0.0;
               point_block(cams[c], ol, B[c]);
               double A[2][6];
               camera_block(ol, A);
@@ -482,12 +483,23 @@ __global__ void __launch_bounds__(NT, NT > 128 ? 1 : 384 / NT) k_batched_lm(Batc
             bool ok = true;
             if (mode == 1) {
               ok = invert_point(V, lam, vi, &det);
-              if (!ok && !isfinite(det)) {   // a point at infinity contributes nothing
+              const bool dead = !ok && !isfinite(det);
+              // A point at infinity enters the gradient (column 7 of the cameras' own blocks), where it is no
+              // number unless the camera sees it well, but not the system.
+              if (__any_sync(0xffffffffu, dead)) {
                 const double zero2[2][6] = {};
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
-                  if (c < N) store_a(Aw + c * 6 * kTileLd, lane, zero2);
-                  r[c][0] = r[c][1] = 0.0;
+                  if (c >= N) continue;
+                  for (int a = 0; a < 6; ++a) {
+                    const double2 u = *reinterpret_cast<const double2*>(Aw + (6 * c + a) * kTileLd + 2 * lane);
+                    const double g = warp_sum(dead ? u.x * r[c][0] + u.y * r[c][1] : 0.0);
+                    if (lane == 4 * a + 3) acc[c * NC - c * (c - 1) / 2][1] += g;
+                  }
+                  if (dead) {
+                    store_a(Aw + c * 6 * kTileLd, lane, zero2);
+                    r[c][0] = r[c][1] = 0.0;
+                  }
                 }
               }
             }
@@ -558,7 +570,28 @@ __global__ void __launch_bounds__(NT, NT > 128 ? 1 : 384 / NT) k_batched_lm(Batc
                       have = b.cam[o0 + t] == i && b.cam[o0 + u] == l && (mode == 1 || t == u);
                     }
                     if (!__any_sync(0xffffffffu, have)) break;
+                    const int at = i * NC - i * (i - 1) / 2 + (l - i);
                     double At[2][6] = {}, Z[8][2] = {};
+                    if (i == l && __any_sync(0xffffffffu, have && dead && t == u)) {   // (as above)
+                      double g[6] = {};
+                      if (have && dead && t == u) {
+                        double rt[2];
+                        ObsLin ol;
+                        project_obs(cams[i], X, b.meas[2 * (size_t)(o0 + t)], b.meas[2 * (size_t)(o0 + t) + 1], ol);
+                        weigh(ol, b.w[o0 + t], rt);
+                        camera_block(ol, At);
+                        for (int a = 0; a < 6; ++a) {
+                          g[a] = At[0][a] * rt[0] + At[1][a] * rt[1];
+                          At[0][a] = At[1][a] = 0.0;
+                        }
+                      }
+                      for (int a = 0; a < 6; ++a) {
+                        const double v = warp_sum(g[a]);
+#pragma unroll
+                        for (int pr = 0; pr < L::kPairs; ++pr)
+                          if (pr == at && lane == 4 * a + 3) acc[pr][1] += v;
+                      }
+                    }
                     if (have && !dead) {
                       double Au[2][6], Bt[2][3], Bu[2][3], rt[2], ru[2], BV[2][3];
                       ObsLin ol;
@@ -590,7 +623,6 @@ __global__ void __launch_bounds__(NT, NT > 128 ? 1 : 384 / NT) k_batched_lm(Batc
                     __syncwarp();
                     double add[2] = {0.0, 0.0};
                     tile_product(Ac, Zw, zrow, 8, lane, add);
-                    const int at = i * NC - i * (i - 1) / 2 + (l - i);
 #pragma unroll
                     for (int pr = 0; pr < L::kPairs; ++pr)
                       if (pr == at) { acc[pr][0] += add[0]; acc[pr][1] += add[1]; }
@@ -639,7 +671,9 @@ __global__ void __launch_bounds__(NT, NT > 128 ? 1 : 384 / NT) k_batched_lm(Batc
         __syncthreads();
         if (wid == 0) {
           const double errs = warp_sum(slots_total(dyn + L::kA + lane, 32));
-          double gx = lane < 6 * N ? fabs(ga[lane]) : 0.0, dx = (mode == 0 && lane < 6 * N) ? udiag[lane] : -1e30;
+          // (fmax leaves out what is no number)
+          double gx = lane < 6 * N ? fmax(fabs(ga[lane]), 0.0) : 0.0;
+          double dx = (mode == 0 && lane < 6 * N) ? fmax(udiag[lane], -1e30) : -1e30;
           gx = warp_max(gx);
           dx = warp_max(dx);
           if (lane == 0) {
